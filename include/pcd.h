@@ -94,9 +94,13 @@ typedef enum {
 } pcd_warm_start;
 
 typedef enum {
-    PCD_SCHED_AUTO = 0,        /* FP32 sweeps: cluster, else tiles (grids of at least 64 x 64
-                                  cells), else persistent, else stream; FP64: persistent, else
-                                  stripes; else launches, as the grid allows */
+    PCD_SCHED_AUTO = 0,        /* FP32 sweeps: tiles that stay on the chip where the grid fits (up
+                                  to about two million cells; reported as PCD_SCHED_TILES, with
+                                  the stop tests of the schedule they stand for: the cluster's
+                                  estimate cycles, the tile passes' or the persistent bands'
+                                  chunks), else tile passes (grids of at least 64 x 64 cells),
+                                  else persistent, else stream; FP64: blocks, else persistent,
+                                  else stripes; else launches, as the grid allows */
     PCD_SCHED_LAUNCHES = 1,    /* one kernel per half sweep, CUDA-graph chunks (any grid) */
     PCD_SCHED_PERSISTENT = 2,  /* one cooperative launch per solve, bands in shared memory
                                   (no NaN cells, band fits on chip) */

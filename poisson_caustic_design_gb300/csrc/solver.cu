@@ -31,6 +31,7 @@
 #include "sor_persist.cuh"
 #include "sor_cluster.cuh"
 #include "sor_blocks.cuh"
+#include "sor_resident.cuh"
 
 namespace pcd {
 
@@ -601,8 +602,10 @@ void SolverWorkspace::release()
     if (flags) cudaFree(flags);
     if (part) cudaFree(part);
     if (bx) cudaFree(bx);
-    r64 = nullptr; xbuf = nullptr; flags = nullptr; part = nullptr; bx = nullptr;
-    xbuf_elems = 0; max_ctas = 0; bx_bytes = 0;
+    if (rx) cudaFree(rx);
+    r64 = nullptr; xbuf = nullptr; flags = nullptr; part = nullptr; bx = nullptr; rx = nullptr;
+    xbuf_elems = 0; max_ctas = 0; bx_bytes = 0; rx_bytes = 0;
+    plans.clear();
     if (partials) cudaFree(partials);
     if (ctl) cudaFree(ctl);
     if (ctl_host) cudaFreeHost(ctl_host);
@@ -1035,6 +1038,204 @@ int solve_cluster(SolverWorkspace &ws, const double *b, double *phi, const Solve
 
 }  // namespace
 
+namespace {
+
+// How the resident sweeps end their launches, so that every grid keeps the
+// stop tests (and with them the sweep counts) of the schedule it is resident
+// for: the cluster's residual-estimate cycles, the tile passes' chunks with a
+// test after every pass, or the persistent bands' chunks.
+struct ResidentRule {
+    int cycle = 0;               // 1: estimate cycles
+    int dep = 1, lag = 0;        // cycle: estimates on multiples of dep, end lag sweeps later
+    int chunk = 0, gran = 0;     // chunk: sweeps per launch, tracked every gran sweeps
+    int sched = PCD_SCHED_TILES; // what the solve reports
+};
+
+template <typename Plan, typename Make>
+int cached_plan(SolverWorkspace &ws, std::vector<int> key, Plan *out, Make make)
+{
+    // entry: status byte, then the plan
+    auto it = ws.plans.find(key);
+    if (it == ws.plans.end()) {
+        Plan p{};
+        const int st = make(&p);
+        if (st != PCD_OK && st != PCD_BAD_ARG) return st;
+        if (ws.plans.size() >= 256) ws.plans.clear();
+        std::vector<char> v(1 + sizeof(Plan));
+        v[0] = (char)st;
+        std::memcpy(v.data() + 1, &p, sizeof(Plan));
+        it = ws.plans.emplace(std::move(key), std::move(v)).first;
+    }
+    std::memcpy(out, it->second.data() + 1, sizeof(Plan));
+    return it->second[0];
+}
+
+enum { kPlanResident = 0, kPlanCluster = 1, kPlanTile = 2, kPlanPersist = 3 };
+
+// FP32 sweeps between FP64 refreshes of the chunked mixed schedules.
+int mixed_chunk(const SolveArgs &a, const pcd_solve_opts &o)
+{
+    const int n = std::max(a.W, a.H);
+    int chunk;
+    if (a.stop == PCD_STOP_MAX_UPDATE)
+        // (the stop test runs after every pass either way)
+        chunk = o.refine_every > 0 ? o.refine_every : std::max(32, std::min(128, n / 32));
+    else
+        // the FP64 refresh costs several FP32 sweeps; FP32 can carry ~2 digits
+        // of the correction, i.e. hundreds of sweeps on large grids
+        chunk = o.refine_every > 0 ? o.refine_every
+                                   : (o.check_every > 0 ? o.check_every : std::max(32, std::min(256, n / 16)));
+    if (chunk > a.max_iter && a.max_iter > 0) chunk = a.max_iter;
+    return chunk;
+}
+
+// Whether (and under which rule) the mixed solve's sweeps run resident.
+int resident_rule(SolverWorkspace &ws, const SolveArgs &a, const pcd_solve_opts &o, ResidentPlan *plan,
+                  ResidentRule *rule)
+{
+    if (o.precision != PCD_PREC_MIXED || o.schedule != PCD_SCHED_AUTO) return PCD_BAD_ARG;
+    const int W = a.W, H = a.H;
+    int st = cached_plan(ws, {kPlanResident, W, H}, plan, [&](ResidentPlan *p) { return resident_plan(ws.dev, W, H, p); });
+    if (st != PCD_OK) return st;
+    ResidentRule r;
+    if (a.stop == PCD_STOP_REL_RESIDUAL) {
+        ClusterPlan cp{};
+        st = cached_plan(ws, {kPlanCluster, W, H}, &cp, [&](ClusterPlan *p) { return cluster_plan(ws.dev, W, H, 4, p); });
+        if (st == PCD_OK) {
+            r.cycle = 1;
+            r.dep = std::max(1, cp.depth);
+            r.lag = cp.rr_l ? cp.depth : 0;
+            *rule = r;
+            return PCD_OK;
+        }
+        if (st != PCD_BAD_ARG) return st;
+    }
+    const int depth = o.check_every > 0 && o.check_every <= 2 ? 2 : 4;
+    TilePlan tp{};
+    st = cached_plan(ws, {kPlanTile, W, H, a.ld % 4, depth}, &tp,
+                     [&](TilePlan *p) { return tile_plan(ws.dev, W, H, a.ld, depth, p); });
+    if (st != PCD_OK && st != PCD_BAD_ARG) return st;
+    if (st == PCD_OK && (long)W * H >= kTileMinCells) {
+        r.chunk = mixed_chunk(a, o);
+        r.gran = o.check_every > 0 ? std::min(o.check_every, 4) : 4;
+    } else {
+        struct { int G; size_t smem; } pp{};
+        st = cached_plan(ws, {kPlanPersist, W, H}, &pp,
+                         [&](decltype(pp) *p) { return persist_grid(ws.dev, W, H, true, &p->G, &p->smem); });
+        if (st != PCD_OK) return st;
+        r.chunk = o.check_every > 0 ? o.check_every : (a.stop == PCD_STOP_MAX_UPDATE ? 16 : 32);
+        if (o.refine_every > 0 && o.refine_every < r.chunk) r.chunk = o.refine_every;
+        r.gran = r.chunk;
+    }
+    if (a.stop != PCD_STOP_MAX_UPDATE) r.gran = 0;
+    if (r.gran > 0 && (r.chunk - 1) / r.gran + 1 > kResidentChecksMax) return PCD_BAD_ARG;
+    *rule = r;
+    return PCD_OK;
+}
+
+// Mixed precision on resident tiles: launches of [FP32 sweeps, FP64 residual
+// refresh, phi += e] until the stop test passes.  The next launch is enqueued
+// before the previous one's control block is read; a launch after the stop
+// returns at once.
+int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const pcd_solve_opts &o,
+                   const ResidentPlan &plan, const ResidentRule &rule, pcd_solve_stats *stats, cudaStream_t s)
+{
+    const int G = plan.TX * plan.TY;
+    const size_t part_at = plan.xb_bytes, gmax_at = part_at + 2 * (size_t)G * sizeof(unsigned long long);
+    const size_t bar_at = gmax_at + kResidentChecksMax * sizeof(unsigned), need = bar_at + 64;
+    if (need > ws.rx_bytes) {
+        if (ws.rx) cudaFree(ws.rx);
+        ws.rx = nullptr;
+        ws.rx_bytes = 0;
+        PCD_CUDA(cudaMalloc(&ws.rx, need));
+        ws.rx_bytes = need;
+    }
+    // epochs start at 0 in every solve: no word of an earlier one may match
+    PCD_CUDA(cudaMemsetAsync(ws.rx, 0, need, s));
+    const int rblocks = grid_blocks((long)a.W * a.H);
+    PCD_CUDA(cudaMemsetAsync(ws.e32, 0, sizeof(float) * (size_t)a.H * a.ld, s));
+    k_refine_residual<false><<<rblocks, kThreads, 0, s>>>(phi, ws.e32, b, ws.mask, ws.r32, ws.ctl, ws.partials, a, 1);
+    PCD_LAUNCHED(1);
+    if (rule.cycle) {
+        // (as the cluster schedule: a passing initial guess is done here)
+        k_refine_update<<<rblocks, kThreads, 0, s>>>(phi, ws.e32, ws.ctl, a);
+        PCD_LAUNCHED(1);
+    }
+
+    ResidentArgs ra{};
+    ra.W = a.W; ra.H = a.H; ra.ld = a.ld;
+    ra.e = ws.e32; ra.r32 = ws.r32; ra.ctl = ws.ctl;
+    char *rx = static_cast<char *>(ws.rx);
+    ra.xb = rx;
+    ra.part = reinterpret_cast<unsigned long long *>(rx + part_at);
+    ra.gmax = reinterpret_cast<unsigned *>(rx + gmax_at);
+    ra.bar = reinterpret_cast<unsigned *>(rx + bar_at);
+    ra.max_iter = a.max_iter;
+    ra.cycle = rule.cycle;
+    ra.nsw = rule.cycle ? (o.refine_every > 0 ? o.refine_every : 2048) : rule.chunk;
+    ra.check_every = o.check_every > 0 ? o.check_every : 16;
+    ra.dep = rule.dep;
+    ra.lag = rule.lag;
+    ra.gran = rule.gran;
+    ra.tol = a.tol;
+    ra.drop = o.refine_drop > 0.0 ? o.refine_drop : 3e-2;
+    for (int c = 0; c < 5; c++) ra.w32[c] = a.w32[c];
+    // a poll is an L2 trip: about two seconds
+    ra.spin_limit = ws.wait_limit > 0 ? ws.wait_limit : 1ll << 21;
+    ra.withhold = ws.withhold_flag;
+
+    PCD_CUDA(cudaEventRecord(ws.k0, s));
+    const long max_launches = rule.cycle ? (long)a.max_iter + 4 : (long)a.max_iter / std::max(1, rule.chunk) + 3;
+    long launched = 0;
+    bool finished = false;
+    while (!finished) {
+        if (launched >= max_launches) {
+            set_error("resident SOR: launch budget exceeded without a done flag");
+            return PCD_TIMEOUT;
+        }
+        PCD_TRY(launch_resident(ra, plan, s));
+        k_refine_residual<false><<<rblocks, kThreads, 0, s>>>(phi, ws.e32, b, ws.mask, ws.r32, ws.ctl, ws.partials, a, 0);
+        PCD_LAUNCHED(1);
+        k_refine_update<<<rblocks, kThreads, 0, s>>>(phi, ws.e32, ws.ctl, a);
+        PCD_LAUNCHED(1);
+        const int slot = (int)(launched & 1);
+        PCD_CUDA(cudaMemcpyAsync(&ws.ctl_host[slot], ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+        PCD_CUDA(cudaEventRecord(ws.ev[slot], s));
+        launched++;
+        if (launched >= 2) {
+            const int prev = (int)((launched - 2) & 1);
+            PCD_CUDA(cudaEventSynchronize(ws.ev[prev]));
+            if (ws.ctl_host[prev].done || ws.ctl_host[prev].error) finished = true;
+        }
+    }
+    PCD_CUDA(cudaEventRecord(ws.k1, s));
+    PCD_CUDA(cudaEventRecord(ws.t1, s));
+    PCD_CUDA(cudaMemcpyAsync(&ws.ctl_host[0], ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+    PCD_CUDA(cudaStreamSynchronize(s));
+    const Ctl &c = ws.ctl_host[0];
+    if (c.error) {
+        set_error("resident SOR: a bounded device wait gave up (status " + std::to_string(c.error) + ")");
+        return c.error;
+    }
+    if (stats) {
+        stats->sweeps = c.sweeps;
+        stats->converged = c.converged;
+        stats->rel_residual = c.rel;
+        stats->max_residual = c.rmax;
+        stats->last_max_update = c.last_max;
+        stats->residual_checks = c.checks;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ws.t0, ws.t1);
+        stats->device_ms = ms;
+        cudaEventElapsedTime(&ms, ws.k0, ws.k1);
+        stats->sweep_ms = ms;
+        stats->schedule_used = rule.sched;
+    }
+    return c.converged ? PCD_OK : PCD_NOT_CONVERGED;
+}
+
+}  // namespace
+
 int residual_rel(SolverWorkspace &ws, const double *b, const double *phi, int W, int H, int ld, cudaStream_t s,
                  double *rel)
 {
@@ -1219,6 +1420,13 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
                 if ((st = blocks_plan(ws.dev, W, H, K, mixed, &bp)) == PCD_OK) break;
         if (st == PCD_OK) return solve_blocks(ws, b, phi, a, precision, o, bp, stats, s);
     }
+    if (!done_already && !masked && precision == PCD_PREC_MIXED) {
+        ResidentPlan rp;
+        ResidentRule rule;
+        const int st = resident_rule(ws, a, o, &rp, &rule);
+        if (st == PCD_OK) return solve_resident(ws, b, phi, a, o, rp, rule, stats, s);
+        if (st != PCD_BAD_ARG) return st;
+    }
     if (!done_already && !masked && precision == PCD_PREC_MIXED && a.stop == PCD_STOP_REL_RESIDUAL &&
         (o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_CLUSTER)) {
         ClusterPlan plan{};
@@ -1281,21 +1489,8 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_stripe_a<double, false, 4>, kStripeThreads, 0));
         ws.stripe_resident = std::max(1, bps) * sms;
     }
-    int chunk;
-    if (a.stop == PCD_STOP_MAX_UPDATE)
-        // mixed: FP32 sweeps between FP64 refreshes (the stop test runs after
-        // every sweep either way)
-        chunk = precision == PCD_PREC_MIXED
-                    ? (o.refine_every > 0 ? o.refine_every : std::max(32, std::min(128, std::max(W, H) / 32)))
-                    : 32;
-    else if (precision == PCD_PREC_MIXED)
-        // the FP64 refresh costs several FP32 sweeps; FP32 can carry ~2 digits
-        // of the correction, i.e. hundreds of sweeps on large grids
-        chunk = o.refine_every > 0 ? o.refine_every
-                                   : (o.check_every > 0 ? o.check_every
-                                                        : std::max(32, std::min(256, std::max(W, H) / 16)));
-    else
-        chunk = o.check_every > 0 ? o.check_every : 32;
+    int chunk = precision == PCD_PREC_MIXED ? mixed_chunk(a, o)
+                : a.stop == PCD_STOP_MAX_UPDATE ? 32 : o.check_every > 0 ? o.check_every : 32;
     if (chunk > a.max_iter && a.max_iter > 0) chunk = a.max_iter;
 
     SolverWorkspace::GraphEntry *ge = nullptr;

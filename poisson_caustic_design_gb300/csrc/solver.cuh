@@ -28,6 +28,8 @@ struct Ctl {
     int nan_cells;               // NaN entries of b
     int error;                   // PCD_TIMEOUT when a bounded device wait gave up
     int stream_out;              // ping-pong buffer holding the latest FP32 correction
+    unsigned int res_epoch;      // resident sweeps: halo exchanges of this solve so far
+    unsigned int res_checks;     // resident sweeps: residual estimates of this solve so far
     unsigned long long maxbits;  // running max |delta| of the current sweep
     double last_max;             // max |delta| of the last full sweep
     double rnorm, bnorm, rmax, rel;
@@ -103,6 +105,13 @@ struct SolverWorkspace {
     // the block schedule's exchange grids (and the mixed form's FP32 rhs grid)
     void *bx = nullptr;
     size_t bx_bytes = 0;
+    // the resident sweeps' exchange words, and behind them the residual
+    // partials, tracked maxima and barrier counter (all zeroed per solve)
+    void *rx = nullptr;
+    size_t rx_bytes = 0;
+    // launch plans by grid size and kind (host arithmetic and device queries
+    // that would otherwise be repeated on every call); bounded
+    std::map<std::vector<int>, std::vector<char>> plans;
 
     struct GraphEntry {
         cudaGraphExec_t exec;

@@ -28,6 +28,7 @@
 
 #include "sor_cluster.cuh"
 #include "sor_planes.cuh"
+#include "sor_quads.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -36,6 +37,7 @@ namespace pcd {
 namespace {
 
 using namespace planes;
+using namespace quads;
 
 __global__ void __launch_bounds__(kClusterThreads, 1) k_sor_cluster(ClusterArgs a)
 {
@@ -147,24 +149,6 @@ __host__ __device__ inline size_t tb_floats(int nmax, int KHp)
 {
     constexpr int HK = 2 * K;
     return (size_t)4 * (nmax + 2 * HK) * KHp + (size_t)8 * HK * KHp;
-}
-
-__device__ __forceinline__ float4 lds4(unsigned a)
-{
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ float lds1(unsigned a)
-{
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ void sts4(unsigned a, const float4 &v)
-{
-    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-                 : "memory");
 }
 
 // The first / last quad of an interior row after the interior form: the

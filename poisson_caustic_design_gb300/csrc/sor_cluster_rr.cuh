@@ -1,6 +1,6 @@
 // sor_cluster_rr.cuh -- register-resident form of the cluster FP32 SOR
-// (included by sor_cluster.cu inside its anonymous namespace, after the
-// shared-memory helpers lds4 / sts4).
+// (included by sor_cluster.cu inside its anonymous namespace; the quad
+// arithmetic is in sor_quads.cuh).
 //
 // Widths W = 8 KQ up to 512, K = 4 or 2 sweeps per halo exchange, L = 2..4
 // rows per warp, NQ = 1 or 2 quads per lane.  A CTA of 16 warps; warp w
@@ -39,50 +39,6 @@ __host__ __device__ inline size_t rr_floats(int K, int NQ, int R)
 {
     const size_t KS = (size_t)128 * NQ;
     return ((size_t)4 * kRRWarps + (size_t)16 * K + (size_t)2 * R) * KS;
-}
-
-// The update of quad_ghost with the parity q as an argument (folded to a
-// constant where the caller's q is one), in packed FP32 pairs: cells (x, y)
-// and (z, w) of the quad share one instruction per step.  nrh is -r32.  The
-// steps and their rounding are those of the scalar form
-// v + w ((l + r) + (u + d) - 4 v - r32).
-__device__ __forceinline__ float4 quad_ghost_q(int q, const float4 &v, const float4 &nrh, const float4 &u,
-                                              const float4 &d, const float4 &m, float ex, float2 wA, float2 wB)
-{
-    const float h0 = q ? ex + m.x : m.x + m.y;
-    const float h1 = q ? m.x + m.y : m.y + m.z;
-    const float h2 = q ? m.y + m.z : m.z + m.w;
-    const float h3 = q ? m.z + m.w : m.w + ex;
-    const float2 vA = make_float2(v.x, v.y), vB = make_float2(v.z, v.w);
-    const float2 m4 = make_float2(-4.f, -4.f);
-    float2 tA = __fadd2_rn(make_float2(h0, h1), __fadd2_rn(make_float2(u.x, u.y), make_float2(d.x, d.y)));
-    float2 tB = __fadd2_rn(make_float2(h2, h3), __fadd2_rn(make_float2(u.z, u.w), make_float2(d.z, d.w)));
-    tA = __fadd2_rn(__ffma2_rn(m4, vA, tA), make_float2(nrh.x, nrh.y));
-    tB = __fadd2_rn(__ffma2_rn(m4, vB, tB), make_float2(nrh.z, nrh.w));
-    const float2 nA = __ffma2_rn(wA, tA, vA), nB = __ffma2_rn(wB, tB, vB);
-    return make_float4(nA.x, nA.y, nB.x, nB.y);
-}
-
-// Largest |nv - v| over the quad (a NaN change does not raise it).
-__device__ __forceinline__ float quad_max_change(const float4 &v, const float4 &nv)
-{
-    return fmaxf(fmaxf(fabsf(nv.x - v.x), fabsf(nv.y - v.y)), fmaxf(fabsf(nv.z - v.z), fabsf(nv.w - v.w)));
-}
-
-// Sum of squares of r32 - L v over the quad (ghost neighbours as above; nrh
-// is -r32).
-__device__ __forceinline__ float quad_ghost_res2(int q, const float4 &v, const float4 &nrh, const float4 &u,
-                                                const float4 &d, const float4 &m, float ex)
-{
-    const float l0 = q ? ex : m.x, r0v = q ? m.x : m.y;
-    const float l1 = q ? m.x : m.y, r1v = q ? m.y : m.z;
-    const float l2 = q ? m.y : m.z, r2v = q ? m.z : m.w;
-    const float l3 = q ? m.z : m.w, r3v = q ? m.w : ex;
-    const float a0 = nrh.x + fmaf(-4.f, v.x, (l0 + r0v) + (u.x + d.x));
-    const float a1 = nrh.y + fmaf(-4.f, v.y, (l1 + r1v) + (u.y + d.y));
-    const float a2 = nrh.z + fmaf(-4.f, v.z, (l2 + r2v) + (u.z + d.z));
-    const float a3 = nrh.w + fmaf(-4.f, v.w, (l3 + r3v) + (u.w + d.w));
-    return fmaf(a0, a0, fmaf(a1, a1, fmaf(a2, a2, a3 * a3)));
 }
 
 template <int K, int L, int NQ>

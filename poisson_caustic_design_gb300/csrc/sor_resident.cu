@@ -1,0 +1,834 @@
+// sor_resident.cu -- FP32 red-black SOR sweeps of the correction equation
+// L e = r32 with the whole grid resident on the chip (sm_103a).
+//
+// The grid is cut into TX x TY tiles, one CTA each, all co-resident
+// (cooperative launch).  A CTA holds its tile plus a halo of 2K cells on every
+// side that has a neighbour; e lives in registers for the whole launch, so
+// does -r32 where a lane holds at most two rows (in shared memory otherwise).
+// K sweeps run between two exchanges: the dependency cone of K red-black
+// sweeps ends inside the halo, whose values are recomputed with the owner's
+// arithmetic and thrown away at the next exchange.
+//
+// Layout: a lane holds L consecutive rows of one lane column (eight cells: one
+// quad of each colour, sor_quads.cuh).  CL lanes side by side make a tile row,
+// so a warp holds 32 / CL groups of L rows.  Horizontal neighbours come by
+// shuffle from the next lane, vertical ones from the lane's own registers and,
+// between groups, from the groups' edge rows in shared memory (double-buffered
+// by colour: one block barrier a half sweep).
+//
+// Exchange: every 32-bit value travels in a 64-bit word together with the
+// epoch it belongs to; the reader polls the words themselves.  No fence, no
+// flag and no second trip stand between a neighbour's store and this CTA's
+// use: a microbenchmark of fence + flag + poll + load needed 4-5 us for the
+// same exchange (sor_blocks.cu pays it).  Words are double-buffered by epoch
+// parity: a CTA overwrites epoch n's word with epoch n + 2 only after it read
+// its neighbours' epoch n + 1, which they publish after reading epoch n.
+// A 64-bit relaxed access is single-copy atomic, so value and epoch are never
+// torn; a vector of two is two such accesses.
+//
+// Two ways to end a launch:
+//   cycle   an FP32 estimate of ||r32 - L e|| every check_every sweeps, its
+//           partials (tagged words as above) read one round later, so that
+//           their trip overlaps the sweeps; the cycle ends `lag` sweeps after
+//           the estimate that passed, from a copy of e written then where the
+//           round has gone further;
+//   chunk   exactly nsw sweeps.  With the max-update stop every tracked
+//           sweep's largest |update| goes to a global maximum; after the last
+//           sweep one grid barrier makes them visible, and if an earlier sweep
+//           already passed the test the chunk runs again from e = 0 up to that
+//           sweep (once a solve), so no sweep ever waits for the test.
+//
+// Bound: latency.  At 512^2 (6 x 25 tiles of 88 x 22 cells, K = 8, 14 warps) a
+// sweep takes 0.62-0.67 us against the one-cluster form's 2.08 (16 SMs,
+// sor_cluster_rr.cuh): 16 half sweeps of about 470 cycles (64 instructions a
+// warp; shuffle, edge row, five dependent packed operations, block barrier)
+// and about 2900 cycles of exchange a round; 1.15-1.2 us at 1024^2 against
+// 5.7 of the tile passes.  Measured on the way: a quad held as consecutive
+// cells needs three packed registers a half sum (35 instructions a quad
+// against 24); -r32 in registers doubles the two-row form's instructions by
+// register moves; a separate update for the border rows set the pace of the
+// grid (0.59 against 0.72 us on one tile); 16-byte exchange accesses fetch
+// each sector twice (1.48 against 1.15 us a sweep at 1024^2); publishing each
+// colour as it becomes final gains nothing.
+#include <algorithm>
+
+#include "sor_resident.cuh"
+#include "sor_quads.cuh"
+
+namespace pcd {
+
+namespace {
+
+using namespace quads;
+
+__device__ __forceinline__ unsigned long long rs_word(float v, unsigned ep)
+{
+    return (unsigned long long)__float_as_uint(v) | ((unsigned long long)ep << 32);
+}
+
+// Four words, one 32-byte sector: a quad in one access (two 16-byte ones fetch
+// the sector twice, and the words of a halo fill the SM's L2 port as it is).
+struct Words {
+    unsigned long long x, y, z, w;
+};
+
+__device__ __forceinline__ void rs_st4(Words *p, const Words &v)
+{
+    asm volatile("st.relaxed.gpu.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v.x), "l"(v.y), "l"(v.z), "l"(v.w)
+                 : "memory");
+}
+
+__device__ __forceinline__ Words rs_ld4(const Words *p)
+{
+    Words v;
+    asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(v.x), "=l"(v.y), "=l"(v.z), "=l"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned long long rs_ld1(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void rs_st1(unsigned long long *p, unsigned long long v)
+{
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ unsigned rs_ld_acquire(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ bool rs_fresh(const Words &v, unsigned ep)
+{
+    return (unsigned)(v.x >> 32) == ep && (unsigned)(v.y >> 32) == ep && (unsigned)(v.z >> 32) == ep &&
+           (unsigned)(v.w >> 32) == ep;
+}
+
+__device__ __forceinline__ Quad rs_quad(const Words &v)
+{
+    return {make_float2(__uint_as_float((unsigned)v.x), __uint_as_float((unsigned)v.y)),
+            make_float2(__uint_as_float((unsigned)v.z), __uint_as_float((unsigned)v.w))};
+}
+
+__device__ __forceinline__ Words rs_words(const Quad &q, unsigned ep)
+{
+    return {rs_word(q.a.x, ep), rs_word(q.a.y, ep), rs_word(q.b.x, ep), rs_word(q.b.y, ep)};
+}
+
+// One more unsuccessful poll: false once the poll budget is spent (then
+// PCD_TIMEOUT is recorded) or another CTA recorded an error.
+__device__ __forceinline__ bool rs_again(const ResidentArgs &a, long long &it)
+{
+    if ((++it & 63) == 0) {
+        if (*(volatile const int *)&a.ctl->error) return false;
+        if (it > a.spin_limit) {
+            atomicCAS(&a.ctl->error, 0, PCD_TIMEOUT);
+            return false;
+        }
+    }
+    return true;
+}
+
+// Most warps of a CTA: as few as the tiles need, for the registers that L rows
+// of both colours take (512 threads of 128 registers spill from L = 4 on).
+__host__ __device__ constexpr int rs_warps(int L) { return L == 2 ? 16 : 12; }
+
+template <int K, int L, int CL, bool RAG>
+struct Tile {
+    static constexpr int G = 32 / CL;              // row groups of a warp
+    static constexpr int NS = RAG ? 2 : 1;         // weight sets of a row: one per parity where lanes differ
+    static_assert(L % 2 == 0, "groups start on even grid rows");
+
+    Quad e[2][L];
+    // Per row: weight omega / cnt (0 outside the grid), as pairs.
+    //   whole lane columns: wa both horizontal neighbours, wb the pair with
+    //   the grid's first or last cell
+    //   RAG: wa / wb of the quad's pairs by parity, and the coefficient of the
+    //   cell's own value (-3 in a last column inside its lane, whose right
+    //   neighbour reads 0)
+    float2 wa[NS][L], wb[NS][L], ca[2], cb[2];
+    bool own, zl, zr;
+    bool brd, gin;           // warp with the grid's first or last row; group with a row of the grid
+    int cl, gi, lr0, y0, H, nvalid;
+    int wlo, whi;            // plane rows of the warp's groups
+    unsigned edge_own, edge_up, edge_dn, edge_c;  // shared addresses; edge_c: bytes from colour 0 to 1
+    unsigned r_s, r_c;       // -r32 planes: shared address of the first row, bytes between colours
+
+    // w4, w3, w2: omega / cnt
+    __device__ __forceinline__ void setup_weights(bool act, int R, float w4, float w3, float w2)
+    {
+#pragma unroll
+        for (int j = 0; j < L; j++) {
+            const int y = y0 + j;
+            const bool in = act && lr0 + j < R && y >= 0 && y < H, mid = y > 0 && y < H - 1;
+            const float wi = !in ? 0.f : mid ? w4 : w3, we = !in ? 0.f : mid ? w3 : w2;
+            if (RAG) {
+#pragma unroll
+                for (int q = 0; q < NS; q++) {
+                    float w[4];
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        const int off = 2 * t + 1 - q, last = nvalid - 1;
+                        const bool edge = (off == 0 && zl) || (off == 7 && zr) || (off == last && nvalid < 8);
+                        w[t] = off > last ? 0.f : edge ? we : wi;
+                    }
+                    wa[q][j] = make_float2(w[0], w[2]);
+                    wb[q][j] = make_float2(w[1], w[3]);
+                }
+            } else {
+                wa[0][j] = make_float2(wi, wi);
+                wb[0][j] = zl ? make_float2(we, wi) : zr ? make_float2(wi, we) : make_float2(wi, wi);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            auto c = [&](int t) { return RAG && nvalid < 8 && 2 * t + 1 - q == nvalid - 1 ? -3.f : -4.f; };
+            ca[q] = make_float2(c(0), c(2));
+            cb[q] = make_float2(c(1), c(3));
+        }
+    }
+    __device__ __forceinline__ float2 weight_a(int q, int j) const { return RAG ? wa[RAG ? q : 0][j] : q && zl ? wb[0][j] : wa[0][j]; }
+    __device__ __forceinline__ float2 weight_b(int q, int j) const { return RAG ? wb[RAG ? q : 0][j] : !q && zr ? wb[0][j] : wa[0][j]; }
+
+    // Publishes the group's edge rows of colour CC.  The grid's first and last
+    // row also go, as the other colour, into the rows just outside the grid:
+    // a missing vertical neighbour takes the cell's own value.  (Those rows
+    // weigh 0, and groups outside the grid publish nothing, so nobody else
+    // writes them.)  Every warp runs the same update; a separate form for the
+    // border rows would set the pace of the whole grid.
+    template <int CC>
+    __device__ __forceinline__ void put_edges()
+    {
+        constexpr int OC = 1 - CC;
+        if (brd) {
+#pragma unroll
+            for (int j = 0; j < L; j++) {
+                if (y0 + j == 0) {
+                    if (j > 0) e[OC][j > 0 ? j - 1 : 0] = e[CC][j];
+                    else stsq(edge_up + (OC ? edge_c : 0u), e[CC][j]);
+                }
+                if (y0 + j == H - 1) {
+                    if (j + 1 < L) e[OC][j + 1 < L ? j + 1 : j] = e[CC][j];
+                    else stsq(edge_dn + (OC ? edge_c : 0u), e[CC][j]);
+                }
+            }
+        }
+        if (gin) {
+            const unsigned a = edge_own + (CC ? edge_c : 0u);
+            stsq(a, e[CC][0]);
+            stsq(a + 16u * CL, e[CC][L - 1]);
+        }
+    }
+
+    // the other colour's cell beyond the lane's eight columns, or beyond the
+    // grid the cell's own value
+    __device__ __forceinline__ float beyond(int q, const Quad &m, const Quad &v) const
+    {
+        const float x = q ? __shfl_up_sync(0xffffffffu, m.b.y, 1) : __shfl_down_sync(0xffffffffu, m.a.x, 1);
+        return (q ? zl : zr) ? (q ? v.a.x : v.b.y) : x;
+    }
+
+    __device__ __forceinline__ Quad rhs(int c, int j) const
+    {
+        return ldsq(r_s + (c ? r_c : 0u) + 16u * (unsigned)(CL * j));
+    }
+
+    // The negated residual of row j's quad of colour CC.
+    template <int CC>
+    __device__ __forceinline__ Quad defect(int j, const Quad &eu, const Quad &ed) const
+    {
+        constexpr int OC = 1 - CC;
+        const int q = 1 - ((j ^ CC) & 1);  // the group's first row is even
+        const Quad &v = e[CC][j], &m = e[OC][j];
+        const float ex = beyond(q, m, v);
+        return quad_defect(q, v, rhs(CC, j), j > 0 ? e[OC][j > 0 ? j - 1 : 0] : eu,
+                           j + 1 < L ? e[OC][j + 1 < L ? j + 1 : j] : ed, m, ex, RAG ? ca[q] : make_float2(-4.f, -4.f),
+                           RAG ? cb[q] : make_float2(-4.f, -4.f));
+    }
+
+    // Half sweep of colour CC.  TR: mx takes the largest |update| of the tile's
+    // own cells (plane rows [olo, ohi)).
+    template <int CC, bool TR>
+    __device__ __forceinline__ void half(float &mx, int olo, int ohi)
+    {
+        constexpr int OC = 1 - CC;
+        const Quad eu = ldsq(edge_up + (OC ? edge_c : 0u));
+        const Quad ed = ldsq(edge_dn + (OC ? edge_c : 0u));
+#pragma unroll
+        for (int j = 0; j < L; j++) {
+            const int q = 1 - ((j ^ CC) & 1);
+            const Quad t = defect<CC>(j, eu, ed), v = e[CC][j];
+            const Quad nv = {__ffma2_rn(weight_a(q, j), t.a, v.a), __ffma2_rn(weight_b(q, j), t.b, v.b)};
+            if (TR && own && lr0 + j >= olo && lr0 + j < ohi) mx = fmaxf(mx, quad_max_change(v, nv));
+            e[CC][j] = nv;
+        }
+        put_edges<CC>();
+    }
+
+    template <int CC>
+    __device__ __forceinline__ float residual_of(int olo, int ohi) const
+    {
+        constexpr int OC = 1 - CC;
+        float acc = 0.f;
+        const Quad eu = ldsq(edge_up + (OC ? edge_c : 0u));
+        const Quad ed = ldsq(edge_dn + (OC ? edge_c : 0u));
+#pragma unroll
+        for (int j = 0; j < L; j++) {
+            const int o = (j ^ CC) & 1;  // offset of the quad's first cell
+            Quad r = defect<CC>(j, eu, ed);
+            if (RAG) {
+                r.a.x = o < nvalid ? r.a.x : 0.f;
+                r.b.x = o + 2 < nvalid ? r.b.x : 0.f;
+                r.a.y = o + 4 < nvalid ? r.a.y : 0.f;
+                r.b.y = o + 6 < nvalid ? r.b.y : 0.f;
+            }
+            const float s2 = fmaf(r.a.x, r.a.x, fmaf(r.b.x, r.b.x, fmaf(r.a.y, r.a.y, r.b.y * r.b.y)));
+            acc += own && lr0 + j >= olo && lr0 + j < ohi ? s2 : 0.f;
+        }
+        return acc;
+    }
+    // Sum of (r32 - L e)^2 over the lane's own cells of plane rows [olo, ohi).
+    __device__ __forceinline__ float residual(int olo, int ohi) const
+    {
+        return residual_of<0>(olo, ohi) + residual_of<1>(olo, ohi);
+    }
+};
+
+// Shared memory of a CTA: the groups' edge rows and, for each colour, one
+// row above the first group and one below the last, the -r32 planes, the landing planes of the halo quads (the same
+// shape, only halo places written) and the table of the halo quads.
+__host__ __device__ inline size_t rs_edge_quads(int CL, int NG) { return (size_t)4 * (NG + 1) * CL; }
+__host__ __device__ inline size_t rs_plane_quads(int L, int CL, int NG) { return (size_t)2 * NG * L * CL; }
+// halo quads of a tile with n own rows: the rows above and below, then the
+// lane columns left and right of the own rows
+__host__ __device__ inline int rs_halo_quads(int K, int CL, int n)
+{
+    return 4 * (2 * K) * CL + n * 4 * (K / 4);
+}
+inline size_t rs_smem(int K, int L, int CL, int NG, int n, bool exchange)
+{
+    size_t b = (rs_edge_quads(CL, NG) + rs_plane_quads(L, CL, NG)) * sizeof(Quad);
+    if (exchange) b += rs_plane_quads(L, CL, NG) * sizeof(Quad) + (size_t)rs_halo_quads(K, CL, n) * sizeof(uint2);
+    return b;
+}
+
+template <int K, int L, int CL, bool RAG>
+__global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentArgs a)
+{
+    using T = Tile<K, L, CL, RAG>;
+    constexpr int HK = 2 * K, HL = HK / 8;  // halo rows, halo lane columns
+    static_assert(K % 4 == 0, "the halo is a whole number of lane columns");
+    extern __shared__ __align__(16) float smem_f[];
+    __shared__ float s_red[32];
+    __shared__ float s_vals[kResidentCtasMax];
+    __shared__ float s_tot;
+    __shared__ double s_lim;  // squared estimate that ends the cycle
+    __shared__ unsigned s_mx[kResidentChecksMax];
+    __shared__ int s_first;
+    Ctl *ctl = a.ctl;
+    {
+        const volatile Ctl *c = ctl;
+        if ((a.cycle ? c->done : c->halt) || c->error) return;  // every CTA reads the same
+    }
+    const int done_before = ((volatile const Ctl *)ctl)->sweeps;
+    const int target0 = min(a.nsw, a.max_iter - done_before);
+    if (target0 < 1) return;
+
+    // ---- the tile and the lane's part of it
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, NW = blockDim.x >> 5, NT = blockDim.x;
+    const int G = gridDim.x, g = blockIdx.x, ty = g / a.TX, tx = g - ty * a.TX;
+    const int H2 = (a.H + 1) >> 1;  // tiles start on even rows
+    const int yb = 2 * (int)((long long)ty * H2 / a.TY), ye = min(a.H, 2 * (int)((long long)(ty + 1) * H2 / a.TY));
+    const int qb = (int)((long long)tx * a.KQ / a.TX), qe = (int)((long long)(tx + 1) * a.KQ / a.TX);
+    const int hr = a.TY > 1 ? HK : 0, hl = a.TX > 1 ? HL : 0;
+    const int n = ye - yb, nq = qe - qb, R = n + 2 * hr;
+    const int ybase = yb - hr, qbase = qb - hl;
+
+    T st;
+    st.cl = lane & (CL - 1);
+    const int h = lane / CL;
+    st.gi = w * T::G + h;
+    st.lr0 = st.gi * L;
+    st.y0 = ybase + st.lr0;
+    const int q = qbase + st.cl;
+    const bool act = st.cl < nq + 2 * hl && q >= 0 && q < a.KQ;
+    st.own = st.cl >= hl && st.cl < hl + nq;
+    st.zl = q == 0;
+    st.nvalid = min(8, a.W - 8 * q);
+    st.zr = q == a.KQ - 1 && st.nvalid == 8;
+    st.H = a.H;
+    st.setup_weights(act, R, a.w32[4], a.w32[3], a.w32[2]);
+    st.gin = st.y0 < a.H && st.y0 + L > 0;
+    st.brd = __any_sync(0xffffffffu, st.gin && (st.y0 <= 0 || st.y0 + L >= a.H));
+    st.wlo = w * T::G * L;
+    st.whi = (w + 1) * T::G * L;
+    const unsigned edge_s = (unsigned)__cvta_generic_to_shared(smem_f);
+    const unsigned grow = 16u * CL;  // bytes of one edge row
+    st.edge_c = 2u * ((unsigned)a.NG + 1u) * grow;
+    st.edge_own = edge_s + (unsigned)(st.gi * 2) * grow + 16u * st.cl;
+    st.edge_up = edge_s + (unsigned)(st.gi > 0 ? 2 * st.gi - 1 : 2 * a.NG) * grow + 16u * st.cl;
+    st.edge_dn = edge_s + (unsigned)(st.gi < a.NG - 1 ? 2 * st.gi + 2 : 2 * a.NG + 1) * grow + 16u * st.cl;
+    for (unsigned z = threadIdx.x; z < rs_edge_quads(CL, a.NG); z += NT) stsq(edge_s + 16u * z, quad_zero());
+    Quad *rp = reinterpret_cast<Quad *>(smem_f) + rs_edge_quads(CL, a.NG);
+    st.r_c = (unsigned)(a.NG * L) * grow;
+    st.r_s = (unsigned)__cvta_generic_to_shared(rp) + (unsigned)st.lr0 * grow + 16u * st.cl;
+    Quad *land = rp + rs_plane_quads(L, CL, a.NG);
+    uint2 *table = reinterpret_cast<uint2 *>(land + rs_plane_quads(L, CL, a.NG));
+    const unsigned land_s = st.r_s + 2u * st.r_c;  // the lane's place in the landing planes
+    const unsigned xplane = (unsigned)a.H * (unsigned)a.KQ;  // exchange quads of one colour
+    // rows of the lane that go out (pub) and come in (imp) at an exchange
+    unsigned pub = 0, imp = 0;
+    int halo_quads = 0;
+    if (G > 1) {
+#pragma unroll
+        for (int j = 0; j < L; j++) {
+            const int lr = st.lr0 + j, y = st.y0 + j;
+            const bool mine = st.own && lr >= hr && lr < hr + n;
+            const bool border = (lr < hr + HK && ty > 0) || (lr >= hr + n - HK && ty < a.TY - 1) ||
+                                (st.cl < 2 * hl && tx > 0) || (st.cl >= nq && tx < a.TX - 1);
+            if (mine && border && !(a.withhold && g == 0)) pub |= 1u << j;
+            if (!mine && act && lr < R && y >= 0 && y < a.H) imp |= 1u << j;
+        }
+        // every halo quad's exchange word and landing place, dealt out over
+        // the threads (the lanes that own the side columns would have 2 L
+        // serial loads each); outside the grid: ~0
+        halo_quads = rs_halo_quads(K, CL, n);
+        for (int id = threadIdx.x; id < halo_quads; id += NT) {
+            constexpr int nt = 4 * HK * CL;
+            int lr, cc, c;
+            if (id < nt) {
+                const int r = id / CL;
+                cc = id & (CL - 1);
+                c = r & 1;
+                lr = (r >> 1) < HK ? (r >> 1) : (r >> 1) + n;
+            } else {
+                const int k = id - nt, sd = k & (2 * HL - 1), r = k / (2 * HL);
+                cc = sd < HL ? sd : nq + sd;
+                c = r & 1;
+                lr = hr + (r >> 1);
+            }
+            const int y = ybase + lr, qq = qbase + cc;
+            const bool in = y >= 0 && y < a.H && qq >= 0 && qq < a.KQ && cc < nq + 2 * hl &&
+                            (id < nt ? a.TY > 1 : a.TX > 1);
+            table[id] = in ? make_uint2((unsigned)c * xplane + (unsigned)y * (unsigned)a.KQ + (unsigned)qq,
+                                        (unsigned)((c * a.NG * L + lr) * CL + cc))
+                           : make_uint2(~0u, 0u);
+        }
+    }
+
+    // ---- -r32 of the tile and its halo; e = 0
+#pragma unroll
+    for (int j = 0; j < L; j++) {
+        const int lr = st.lr0 + j, y = st.y0 + j, par = y & 1;
+        float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A;
+        if (lr < R && y >= 0 && y < a.H && act) {
+            const float *p = a.r32 + (size_t)y * a.ld + 8 * q;
+            if (a.vec && st.nvalid == 8) {
+                A = *reinterpret_cast<const float4 *>(p);
+                B = *reinterpret_cast<const float4 *>(p + 4);
+            } else {
+                float t[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) t[k] = k < st.nvalid ? p[k] : 0.f;
+                A = make_float4(t[0], t[1], t[2], t[3]);
+                B = make_float4(t[4], t[5], t[6], t[7]);
+            }
+        }
+        const Quad ev = {make_float2(-A.x, -B.x), make_float2(-A.z, -B.z)};
+        const Quad od = {make_float2(-A.y, -B.y), make_float2(-A.w, -B.w)};
+        // colour c holds the cells at offsets ((y & 1) ^ c) + 2 t
+        stsq(st.r_s + grow * (unsigned)j, par ? od : ev);
+        stsq(st.r_s + st.r_c + grow * (unsigned)j, par ? ev : od);
+    }
+    const double bnorm = ((volatile const Ctl *)ctl)->bnorm;
+    const double rstart = ((volatile const Ctl *)ctl)->rnorm;
+    if (threadIdx.x == 0) {
+        const double stop_abs = kFp32StopFrac * a.tol * bnorm, drop_abs = a.drop * rstart;
+        s_lim = fmax(stop_abs * stop_abs, drop_abs * drop_abs);
+    }
+    unsigned ep = ((volatile const Ctl *)ctl)->res_epoch;     // exchanges so far
+    unsigned ck = ((volatile const Ctl *)ctl)->res_checks;    // estimates so far
+
+    // the tile's own rows of e to global memory
+    auto store_own = [&]() {
+#pragma unroll
+        for (int j = 0; j < L; j++) {
+            const int lr = st.lr0 + j, y = st.y0 + j;
+            if (!st.own || lr < hr || lr >= hr + n) continue;
+            const Quad ev = (y & 1) ? st.e[1][j] : st.e[0][j], od = (y & 1) ? st.e[0][j] : st.e[1][j];
+            float *p = a.e + (size_t)y * a.ld + 8 * q;
+            if (a.vec && st.nvalid == 8) {
+                *reinterpret_cast<float4 *>(p) = make_float4(ev.a.x, od.a.x, ev.b.x, od.b.x);
+                *reinterpret_cast<float4 *>(p + 4) = make_float4(ev.a.y, od.a.y, ev.b.y, od.b.y);
+            } else {
+                const float t[8] = {ev.a.x, od.a.x, ev.b.x, od.b.x, ev.a.y, od.a.y, ev.b.y, od.b.y};
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k < st.nvalid) p[k] = t[k];
+            }
+        }
+    };
+
+    const bool track0 = a.gran > 0;
+    if (track0)
+        for (int t = threadIdx.x; t < kResidentChecksMax; t += NT) s_mx[t] = 0u;
+
+    int sweeps = 0, target = target0, passed = -1;
+    bool track = track0, failed = false, saved = false;
+    float last_max = 0.f;
+    for (int phase = 0;; phase++) {
+#pragma unroll
+        for (int j = 0; j < L; j++) st.e[0][j] = st.e[1][j] = quad_zero();
+        st.template put_edges<0>();
+        st.template put_edges<1>();
+        __syncthreads();
+        sweeps = 0;
+        int next_check = a.cycle ? (a.check_every + a.dep - 1) / a.dep * a.dep : 0x7fffffff;
+        int snap_at = -1, next_tr = a.gran;
+        bool pending = false, to_post = false, est_now = false;
+        for (;;) {
+            if (est_now) {
+                // an estimate of the state at `sweeps`; its partials wait in
+                // s_red for the next block barrier
+                float v = st.residual(hr, hr + n);
+                v = warp_sum_f(v);
+                if (lane == 0) s_red[w] = v;
+                est_now = false;
+                to_post = pending = true;
+                ++ck;
+                snap_at = sweeps + a.lag;
+                if (a.lag == 0) store_own();
+            }
+            const int kr = min(K, min(target, next_check) - sweeps);
+            // half sweep i relaxes the rows within 2 kr - 1 - i of the tile's
+            // own (the dependency cone); a warp further out sits it out.  The
+            // other rows outside the cone are relaxed along, and overwritten
+            // at the next exchange.
+            const int live = 2 * kr - 1 - max(hr - st.whi, st.wlo - hr - n);
+            // stretches of plain sweeps, cut where something else is due
+            for (int t = 0; t < kr;) {
+                const int s0 = sweeps + t;
+                if (track && (s0 + 1 == next_tr || s0 + 1 == target)) {
+                    float mx = 0.f;
+                    if (2 * t < live) st.template half<0, true>(mx, hr, hr + n);
+                    __syncthreads();
+                    if (2 * t + 1 < live) st.template half<1, true>(mx, hr, hr + n);
+                    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                    if (lane == 0 && mx > 0.f) atomicMax(&s_mx[s0 / a.gran], __float_as_uint(mx));
+                    __syncthreads();
+                    if (s0 + 1 == next_tr) next_tr += a.gran;
+                    t++;
+                    continue;
+                }
+                int end = to_post ? t + 1 : kr;
+                if (track) end = min(end, min(next_tr, target) - 1 - sweeps);
+                if (snap_at > s0) end = min(end, snap_at - sweeps);
+                float none = 0.f;
+                int i = 2 * t;
+#pragma unroll 1
+                do {
+                    if (i < live) st.template half<0, false>(none, 0, 0);
+                    __syncthreads();
+                    if (i + 1 < live) st.template half<1, false>(none, 0, 0);
+                    __syncthreads();
+                    i += 2;
+                } while (i < 2 * end);
+                t = end;
+                if (to_post) {
+                    if (w == 0) {
+                        float x = lane < NW ? s_red[lane] : 0.f;
+                        x = warp_sum_f(x);
+                        if (lane == 0) {
+                            if (G == 1) s_tot = x;
+                            else if (!(a.withhold && g == 0)) rs_st1(a.part + (size_t)(ck & 1) * G + g, rs_word(x, ck));
+                        }
+                    }
+                    to_post = false;
+                }
+                if (sweeps + t == snap_at && a.lag > 0 && t < kr) store_own();
+            }
+            sweeps += kr;
+            const bool last = sweeps >= target;
+            const bool decide = pending && sweeps >= snap_at;
+            if (decide && G > 1) {
+                // the partials of every CTA, posted at least half a sweep ago
+                for (int t = threadIdx.x; t < G; t += NT) {
+                    const unsigned long long *p = a.part + (size_t)(ck & 1) * G + t;
+                    long long it = 0;
+                    unsigned long long v = rs_ld1(p);
+                    while ((unsigned)(v >> 32) != ck && !failed) {
+                        if (!rs_again(a, it)) failed = true;
+                        v = rs_ld1(p);
+                    }
+                    s_vals[t] = __uint_as_float((unsigned)v);
+                }
+            }
+            if (!last && G > 1) {
+                ++ep;
+                Words *xb = reinterpret_cast<Words *>(a.xb) + (size_t)(ep & 1) * 2 * xplane;
+                // ---- own border quads out
+                if (pub) {
+                    Words *p = xb + ((long)st.y0 * a.KQ + q);
+#pragma unroll
+                    for (int j = 0; j < L; j++, p += a.KQ)
+                        if (pub >> j & 1u) {
+                            rs_st4(p, rs_words(st.e[0][j], ep));
+                            rs_st4(p + xplane, rs_words(st.e[1][j], ep));
+                        }
+                }
+                // ---- halo quads in
+                constexpr int U = L <= 4 ? 4 : 2;
+                for (int id0 = threadIdx.x; id0 < halo_quads; id0 += U * NT) {
+                    uint2 at[U];
+                    bool any = false;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        at[u] = id0 + u * NT < halo_quads ? table[id0 + u * NT] : make_uint2(~0u, 0u);
+                        any = any || at[u].x != ~0u;
+                    }
+                    long long it = 0;
+                    while (any && !failed) {
+                        any = false;
+                        Words v[U];
+#pragma unroll
+                        for (int u = 0; u < U; u++)
+                            if (at[u].x != ~0u) v[u] = rs_ld4(xb + at[u].x);
+#pragma unroll
+                        for (int u = 0; u < U; u++)
+                            if (at[u].x != ~0u) {
+                                if (rs_fresh(v[u], ep)) {
+                                    land[at[u].y] = rs_quad(v[u]);
+                                    at[u].x = ~0u;
+                                } else {
+                                    any = true;
+                                }
+                            }
+                        if (any && !rs_again(a, it)) failed = true;
+                    }
+                }
+                __syncthreads();
+                if (imp) {
+#pragma unroll
+                    for (int j = 0; j < L; j++)
+                        if (imp >> j & 1u) {
+                            st.e[0][j] = ldsq(land_s + grow * (unsigned)j);
+                            st.e[1][j] = ldsq(land_s + st.r_c + grow * (unsigned)j);
+                        }
+                }
+                st.template put_edges<0>();
+                st.template put_edges<1>();
+            }
+            if (G > 1 ? __syncthreads_or(failed) : 0) { failed = true; break; }
+            if (decide) {
+                if (G > 1) {
+                    // every CTA sums the same partials in the same order
+                    if (w == 0) {
+                        float x = 0.f;
+                        for (int t = lane; t < G; t += 32) x += s_vals[t];
+                        x = warp_sum_f(x);
+                        if (lane == 0) s_tot = x;
+                    }
+                    __syncthreads();
+                }
+                pending = false;
+                const double est2 = (double)s_tot;
+                if (est2 <= s_lim) {
+                    if (sweeps > snap_at) saved = true;  // e of sweep snap_at was written then
+                    sweeps = snap_at;
+                    break;
+                }
+                __syncthreads();
+            }
+            if (last) break;
+            if (sweeps >= next_check) {
+                est_now = true;
+                next_check = (sweeps + a.check_every + a.dep - 1) / a.dep * a.dep;
+            }
+        }
+        if (failed || !track) break;
+        // ---- max-update stop: the first tracked sweep that passed
+        const int np = (target - 1) / a.gran + 1;
+        __syncthreads();
+        for (int t = threadIdx.x; t < np; t += NT)
+            if (s_mx[t]) atomicMax(&a.gmax[t], s_mx[t]);
+        if (threadIdx.x == 0) s_first = np;
+        __syncthreads();
+        if (G > 1) {
+            if (threadIdx.x == 0 && !(a.withhold && g == 0)) {
+                __threadfence();
+                atomicAdd(a.bar, 1u);
+            }
+            if (threadIdx.x == 0) {
+                long long it = 0;
+                while (rs_ld_acquire(a.bar) < (unsigned)G && !failed)
+                    if (!rs_again(a, it)) failed = true;
+            }
+            if (__syncthreads_or(failed)) { failed = true; break; }
+        } else {
+            __threadfence();
+            __syncthreads();
+        }
+        for (int t = threadIdx.x; t < np; t += NT)
+            if ((double)__uint_as_float(__ldcg(a.gmax + t)) < a.tol) atomicMin(&s_first, t);
+        __syncthreads();
+        const int first = s_first;
+        last_max = __uint_as_float(__ldcg(a.gmax + min(first, np - 1)));
+        if (first < np) {
+            passed = min((first + 1) * a.gran, target);
+            if (passed < target) {
+                target = passed;
+                track = false;
+                continue;  // once more from e = 0, up to the sweep that passed
+            }
+        }
+        break;
+    }
+    if (failed) return;  // the error word is set; the solve reports it
+    if (!saved) store_own();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
+            volatile Ctl *c = ctl;
+            const int s = done_before + sweeps;
+            c->sweeps = s;
+            if (track0) {
+                c->last_max = (double)last_max;
+                if (passed >= 0) {
+                    c->converged = 1;
+                    c->halt = 1;
+                }
+                const int np = (target0 - 1) / a.gran + 1;
+                for (int t = 0; t < np; t++) ((volatile unsigned *)a.gmax)[t] = 0u;
+                *(volatile unsigned *)a.bar = 0u;
+            }
+            if (s >= a.max_iter) c->halt = 1;
+            c->res_epoch = ep;
+            c->res_checks = ck;
+            c->blocks_done = 0;
+            __threadfence();
+        }
+    }
+}
+
+template <int K, bool RAG>
+const void *rs_kernel_l(int L, int CL)
+{
+    if (CL == 8) return K == 4 && L == 2 ? (const void *)k_sor_resident<4, 2, 8, RAG> : nullptr;
+    if (CL != 16) return nullptr;
+    switch (L) {
+    case 2: return (const void *)k_sor_resident<K, 2, 16, RAG>;
+    case 4: return (const void *)k_sor_resident<K, 4, 16, RAG>;
+    }
+    if constexpr (!RAG) {
+        // (partial lane columns need twice the weight registers)
+        switch (L) {
+        case 6: return (const void *)k_sor_resident<K, 6, 16, RAG>;
+        case 8: return (const void *)k_sor_resident<K, 8, 16, RAG>;
+        }
+    }
+    return nullptr;
+}
+
+const void *rs_kernel(int K, int L, int CL, bool rag)
+{
+    if (K == 4) return rag ? rs_kernel_l<4, true>(L, CL) : rs_kernel_l<4, false>(L, CL);
+    if (K == 8) return rag ? rs_kernel_l<8, true>(L, CL) : rs_kernel_l<8, false>(L, CL);
+    return nullptr;
+}
+
+}  // namespace
+
+int resident_plan(int dev, int W, int H, ResidentPlan *plan)
+{
+    if (W < 16 || H < 16) return PCD_BAD_ARG;
+    int sms = 0, max_smem = 0, coop = 0;
+    PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    PCD_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    PCD_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return PCD_BAD_ARG;
+    sms = std::min(sms, kResidentCtasMax);
+    const int KQ = (W + 7) / 8, H2 = (H + 1) / 2;
+    ResidentPlan best;
+    double best_t = 0.0;
+    for (int K : {4, 8})
+        for (int CL : {8, 16})
+            for (int L : {2, 4, 6, 8}) {
+                if (!rs_kernel(K, L, CL, W % 8 != 0)) continue;
+                const int G = 32 / CL, HK = 2 * K, HL = HK / 8;
+                for (int TX = 1; TX <= std::min(sms, KQ); TX++) {
+                    const int nq = (KQ + TX - 1) / TX;
+                    if (nq + (TX > 1 ? 2 * HL : 0) > CL) continue;
+                    if (TX > 1 && KQ / TX < HL) break;
+                    // most tile rows whose tiles hold a neighbour's whole halo
+                    int tymax = sms / TX;
+                    while (tymax > 1 && 2 * (H2 / tymax) - H % 2 < HK) tymax--;
+                    for (int TY : {tymax, 1}) {
+                        const int n = std::min(H, 2 * ((H2 + TY - 1) / TY)), R = n + (TY > 1 ? 2 * HK : 0);
+                        const int NW = std::max(4, ((R + L - 1) / L + G - 1) / G), NG = NW * G;
+                        if (NW > rs_warps(L)) continue;
+                        const size_t smem = rs_smem(K, L, CL, NG, n, TX * TY > 1);
+                        if (smem + 8192 > (size_t)max_smem) continue;
+                        // ns of a sweep.  Without exchanges (one-tile grids,
+                        // 1, 2 and 3 warps a scheduler) it measured, L = 2:
+                        // 284, 376, 468; L = 4: 362, 504, 650; L = 6: 546,
+                        // 760, 1027; L = 8: 796, 1007, 1270.  An exchange
+                        // measured 1.2-1.4 us with L = 2 and 1.8-2.3 us
+                        // above; warps outside the cone save 10-15%.
+                        const int wps = (NW + 3) / 4;
+                        double t = (L == 2 ? 284 : L == 4 ? 362 : L == 6 ? 546 : 796) +
+                                   (wps - 1) * (L == 2 ? 92 : L == 4 ? 144 : 240);
+                        if (TX * TY > 1) t = (K == 8 ? 0.85 : 0.9) * t + (L == 2 ? 1300.0 : 2000.0) / K;
+                        if (best.L == 0 || t < best_t) {
+                            best_t = t;
+                            best.K = K;
+                            best.L = L;
+                            best.CL = CL;
+                            best.TX = TX;
+                            best.TY = TY;
+                            best.NW = NW;
+                            best.NG = NG;
+                            best.R = R;
+                            best.KQ = KQ;
+                            best.smem = smem;
+                            best.xb_bytes = TX * TY > 1 ? (size_t)4 * H * KQ * 32 : 0;
+                        }
+                    }
+                }
+            }
+    if (!best.L) return PCD_BAD_ARG;
+    *plan = best;
+    return PCD_OK;
+}
+
+int launch_resident(ResidentArgs &a, const ResidentPlan &p, cudaStream_t s)
+{
+    const void *fn = rs_kernel(p.K, p.L, p.CL, a.W % 8 != 0);
+    if (!fn) {
+        set_error("resident SOR: no kernel for this plan");
+        return PCD_BAD_ARG;
+    }
+    a.KQ = p.KQ;
+    a.TX = p.TX;
+    a.TY = p.TY;
+    a.NG = p.NG;
+    a.R = p.R;
+    a.vec = a.ld % 4 == 0;
+    PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    void *params[] = {&a};
+    if (p.TX * p.TY == 1) PCD_CUDA(cudaLaunchKernel(fn, dim3(1), dim3(32 * p.NW), params, p.smem, s));
+    else PCD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.TX * p.TY), dim3(32 * p.NW), params, p.smem, s));
+    count_launches(1);
+    return PCD_OK;
+}
+
+}  // namespace pcd
