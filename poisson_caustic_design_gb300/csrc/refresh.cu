@@ -1,0 +1,291 @@
+// refresh.cu -- the FP64 passes of a solve (sm_103a).
+//
+// This part runs one FP64 operation per SM and half clock (1/56 of the FP32
+// rate), so these passes are bound by the number of FP64 instructions, not by
+// memory: 24 bytes read and 12 written a cell take 80 us at 4096^2, eight FP64
+// operations a cell 240.
+//
+// k_refresh folds the FP32 correction into the potential and renews the
+// residual in one pass:  xi = phi + e,  r = b - (sum of neighbours - cnt xi).
+// A warp walks down a strip of 30 columns (lanes 1 to 30; lanes 0 and 31 the
+// columns beside it).  With D(x, y) = xi(x+1, y) + xi(x, y+1) the neighbour sum
+// of (x, y) is D(x-1, y-1) + D(x, y), so a cell costs two additions for it
+// instead of three, one shuffle each way, and xi is formed once:  widen e, add,
+// D, D + D, multiply-add, subtract, multiply-add for the norm, narrow r.  (One
+// thread a cell forming xi of all five cells and counting neighbours in FP64
+// took about 24.)  Cells outside the grid read 0.
+//
+// xi goes to the other of two buffers, because a neighbouring strip may still
+// need the old phi; the control block says which one holds the potential.
+#include <algorithm>
+
+#include "refresh.cuh"
+
+namespace pcd {
+
+namespace {
+
+constexpr int kRefreshWarps = 4;      // warps of a block: one or two blocks fill the FP64 pipes of an SM
+constexpr int kRefreshCols = 30;      // columns a warp owns
+constexpr int kStartThreads = 256;
+
+__device__ __forceinline__ int rf_load(const int *p) { return *(const volatile int *)p; }
+
+__device__ __forceinline__ bool is_nan_bits(double v)
+{
+    return ((unsigned long long)__double_as_longlong(v) << 1) > 0xffe0000000000000ull;
+}
+
+// Running max of |r| on the bit patterns (they order like the values; NaN
+// does not raise it), off the FP64 pipe.
+__device__ __forceinline__ unsigned long long max_abs_bits(unsigned long long m, double r)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+    return b > m && b <= 0x7ff0000000000000ull ? b : m;
+}
+
+__device__ __forceinline__ bool rf_last_block(Ctl *ctl, int nblk)
+{
+    __shared__ bool is_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        is_last = atomicAdd(&ctl->blocks_done_r, 1u) == (unsigned)nblk - 1u;
+    }
+    __syncthreads();
+    if (is_last) __threadfence();
+    return is_last;
+}
+
+// Sums the blocks' partials in a fixed order (every thread of the block
+// calls); thread 0 has the result.
+__device__ void rf_sum_partials(const double *partials, int nblk, double (&v)[3])
+{
+    v[0] = v[1] = v[2] = 0.0;
+    for (int k = threadIdx.x; k < nblk; k += blockDim.x) {
+        v[0] += __ldcg(partials + 3 * k);
+        v[1] += __ldcg(partials + 3 * k + 1);
+        v[2] = nan_skip_max(v[2], __ldcg(partials + 3 * k + 2));
+    }
+    block_reduce<3, 4u>(v);
+}
+
+__global__ void __launch_bounds__(32 * kRefreshWarps)
+    k_refresh(const RefreshJob *__restrict__ jobs, RefreshJob one, int njobs, double tol)
+{
+    RefreshJob J = one;
+    if (jobs) {
+        int lo = 0, hi = njobs - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(&jobs[mid].blk0) <= (int)blockIdx.x) lo = mid;
+            else hi = mid - 1;
+        }
+        J = jobs[lo];
+    }
+    Ctl *ctl = J.ctl;
+    if (rf_load(&ctl->done) || rf_load(&ctl->error) || rf_load(&ctl->nan_cells)) return;
+    const int side = rf_load(&ctl->phi_side);
+    const double *__restrict__ pin = side ? J.phi2 : J.phi;
+    double *__restrict__ pout = side ? J.phi : J.phi2;
+    const float *__restrict__ e = rf_load(&ctl->stream_out) ? J.e1 : J.e0;
+    const int W = J.W, H = J.H, ld = J.ld;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int strips = (W + kRefreshCols - 1) / kRefreshCols, pieces = (H + J.rows - 1) / J.rows;
+    double acc = 0.0;
+    unsigned long long mbits = 0ull;
+    for (int item = ((int)blockIdx.x - J.blk0) * kRefreshWarps + w; item < strips * pieces;
+         item += J.nblk * kRefreshWarps) {
+        const int piece = item / strips, strip = item - piece * strips;
+        const int x = strip * kRefreshCols + lane - 1;
+        const bool in = x >= 0 && x < W, own = in && lane >= 1 && lane <= kRefreshCols;
+        const int y0 = piece * J.rows, y1 = min(y0 + J.rows, H);
+        const double c2 = (double)((x > 0) + (x < W - 1) + 2), c1 = c2 - 1.0, c0 = c2 - 2.0;
+        const size_t at = in ? (size_t)x : 0;
+        auto load = [&](int y, double &p, float &ev) {
+            const bool ok = in && y >= 0 && y < H;
+            const size_t i = (size_t)(ok ? y : 0) * ld + at;
+            p = ok ? pin[i] : 0.0;
+            ev = ok ? e[i] : 0.f;
+        };
+        // rows y0 - 1, y0 and y0 + 1; then one row ahead of the one in hand
+        double pa, pb, pc, bc;
+        float ea, eb, ec;
+        load(y0 - 1, pa, ea);
+        load(y0, pb, eb);
+        load(y0 + 1, pc, ec);
+        bc = own ? J.b[(size_t)y0 * ld + at] : 0.0;
+        const double xa = pa + (double)ea;
+        double xc = pb + (double)eb;
+        // D(x, y0 - 1)
+        double dp = __shfl_down_sync(0xffffffffu, xa, 1) + xc;
+        for (int y = y0; y < y1; y++) {
+            double pn, bn = 0.0;
+            float en;
+            load(y + 2, pn, en);
+            if (own && y + 1 < y1) bn = J.b[(size_t)(y + 1) * ld + at];
+            const double xn = pc + (double)ec;
+            const double d = __shfl_down_sync(0xffffffffu, xc, 1) + xn;
+            const double sum = __shfl_up_sync(0xffffffffu, dp, 1) + d;
+            const bool top = y > 0, bot = y < H - 1;
+            const double cnt = top && bot ? c2 : top || bot ? c1 : c0;
+            const double r = fma(cnt, xc, bc) - sum;
+            if (own) {
+                const size_t i = (size_t)y * ld + at;
+                pout[i] = xc;
+                J.r32[i] = (float)r;
+                acc = fma(r, r, acc);
+                mbits = max_abs_bits(mbits, r);
+            }
+            dp = d;
+            xc = xn;
+            pc = pn;
+            ec = en;
+            bc = bn;
+        }
+    }
+    double v[3] = {acc, 0.0, __longlong_as_double((long long)mbits)};
+    block_reduce<3, 4u>(v);
+    if (threadIdx.x == 0) {
+        double *p = J.partials + 3 * ((int)blockIdx.x - J.blk0);
+        p[0] = v[0];
+        p[1] = 0.0;
+        p[2] = v[2];
+    }
+    if (!rf_last_block(ctl, J.nblk)) return;
+    rf_sum_partials(J.partials, J.nblk, v);
+    if (threadIdx.x == 0) {
+        volatile Ctl *c = ctl;
+        const double rn = sqrt(v[0]), bn = c->bnorm, rel = bn > 0.0 ? rn / bn : rn;
+        c->rnorm = rn;
+        c->rmax = v[2];
+        c->rel = rel;
+        c->checks = c->checks + 1;
+        if (tol >= 0.0 && rel <= tol) {
+            c->converged = 1;
+            c->halt = 1;
+        }
+        if (c->halt) c->done = 1;
+        c->phi_side = side ^ 1;
+        c->stream_out = 0;
+        c->blocks_done_r = 0;
+        __threadfence();
+    }
+}
+
+__global__ void __launch_bounds__(kStartThreads) k_phi_settle(RefreshJob J)
+{
+    if (!rf_load(&J.ctl->phi_side)) return;
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < J.W; x += gridDim.x * blockDim.x)
+        for (int y = blockIdx.y; y < J.H; y += gridDim.y) J.phi[(size_t)y * J.ld + x] = J.phi2[(size_t)y * J.ld + x];
+}
+
+template <bool ZERO>
+__global__ void __launch_bounds__(kStartThreads)
+    k_start(const double *__restrict__ b, double *__restrict__ phi, uint8_t *__restrict__ mask,
+            double *__restrict__ r64, float *__restrict__ r32, Ctl *ctl, double *partials, SolveArgs a, int test)
+{
+    const int W = a.W, H = a.H, ld = a.ld;
+    double v[3] = {0.0, 0.0, 0.0};
+    unsigned long long mbits = 0ull;
+    int nans = 0;
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < W; x += gridDim.x * blockDim.x) {
+        for (int y = blockIdx.y; y < H; y += gridDim.y) {
+            const size_t i = (size_t)y * ld + x;
+            const bool l = x > 0 && !is_nan_bits(b[i - 1]), u = y > 0 && !is_nan_bits(b[i - ld]);
+            const bool rt = x < W - 1 && !is_nan_bits(b[i + 1]), d = y < H - 1 && !is_nan_bits(b[i + ld]);
+            const double bi = b[i];
+            const bool nan = is_nan_bits(bi);
+            mask[i] = (uint8_t)((l ? 1 : 0) | (u ? 2 : 0) | (rt ? 4 : 0) | (d ? 8 : 0) | (nan ? 16 : 0));
+            double r = bi;
+            if (ZERO) {
+                phi[i] = 0.0;
+            } else if (!nan) {
+                double sum = 0.0;
+                if (l) sum += phi[i - 1];
+                if (u) sum += phi[i - ld];
+                if (rt) sum += phi[i + 1];
+                if (d) sum += phi[i + ld];
+                r = bi - (sum - (double)((int)l + (int)u + (int)rt + (int)d) * phi[i]);
+            }
+            if (r64 && !nan) r64[i] = r;
+            if (r32) r32[i] = (float)r;
+            if (nan) {
+                nans++;
+                continue;
+            }
+            if (!ZERO) v[0] = fma(r, r, v[0]);
+            v[1] = fma(bi, bi, v[1]);
+            mbits = max_abs_bits(mbits, r);
+        }
+    }
+    if (ZERO) v[0] = v[1];
+    if (nans) atomicAdd(&ctl->nan_cells, nans);
+    v[2] = __longlong_as_double((long long)mbits);
+    block_reduce<3, 4u>(v);
+    const int blk = blockIdx.y * gridDim.x + blockIdx.x, nblk = gridDim.x * gridDim.y;
+    if (threadIdx.x == 0) {
+        partials[3 * blk] = v[0];
+        partials[3 * blk + 1] = v[1];
+        partials[3 * blk + 2] = v[2];
+    }
+    if (!rf_last_block(ctl, nblk)) return;
+    rf_sum_partials(partials, nblk, v);
+    if (threadIdx.x == 0) {
+        volatile Ctl *c = ctl;
+        const double rn = sqrt(v[0]), bn = sqrt(v[1]), rel = bn > 0.0 ? rn / bn : rn;
+        c->rnorm = rn;
+        c->bnorm = bn;
+        c->rmax = v[2];
+        c->rel = rel;
+        c->checks = c->checks + 1;
+        if (test && rel <= a.tol) {
+            c->converged = 1;
+            c->halt = 1;
+            c->done = 1;
+        }
+        c->blocks_done_r = 0;
+        __threadfence();
+    }
+}
+
+}  // namespace
+
+int refresh_shape(int W, int H, int cap, int *rows)
+{
+    const int strips = ceil_div(W, kRefreshCols);
+    // a piece's two rows of overlap cost a quarter of a row's work each; the
+    // FP64 pipes want 4 warps an SM, and twice that to hide the loads
+    int r = 32;
+    while (r > 8 && (long)strips * ceil_div(H, r) < 152L * 2 * kRefreshWarps) r >>= 1;
+    *rows = r;
+    return std::max(1, std::min(cap, ceil_div((long)strips * ceil_div(H, r), kRefreshWarps)));
+}
+
+int launch_refresh(const RefreshJob *jobs, const RefreshJob &one, int njobs, int blocks, double tol, cudaStream_t s)
+{
+    k_refresh<<<blocks, 32 * kRefreshWarps, 0, s>>>(jobs, one, njobs, tol);
+    PCD_LAUNCHED(1);
+    return PCD_OK;
+}
+
+int launch_phi_settle(const RefreshJob &job, cudaStream_t s)
+{
+    const int gx = std::min(ceil_div(job.W, kStartThreads), 2432);
+    k_phi_settle<<<dim3(gx, std::max(1, std::min(job.H, 2432 / gx))), kStartThreads, 0, s>>>(job);
+    PCD_LAUNCHED(1);
+    return PCD_OK;
+}
+
+int launch_start(const double *b, double *phi, uint8_t *mask, double *r64, float *r32, Ctl *ctl, double *partials,
+                 int max_partials, const SolveArgs &a, bool zero, bool test, cudaStream_t s)
+{
+    const int gx = std::min(ceil_div(a.W, kStartThreads), max_partials);
+    const dim3 grid(gx, std::max(1, std::min(a.H, max_partials / gx)));
+    if (zero) k_start<true><<<grid, kStartThreads, 0, s>>>(b, phi, mask, r64, r32, ctl, partials, a, test ? 1 : 0);
+    else k_start<false><<<grid, kStartThreads, 0, s>>>(b, phi, mask, r64, r32, ctl, partials, a, test ? 1 : 0);
+    PCD_LAUNCHED(1);
+    return PCD_OK;
+}
+
+}  // namespace pcd

@@ -32,6 +32,7 @@
 #include "sor_cluster.cuh"
 #include "sor_blocks.cuh"
 #include "sor_resident.cuh"
+#include "refresh.cuh"
 
 namespace pcd {
 
@@ -640,6 +641,26 @@ int launch_stripes(T *phi, const T *rhs, Ctl *ctl, const SolveArgs &a, int R, in
     return PCD_OK;
 }
 
+// The FP64 refresh of a single solve: the potential alternates between phi and
+// the workspace's r64.
+RefreshJob refresh_job(const SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a)
+{
+    RefreshJob j{};
+    j.b = b;
+    j.phi = phi;
+    j.phi2 = ws.r64;
+    j.e0 = ws.e32;
+    j.e1 = ws.e32b;
+    j.r32 = ws.r32;
+    j.ctl = ws.ctl;
+    j.partials = ws.partials;
+    j.W = a.W;
+    j.H = a.H;
+    j.ld = a.ld;
+    j.nblk = refresh_shape(a.W, a.H, kResidualBlocksMax, &j.rows);
+    return j;
+}
+
 // Enqueues one chunk of `sweeps` sweeps (plus the checks that follow them) on s.
 template <bool MASKED>
 int enqueue_chunk(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, int precision,
@@ -675,13 +696,14 @@ int enqueue_chunk(SolverWorkspace &ws, const double *b, double *phi, const Solve
             const float *ein = (k & 1) ? ws.e32b : ws.e32;
             float *eout = (k & 1) ? ws.e32 : ws.e32b;
             const int nsw = std::min(sp.tile_sweeps, sweeps - done);
-            PCD_TRY(launch_tile(sp.tile, ein, eout, ws.r32, ws.ctl, a, nsw, (k & 1) ? 0 : 1, track, s));
+            PCD_TRY(launch_tile(sp.tile, ein, eout, ws.r32, ws.ctl, a, nsw, (k & 1) ? 0 : 1, track, k == 0, s));
             done += nsw;
             n++;
         }
-        k_stream_settle<<<rblocks, kThreads, 0, s>>>(ws.e32, ws.e32b, ws.ctl, a);
-        n++;
-        sweeps = 0;
+        PCD_TRY(launch_refresh(nullptr, refresh_job(ws, b, phi, a), 1, refresh_job(ws, b, phi, a).nblk,
+                               a.stop == PCD_STOP_REL_RESIDUAL ? a.tol : -1.0, s));
+        *nodes = n + 1;
+        return PCD_OK;
     }
     if (!MASKED && sched == PCD_SCHED_STREAM) {
         // launch k reads buffer k&1 and writes the other (two sweeps per
@@ -971,12 +993,8 @@ int solve_cluster(SolverWorkspace &ws, const double *b, double *phi, const Solve
                   const ClusterPlan &plan, pcd_solve_stats *stats, cudaStream_t s)
 {
     const int rblocks = grid_blocks((long)a.W * a.H);
+    // (r32 and the norms of the initial guess are the start's)
     PCD_CUDA(cudaMemsetAsync(ws.e32, 0, sizeof(float) * (size_t)a.H * a.ld, s));
-    // r32 = b - L phi0; ||b||; stop test on the initial guess
-    k_refine_residual<false><<<rblocks, kThreads, 0, s>>>(phi, ws.e32, b, ws.mask, ws.r32, ws.ctl, ws.partials, a, 1);
-    PCD_LAUNCHED(1);
-    k_refine_update<<<rblocks, kThreads, 0, s>>>(phi, ws.e32, ws.ctl, a);
-    PCD_LAUNCHED(1);
 
     ClusterArgs ca{};
     ca.W = a.W; ca.H = a.H; ca.ld = a.ld; ca.khp = plan.khp;
@@ -1136,9 +1154,11 @@ int resident_rule(SolverWorkspace &ws, const SolveArgs &a, const pcd_solve_opts 
 // Mixed precision on resident tiles: launches of [FP32 sweeps, FP64 residual
 // refresh, phi += e] until the stop test passes.  The next launch is enqueued
 // before the previous one's control block is read; a launch after the stop
-// returns at once.
+// returns at once.  The NaN count of b is read with the first control block:
+// where there are any nothing has been done (*nans tells the caller).
 int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const pcd_solve_opts &o,
-                   const ResidentPlan &plan, const ResidentRule &rule, pcd_solve_stats *stats, cudaStream_t s)
+                   const ResidentPlan &plan, const ResidentRule &rule, pcd_solve_stats *stats, int *nans,
+                   cudaStream_t s)
 {
     const int G = plan.TX * plan.TY;
     const size_t part_at = plan.xb_bytes, gmax_at = part_at + 2 * (size_t)G * sizeof(unsigned long long);
@@ -1152,15 +1172,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     }
     // epochs start at 0 in every solve: no word of an earlier one may match
     PCD_CUDA(cudaMemsetAsync(ws.rx, 0, need, s));
-    const int rblocks = grid_blocks((long)a.W * a.H);
-    PCD_CUDA(cudaMemsetAsync(ws.e32, 0, sizeof(float) * (size_t)a.H * a.ld, s));
-    k_refine_residual<false><<<rblocks, kThreads, 0, s>>>(phi, ws.e32, b, ws.mask, ws.r32, ws.ctl, ws.partials, a, 1);
-    PCD_LAUNCHED(1);
-    if (rule.cycle) {
-        // (as the cluster schedule: a passing initial guess is done here)
-        k_refine_update<<<rblocks, kThreads, 0, s>>>(phi, ws.e32, ws.ctl, a);
-        PCD_LAUNCHED(1);
-    }
+    const RefreshJob job = refresh_job(ws, b, phi, a);
 
     ResidentArgs ra{};
     ra.W = a.W; ra.H = a.H; ra.ld = a.ld;
@@ -1194,10 +1206,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
             return PCD_TIMEOUT;
         }
         PCD_TRY(launch_resident(ra, plan, s));
-        k_refine_residual<false><<<rblocks, kThreads, 0, s>>>(phi, ws.e32, b, ws.mask, ws.r32, ws.ctl, ws.partials, a, 0);
-        PCD_LAUNCHED(1);
-        k_refine_update<<<rblocks, kThreads, 0, s>>>(phi, ws.e32, ws.ctl, a);
-        PCD_LAUNCHED(1);
+        PCD_TRY(launch_refresh(nullptr, job, 1, job.nblk, a.stop == PCD_STOP_REL_RESIDUAL ? a.tol : -1.0, s));
         const int slot = (int)(launched & 1);
         PCD_CUDA(cudaMemcpyAsync(&ws.ctl_host[slot], ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
         PCD_CUDA(cudaEventRecord(ws.ev[slot], s));
@@ -1205,14 +1214,17 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
         if (launched >= 2) {
             const int prev = (int)((launched - 2) & 1);
             PCD_CUDA(cudaEventSynchronize(ws.ev[prev]));
-            if (ws.ctl_host[prev].done || ws.ctl_host[prev].error) finished = true;
+            const Ctl &c = ws.ctl_host[prev];
+            if (c.done || c.error || c.nan_cells) finished = true;
         }
     }
+    PCD_TRY(launch_phi_settle(job, s));
     PCD_CUDA(cudaEventRecord(ws.k1, s));
     PCD_CUDA(cudaEventRecord(ws.t1, s));
     PCD_CUDA(cudaMemcpyAsync(&ws.ctl_host[0], ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     PCD_CUDA(cudaStreamSynchronize(s));
     const Ctl &c = ws.ctl_host[0];
+    *nans = c.nan_cells;
     if (c.error) {
         set_error("resident SOR: a bounded device wait gave up (status " + std::to_string(c.error) + ")");
         return c.error;
@@ -1384,18 +1396,20 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     PCD_CUDA(cudaEventRecord(ws.t0, s));
     PCD_CUDA(cudaMemsetAsync(ws.ctl, 0, sizeof(Ctl), s));
     const int rblocks = grid_blocks((long)W * H);
-    k_mask<<<rblocks, kThreads, 0, s>>>(b, ws.mask, W, H, ld, ws.ctl);
-    PCD_LAUNCHED(1);
-    if (!o.warm_start) {
-        k_fill<<<rblocks, kThreads, 0, s>>>(phi, W, H, ld, 0.0);
-        PCD_LAUNCHED(1);
+    ResidentPlan rp;
+    ResidentRule rule;
+    const int resident = a.max_iter > 0 ? resident_rule(ws, a, o, &rp, &rule) : PCD_BAD_ARG;
+    if (resident != PCD_OK && resident != PCD_BAD_ARG) return resident;
+    // mask, initial FP64 residual and norms (valid with or without NaN cells);
+    // r64 for the mixed schedules that carry the residual on
+    PCD_TRY(launch_start(b, phi, ws.mask, precision == PCD_PREC_MIXED && resident != PCD_OK ? ws.r64 : nullptr,
+                         precision == PCD_PREC_MIXED ? ws.r32 : nullptr, ws.ctl, ws.partials, kResidualBlocksMax, a,
+                         !o.warm_start, a.stop == PCD_STOP_REL_RESIDUAL, s));
+    if (resident == PCD_OK) {
+        int nans = 0;
+        const int st = solve_resident(ws, b, phi, a, o, rp, rule, stats, &nans, s);
+        if (!nans) return st;
     }
-    // Initial FP64 residual (masked form: valid with or without NaN cells);
-    // it also yields ||b|| and, for the mixed form, the FP64 residual r64.
-    k_residual64<true><<<rblocks, kThreads, 0, s>>>(phi, b, ws.mask, ws.ctl, ws.partials, a,
-                                                   a.stop == PCD_STOP_REL_RESIDUAL, 1, 0,
-                                                   precision == PCD_PREC_MIXED ? ws.r64 : nullptr);
-    PCD_LAUNCHED(1);
     PCD_CUDA(cudaMemcpyAsync(ws.ctl_host, ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     PCD_CUDA(cudaStreamSynchronize(s));
     const int masked = ws.ctl_host[0].nan_cells > 0 ? 1 : 0;
@@ -1420,13 +1434,6 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
                 if ((st = blocks_plan(ws.dev, W, H, K, mixed, &bp)) == PCD_OK) break;
         if (st == PCD_OK) return solve_blocks(ws, b, phi, a, precision, o, bp, stats, s);
     }
-    if (!done_already && !masked && precision == PCD_PREC_MIXED) {
-        ResidentPlan rp;
-        ResidentRule rule;
-        const int st = resident_rule(ws, a, o, &rp, &rule);
-        if (st == PCD_OK) return solve_resident(ws, b, phi, a, o, rp, rule, stats, s);
-        if (st != PCD_BAD_ARG) return st;
-    }
     if (!done_already && !masked && precision == PCD_PREC_MIXED && a.stop == PCD_STOP_REL_RESIDUAL &&
         (o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_CLUSTER)) {
         ClusterPlan plan{};
@@ -1449,14 +1456,6 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         int one = 1;
         PCD_CUDA(cudaMemcpyAsync(&ws.ctl->halt, &one, sizeof(int), cudaMemcpyHostToDevice, s));
         PCD_CUDA(cudaMemcpyAsync(&ws.ctl->done, &one, sizeof(int), cudaMemcpyHostToDevice, s));
-    } else if (precision == PCD_PREC_MIXED) {
-        // first right-hand side of the FP32 correction sweeps
-        PCD_CUDA(cudaMemsetAsync(ws.e32, 0, sizeof(float) * (size_t)H * ld, s));
-        if (masked)
-            k_refine_residual<true><<<rblocks, kThreads, 0, s>>>(phi, ws.e32, b, ws.mask, ws.r32, ws.ctl, ws.partials, a, 1);
-        else
-            k_refine_residual<false><<<rblocks, kThreads, 0, s>>>(phi, ws.e32, b, ws.mask, ws.r32, ws.ctl, ws.partials, a, 1);
-        PCD_LAUNCHED(1);
     }
 
     // HBM grids without NaN cells: ping-pong tile passes or stream sweeps
@@ -1482,6 +1481,10 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     } else if (!masked && H >= 3 && W <= 2 * kRowCellsMax * kStripeThreads && o.schedule != PCD_SCHED_LAUNCHES) {
         sched = PCD_SCHED_STRIPES;
     }
+    // (r32, the first right-hand side of the FP32 sweeps, is the start's; the
+    // tile passes start from 0 without reading it)
+    if (!done_already && precision == PCD_PREC_MIXED && sched != PCD_SCHED_TILES)
+        PCD_CUDA(cudaMemsetAsync(ws.e32, 0, sizeof(float) * (size_t)H * ld, s));
     const bool stripes = sched == PCD_SCHED_STRIPES;
     if (stripes && ws.stripe_resident == 0) {
         int sms = 0, bps = 0;
@@ -1519,6 +1522,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
             if (flag_done(ws.ctl_host[prev])) finished = 1;
         }
     }
+    if (sched == PCD_SCHED_TILES && !done_already) PCD_TRY(launch_phi_settle(refresh_job(ws, b, phi, a), s));
     PCD_CUDA(cudaEventRecord(ws.k1, s));
     // Final statistics (FP64 residual of the returned phi).
     if (precision != PCD_PREC_MIXED) {

@@ -28,6 +28,7 @@ struct Ctl {
     int nan_cells;               // NaN entries of b
     int error;                   // PCD_TIMEOUT when a bounded device wait gave up
     int stream_out;              // ping-pong buffer holding the latest FP32 correction
+    int phi_side;                // refreshes: 1 while the potential sits in the second buffer
     unsigned int res_epoch;      // resident sweeps: halo exchanges of this solve so far
     unsigned int res_checks;     // resident sweeps: residual estimates of this solve so far
     unsigned long long maxbits;  // running max |delta| of the current sweep

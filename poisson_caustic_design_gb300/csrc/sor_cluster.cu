@@ -630,16 +630,16 @@ int tile_plan(int dev, int W, int H, int ld, int depth, TilePlan *plan)
 }
 
 int launch_tile(const TilePlan &p, const float *ein, float *eout, const float *r32, Ctl *ctl, const SolveArgs &a,
-                int nsw, int out_idx, bool track, cudaStream_t s)
+                int nsw, int out_idx, bool track, bool zero, cudaStream_t s)
 {
     const void *fn = tile_kernel(p.K, p.L, p.NQ, track);
     if (!fn || nsw < 1 || nsw > p.K) {
         set_error("tile SOR: no kernel for this plan");
         return PCD_BAD_ARG;
     }
-    using Fn = void (*)(const float *, float *, const float *, Ctl *, SolveArgs, int, int, int, int);
+    using Fn = void (*)(const float *, float *, const float *, Ctl *, SolveArgs, int, int, int, int, int);
     reinterpret_cast<Fn>(const_cast<void *>(fn))<<<p.grid, kRRThreads, p.smem, s>>>(ein, eout, r32, ctl, a, p.ncol,
-                                                                                    p.nrow, nsw, out_idx);
+                                                                                    p.nrow, nsw, out_idx, zero ? 1 : 0);
     return PCD_OK;
 }
 

@@ -83,8 +83,9 @@ int launch_tile_batch(const TileJob *d_jobs, int njobs, int ntiles, int nsw, int
 // applies.
 int tile_plan(int dev, int W, int H, int ld, int depth, TilePlan *plan);
 // One pass of nsw <= K sweeps from ein into eout (fewer at the sweep cap);
-// track: the pass reports the largest |update| of its last sweep.
+// track: the pass reports the largest |update| of its last sweep; zero: the
+// correction starts at 0 and ein is not read.
 int launch_tile(const TilePlan &p, const float *ein, float *eout, const float *r32, Ctl *ctl, const SolveArgs &a,
-                int nsw, int out_idx, bool track, cudaStream_t s);
+                int nsw, int out_idx, bool track, bool zero, cudaStream_t s);
 
 }  // namespace pcd

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
     Ctl *ctl = a.ctl;
     {
         const volatile Ctl *c = ctl;
-        if ((a.cycle ? c->done : c->halt) || c->error) return;  // every CTA reads the same
+        if (c->halt || c->done || c->error || c->nan_cells) return;  // every CTA reads the same
     }
     const int done_before = ((volatile const Ctl *)ctl)->sweeps;
     const int target0 = min(a.nsw, a.max_iter - done_before);

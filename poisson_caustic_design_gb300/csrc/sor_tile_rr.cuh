@@ -87,12 +87,12 @@ __device__ __forceinline__ void tile_setup(RRState<K, L, NQ> &st, const TileGeom
     }
 }
 
-// e of the tile's rows into registers and -r32 into the shared planes (zero
+// e of the tile's rows (zero: 0) into registers and -r32 into the shared planes (zero
 // outside the grid), then the warps' edge rows.
 template <int K, int L, int NQ>
 __device__ __forceinline__ void tile_load(RRState<K, L, NQ> &st, float *rp, const TileGeom &g,
                                           const float *__restrict__ ein, const float *__restrict__ r32, int H,
-                                          int ld)
+                                          int ld, bool zero = false)
 {
     constexpr int KS = RRState<K, L, NQ>::KS, R = kRRWarps * L;
 #pragma unroll
@@ -104,8 +104,10 @@ __device__ __forceinline__ void tile_load(RRState<K, L, NQ> &st, float *rp, cons
             float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A, RA = A, RB = A;
             if (y >= 0 && y < H && st.act[i]) {
                 const size_t p = (size_t)y * ld + g.x0 + 8 * qi;
-                A = ldg4(ein + p);
-                B = ldg4(ein + p + 4);
+                if (!zero) {
+                    A = ldg4(ein + p);
+                    B = ldg4(ein + p + 4);
+                }
                 RA = ldg4(r32 + p);
                 RB = ldg4(r32 + p + 4);
             }
@@ -199,12 +201,12 @@ __device__ __forceinline__ void tile_state_init(RRState<K, L, NQ> &st, const flo
 template <int K, int L, int NQ, bool TRACK>
 __global__ void __launch_bounds__(kRRThreads, 1)
     k_sor_tile_rr(const float *__restrict__ ein, float *__restrict__ eout, const float *__restrict__ r32, Ctl *ctl,
-                  SolveArgs a, int ncol, int nrow, int nsw, int out_idx)
+                  SolveArgs a, int ncol, int nrow, int nsw, int out_idx, int zero)
 {
     using S = RRState<K, L, NQ>;
     constexpr int HK = S::HK, KS = S::KS, N = kRRWarps * L - 2 * HK;
     static_assert(N > 0, "tile without interior rows");
-    if (*(volatile const int *)&ctl->halt) return;
+    if (*(volatile const int *)&ctl->halt || *(volatile const int *)&ctl->nan_cells) return;
     const int kr = min(nsw, a.max_iter - *(volatile const int *)&ctl->sweeps);
     if (kr < 1) return;  // every CTA reads the same count
     extern __shared__ __align__(16) float smem_f[];
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(kRRThreads, 1)
         const TileGeom g = tile_geom(tile, ncol, W, N, HK);
         tile_setup(st, g, W, H, a.w32);
         __syncthreads();  // the previous tile's half sweeps are done with the edge rows and planes
-        tile_load(st, rp, g, ein, r32, H, ld);
+        tile_load(st, rp, g, ein, r32, H, ld, zero != 0);
         if (tile + (int)gridDim.x < ntiles)
             tile_prefetch<L, NQ>(tile_geom(tile + (int)gridDim.x, ncol, W, N, HK), ein, r32, W, H, ld);
         __syncthreads();
