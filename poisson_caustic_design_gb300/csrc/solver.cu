@@ -31,6 +31,7 @@
 #include "sor_persist.cuh"
 #include "sor_cluster.cuh"
 #include "sor_blocks.cuh"
+#include "sor_blocks64.cuh"
 #include "sor_resident.cuh"
 #include "refresh.cuh"
 
@@ -817,6 +818,46 @@ int get_chunk_graph(SolverWorkspace &ws, const double *b, double *phi, const Sol
 
 namespace {
 
+template <typename Plan, typename Make>
+int cached_plan(SolverWorkspace &ws, std::vector<int> key, Plan *out, Make make)
+{
+    // entry: status byte, then the plan
+    auto it = ws.plans.find(key);
+    if (it == ws.plans.end()) {
+        Plan p{};
+        const int st = make(&p);
+        if (st != PCD_OK && st != PCD_BAD_ARG) return st;
+        if (ws.plans.size() >= 256) ws.plans.clear();
+        std::vector<char> v(1 + sizeof(Plan));
+        v[0] = (char)st;
+        std::memcpy(v.data() + 1, &p, sizeof(Plan));
+        it = ws.plans.emplace(std::move(key), std::move(v)).first;
+    }
+    std::memcpy(out, it->second.data() + 1, sizeof(Plan));
+    return it->second[0];
+}
+
+enum { kPlanResident, kPlanCluster, kPlanTile, kPlanPersist, kPlanBlocks, kPlanBlocks64 };
+
+// Polls of a tagged word before a wait gives up: each is an L2 trip, together
+// about two seconds.
+constexpr long long kWordPolls = 1ll << 21;
+
+// The tagged words' buffer, zeroed: tags start at 1 in every solve, and no word
+// of an earlier one may match.
+int reserve_words(SolverWorkspace &ws, size_t need, cudaStream_t s)
+{
+    if (need > ws.rx_bytes) {
+        if (ws.rx) cudaFree(ws.rx);
+        ws.rx = nullptr;
+        ws.rx_bytes = 0;
+        PCD_CUDA(cudaMalloc(&ws.rx, need));
+        ws.rx_bytes = need;
+    }
+    PCD_CUDA(cudaMemsetAsync(ws.rx, 0, need, s));
+    return PCD_OK;
+}
+
 // One cooperative launch per solve (sor_persist.cu), bracketed by the FP64
 // residual kernels that supply ||b|| / r64 before and the exact statistics after.
 int solve_persistent(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, int precision,
@@ -907,48 +948,20 @@ int reserve_ctas(SolverWorkspace &ws, int G)
     return PCD_OK;
 }
 
-// One cooperative launch per solve on 2-D blocks with deep halos
-// (sor_blocks.cu), then the exact FP64 statistics of the returned phi.
-int solve_blocks(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, int precision,
-                 const pcd_solve_opts &o, const BlocksPlan &bp, pcd_solve_stats *stats, cudaStream_t s)
+// Sweeps between the stop tests of the block schedule: a test costs an all-to-
+// all exchange of partials (a few L2 round trips), so every 16 sweeps for the
+// max-update stop and 32 for the relative residual, a multiple of the plan's
+// sweeps per exchange.
+int blocks_check_every(const SolveArgs &a, const pcd_solve_opts &o, const BlocksPlan &bp)
 {
-    const bool mixed = precision == PCD_PREC_MIXED;
-    const int G = bp.TY * bp.TX;
-    const int xs = (a.W + 3) & ~3;
-    const size_t elt = mixed ? sizeof(float) : sizeof(double);
-    const size_t need = 2 * (size_t)a.H * xs * elt + (mixed ? (size_t)a.H * xs * sizeof(float) : 0);
-    if (need > ws.bx_bytes) {
-        if (ws.bx) cudaFree(ws.bx);
-        ws.bx = nullptr;
-        ws.bx_bytes = 0;
-        PCD_CUDA(cudaMalloc(&ws.bx, need));
-        ws.bx_bytes = need;
-    }
-    PCD_TRY(reserve_ctas(ws, G));
-    PCD_CUDA(cudaMemsetAsync(ws.flags, 0, (G + 1) * sizeof(unsigned), s));
+    const int ce = o.check_every > 0 ? o.check_every : (a.stop == PCD_STOP_MAX_UPDATE ? 16 : 32);
+    return std::max(bp.K, (ce + bp.K - 1) / bp.K * bp.K);
+}
 
-    BlocksArgs ba{};
-    ba.W = a.W; ba.H = a.H; ba.ld = a.ld;
-    ba.TY = bp.TY; ba.TX = bp.TX; ba.G = G; ba.K = bp.K; ba.RTmax = bp.RTmax; ba.xs = xs;
-    ba.b = b; ba.phi = phi; ba.r64 = ws.r64;
-    ba.xb = ws.bx;
-    ba.r32x = mixed ? reinterpret_cast<float *>(static_cast<char *>(ws.bx) + 2 * (size_t)a.H * xs * elt) : nullptr;
-    ba.flags = ws.flags; ba.part = ws.part; ba.ctl = ws.ctl;
-    ba.stop = a.stop; ba.max_iter = a.max_iter; ba.tol = a.tol; ba.omega = a.omega;
-    // a stop test costs a grid barrier (a few L2 round trips): every 16
-    // sweeps for the max-update stop, 32 for the relative residual
-    int ce = o.check_every > 0 ? o.check_every : (a.stop == PCD_STOP_MAX_UPDATE ? 16 : 32);
-    ce = std::max(bp.K, (ce + bp.K - 1) / bp.K * bp.K);  // a multiple of the sweeps per exchange
-    ba.check_every = ce;
-    ba.cycle_cap = o.refine_every > 0 ? o.refine_every : 2048;
-    ba.drop = o.refine_drop > 0.0 ? o.refine_drop : 3e-2;
-    for (int c = 0; c < 5; c++) { ba.w64[c] = a.w64[c]; ba.w32[c] = a.w32[c]; }
-    ba.spin_limit = ws.wait_limit > 0 ? ws.wait_limit : 1ll << 24;
-    ba.withhold = ws.withhold_flag;
-    PCD_CUDA(cudaEventRecord(ws.k0, s));
-    PCD_TRY(launch_blocks(ba, mixed, bp.smem, s));
-    PCD_CUDA(cudaEventRecord(ws.k1, s));
-
+// The end of a block solve: the exact FP64 statistics of the returned phi.
+int finish_blocks(SolverWorkspace &ws, const double *b, const double *phi, const SolveArgs &a, int ce,
+                  pcd_solve_stats *stats, cudaStream_t s)
+{
     // exact FP64 statistics of the returned phi
     const int rblocks = grid_blocks((long)a.W * a.H);
     k_residual64<false><<<rblocks, kThreads, 0, s>>>(phi, b, ws.mask, ws.ctl, ws.partials, a, 0, 1, 0);
@@ -979,6 +992,79 @@ int solve_blocks(SolverWorkspace &ws, const double *b, double *phi, const SolveA
         stats->check_every_used = ce;
     }
     return converged ? PCD_OK : PCD_NOT_CONVERGED;
+}
+
+// One cooperative launch per solve on 2-D blocks with deep halos
+// (sor_blocks.cu), then the exact FP64 statistics of the returned phi.
+int solve_blocks(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const pcd_solve_opts &o,
+                 const BlocksPlan &bp, pcd_solve_stats *stats, cudaStream_t s)
+{
+    const int G = bp.TY * bp.TX;
+    const int xs = (a.W + 3) & ~3;
+    const size_t need = 3 * (size_t)a.H * xs * sizeof(float);
+    if (need > ws.bx_bytes) {
+        if (ws.bx) cudaFree(ws.bx);
+        ws.bx = nullptr;
+        ws.bx_bytes = 0;
+        PCD_CUDA(cudaMalloc(&ws.bx, need));
+        ws.bx_bytes = need;
+    }
+    PCD_TRY(reserve_ctas(ws, G));
+    PCD_CUDA(cudaMemsetAsync(ws.flags, 0, (G + 1) * sizeof(unsigned), s));
+
+    BlocksArgs ba{};
+    ba.W = a.W; ba.H = a.H; ba.ld = a.ld;
+    ba.TY = bp.TY; ba.TX = bp.TX; ba.G = G; ba.K = bp.K; ba.RTmax = bp.RTmax; ba.xs = xs;
+    ba.phi = phi; ba.r64 = ws.r64;
+    ba.xb = static_cast<float *>(ws.bx);
+    ba.r32x = static_cast<float *>(ws.bx) + 2 * (size_t)a.H * xs;
+    ba.flags = ws.flags; ba.part = ws.part; ba.ctl = ws.ctl;
+    ba.stop = a.stop; ba.max_iter = a.max_iter; ba.tol = a.tol;
+    const int ce = blocks_check_every(a, o, bp);
+    ba.check_every = ce;
+    ba.cycle_cap = o.refine_every > 0 ? o.refine_every : 2048;
+    ba.drop = o.refine_drop > 0.0 ? o.refine_drop : 3e-2;
+    for (int c = 0; c < 5; c++) ba.w32[c] = a.w32[c];
+    ba.spin_limit = ws.wait_limit > 0 ? ws.wait_limit : 1ll << 24;
+    ba.withhold = ws.withhold_flag;
+    PCD_CUDA(cudaEventRecord(ws.k0, s));
+    PCD_TRY(launch_blocks(ba, bp.smem, s));
+    PCD_CUDA(cudaEventRecord(ws.k1, s));
+
+    return finish_blocks(ws, b, phi, a, ce, stats, s);
+}
+
+// The FP64 form (sor_blocks64.cu), on grids that bp, the layout of the rule
+// below, fits; bp also fixes the stop tests' spacing.
+int solve_blocks64(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const pcd_solve_opts &o,
+                   const BlocksPlan &bp, pcd_solve_stats *stats, cudaStream_t s)
+{
+    Blocks64Plan plan;
+    const int st = cached_plan(ws, {kPlanBlocks64, a.W, a.H, o.block_sweeps}, &plan, [&](Blocks64Plan *p) {
+        return blocks64_plan(ws.dev, a.W, a.H, o.block_sweeps, p);
+    });
+    if (st != PCD_OK) {
+        if (st == PCD_BAD_ARG) set_error("block SOR: no FP64 layout for this grid");
+        return st;
+    }
+    const size_t part_at = plan.xb_bytes, need = part_at + (size_t)2 * plan.TY * plan.TX * 32;
+    PCD_TRY(reserve_words(ws, need, s));
+    Blocks64Args ba{};
+    ba.W = a.W; ba.H = a.H; ba.ld = a.ld;
+    ba.b = b; ba.phi = phi;
+    ba.xb = ws.rx;
+    ba.part = static_cast<char *>(ws.rx) + part_at;
+    ba.ctl = ws.ctl;
+    ba.stop = a.stop; ba.max_iter = a.max_iter; ba.tol = a.tol; ba.omega = a.omega;
+    const int ce = blocks_check_every(a, o, bp);
+    ba.check_every = ce;
+    for (int c = 0; c < 5; c++) ba.w64[c] = a.w64[c];
+    ba.spin_limit = ws.wait_limit > 0 ? ws.wait_limit : kWordPolls;
+    ba.withhold = ws.withhold_flag;
+    PCD_CUDA(cudaEventRecord(ws.k0, s));
+    PCD_TRY(launch_blocks64(ba, plan, s));
+    PCD_CUDA(cudaEventRecord(ws.k1, s));
+    return finish_blocks(ws, b, phi, a, ce, stats, s);
 }
 
 }  // namespace
@@ -1069,27 +1155,6 @@ struct ResidentRule {
     int sched = PCD_SCHED_TILES; // what the solve reports
 };
 
-template <typename Plan, typename Make>
-int cached_plan(SolverWorkspace &ws, std::vector<int> key, Plan *out, Make make)
-{
-    // entry: status byte, then the plan
-    auto it = ws.plans.find(key);
-    if (it == ws.plans.end()) {
-        Plan p{};
-        const int st = make(&p);
-        if (st != PCD_OK && st != PCD_BAD_ARG) return st;
-        if (ws.plans.size() >= 256) ws.plans.clear();
-        std::vector<char> v(1 + sizeof(Plan));
-        v[0] = (char)st;
-        std::memcpy(v.data() + 1, &p, sizeof(Plan));
-        it = ws.plans.emplace(std::move(key), std::move(v)).first;
-    }
-    std::memcpy(out, it->second.data() + 1, sizeof(Plan));
-    return it->second[0];
-}
-
-enum { kPlanResident = 0, kPlanCluster = 1, kPlanTile = 2, kPlanPersist = 3 };
-
 // FP32 sweeps between FP64 refreshes of the chunked mixed schedules.
 int mixed_chunk(const SolveArgs &a, const pcd_solve_opts &o)
 {
@@ -1163,15 +1228,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     const int G = plan.TX * plan.TY;
     const size_t part_at = plan.xb_bytes, gmax_at = part_at + 2 * (size_t)G * sizeof(unsigned long long);
     const size_t bar_at = gmax_at + kResidentChecksMax * sizeof(unsigned), need = bar_at + 64;
-    if (need > ws.rx_bytes) {
-        if (ws.rx) cudaFree(ws.rx);
-        ws.rx = nullptr;
-        ws.rx_bytes = 0;
-        PCD_CUDA(cudaMalloc(&ws.rx, need));
-        ws.rx_bytes = need;
-    }
-    // epochs start at 0 in every solve: no word of an earlier one may match
-    PCD_CUDA(cudaMemsetAsync(ws.rx, 0, need, s));
+    PCD_TRY(reserve_words(ws, need, s));
     const RefreshJob job = refresh_job(ws, b, phi, a);
 
     ResidentArgs ra{};
@@ -1192,8 +1249,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     ra.tol = a.tol;
     ra.drop = o.refine_drop > 0.0 ? o.refine_drop : 3e-2;
     for (int c = 0; c < 5; c++) ra.w32[c] = a.w32[c];
-    // a poll is an L2 trip: about two seconds
-    ra.spin_limit = ws.wait_limit > 0 ? ws.wait_limit : 1ll << 21;
+    ra.spin_limit = ws.wait_limit > 0 ? ws.wait_limit : kWordPolls;
     ra.withhold = ws.withhold_flag;
 
     PCD_CUDA(cudaEventRecord(ws.k0, s));
@@ -1416,8 +1472,8 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     const bool done_already = ws.ctl_host[0].converged != 0 || a.max_iter == 0;
 
     // FP64 sweeps: the block schedule (on chip, 2-D blocks, one L2 exchange per
-    // K sweeps) before the persistent bands (one per half sweep): 6.4 against
-    // 16.0 us per 512^2 sweep, 17 against 28 us (stripes) at 1024^2
+    // K sweeps) before the persistent bands (one per half sweep, 16.0 us a
+    // 512^2 sweep) and the stripes
     const bool auto_blocks = o.schedule == PCD_SCHED_AUTO && precision == PCD_PREC_FP64 &&
                              (long)W * H >= kTileMinCells;
     if (!done_already && !masked && (o.schedule == PCD_SCHED_BLOCKS || auto_blocks)) {
@@ -1428,11 +1484,15 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
             set_error("pcd solve: block_sweeps must be 0 (auto) or 1..8");
             return PCD_BAD_ARG;
         }
-        if (o.block_sweeps > 0) st = blocks_plan(ws.dev, W, H, o.block_sweeps, mixed, &bp);
-        else
+        st = cached_plan(ws, {kPlanBlocks, W, H, o.block_sweeps, mixed ? 1 : 0}, &bp, [&](BlocksPlan *p) {
+            if (o.block_sweeps > 0) return blocks_plan(ws.dev, W, H, o.block_sweeps, mixed, p);
+            int r = PCD_BAD_ARG;
             for (int K : {mixed ? 8 : 4, 4, 2, 1})
-                if ((st = blocks_plan(ws.dev, W, H, K, mixed, &bp)) == PCD_OK) break;
-        if (st == PCD_OK) return solve_blocks(ws, b, phi, a, precision, o, bp, stats, s);
+                if ((r = blocks_plan(ws.dev, W, H, K, mixed, p)) == PCD_OK) break;
+            return r;
+        });
+        if (st == PCD_OK)
+            return mixed ? solve_blocks(ws, b, phi, a, o, bp, stats, s) : solve_blocks64(ws, b, phi, a, o, bp, stats, s);
     }
     if (!done_already && !masked && precision == PCD_PREC_MIXED && a.stop == PCD_STOP_REL_RESIDUAL &&
         (o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_CLUSTER)) {

@@ -1,5 +1,6 @@
-// sor_blocks.cu -- persistent red-black SOR over 2-D blocks with deep halos
-// (sm_103a): one cooperative launch per solve, the whole chip on one grid.
+// sor_blocks.cu -- persistent FP32 red-black SOR over 2-D blocks with deep
+// halos, mixed precision (sm_103a): one cooperative launch per solve, the whole
+// chip on one grid.
 //
 // The grid is cut into TY x TX blocks, one CTA each.  A CTA keeps the region
 // of its block -- the owned cells plus a halo of h = 2K cells on every side --
@@ -24,26 +25,16 @@
 // the region's columns beyond the halo ring, hold 0 and are never relaxed;
 // guard rows above and below the region hold 0.
 //
-// Update: with w = omega / cnt (cnt the in-grid neighbours) the reference's
-// phi += w (sum - cnt phi - b) (solver.cpp:47) is phi' = (1 - omega) phi +
-// w (sum - b), since w cnt = omega; with w b kept per cell that is two FMAs
-// after the neighbour sum (5 FP64 operations per cell).  Missing neighbours
-// read 0, so the sum runs over the in-grid neighbours as in solver.cpp:29-44.
-//
-// Forms:
-//   FP64 (plain): phi and b in FP64; stop tests every check_every sweeps
-//     (the FP64 residual of the owned cells, or the last sweep's max |delta|)
-//     with a grid barrier and partials summed in a fixed order.
-//   MIXED: FP32 correction e on the FP32 right-hand side r32 = (float) r; an
-//     FP32 residual estimate every check_every sweeps ends a cycle once it
-//     fell by `drop` (or below 0.9 tol); the cycle's end folds e into phi in
-//     FP64 inside the launch: r -= L e (FP64, e widened exactly), phi += e,
-//     r32 = (float) r, e = 0, the FP64 norm of r as the stop test.
+// FP32 correction e on the FP32 right-hand side r32 = (float) r; an FP32
+// residual estimate every check_every sweeps ends a cycle once it fell by
+// `drop` (or below 0.9 tol); the cycle's end folds e into phi in FP64 inside
+// the launch: r -= L e (FP64, e widened exactly), phi += e, r32 = (float) r,
+// e = 0, the FP64 norm of r as the stop test.  (The FP64 sweeps have a kernel
+// of their own, sor_blocks64.cu, which exchanges tagged words instead.)
 //
 // Every wait is bounded: a flag or barrier wait gives up after spin_limit
 // polls, records PCD_TIMEOUT in the control block and every CTA returns.
 #include <algorithm>
-#include <type_traits>
 
 #include "sor_blocks.cuh"
 
@@ -115,17 +106,6 @@ __device__ bool bl_wait_neighbours(const BlocksArgs &a, int ty, int tx, unsigned
     return ok;
 }
 
-template <typename T>
-__device__ __forceinline__ T bl_fma(T a, T b, T c)
-{
-    return fma(a, b, c);
-}
-template <>
-__device__ __forceinline__ float bl_fma<float>(float a, float b, float c)
-{
-    return fmaf(a, b, c);
-}
-
 // Per-CTA geometry and per-lane column state.
 template <typename T>
 struct BlockState {
@@ -142,13 +122,6 @@ struct BlockState {
     __device__ T *bsrow(int c, int r) const { return BS + (size_t)c * ps + (size_t)(r + 1) * 32; }
     __device__ T *burow(int c, int r) const { return BU + (size_t)c * ps + (size_t)(r + 1) * 32; }
 };
-
-template <typename T>
-__device__ __forceinline__ T weight_of(const BlocksArgs &a, int cnt)
-{
-    if (sizeof(T) == 8) return (T)a.w64[cnt];
-    return (T)a.w32[cnt];
-}
 
 template <typename T>
 __device__ void block_setup(BlockState<T> &s, const BlocksArgs &a, unsigned char *smem)
@@ -180,10 +153,10 @@ __device__ void block_setup(BlockState<T> &s, const BlocksArgs &a, unsigned char
     s.own1 = gx1 >= s.x0 && gx1 < s.x1;
     s.cx0 = (gx0 > 0) + (gx0 < a.W - 1);
     s.cx1 = (gx1 > 0) + (gx1 < a.W - 1);
-    s.wi0 = weight_of<T>(a, min(4, s.cx0 + 2));
-    s.wi1 = weight_of<T>(a, min(4, s.cx1 + 2));
-    s.we0 = weight_of<T>(a, s.cx0 + 1);
-    s.we1 = weight_of<T>(a, s.cx1 + 1);
+    s.wi0 = a.w32[min(4, s.cx0 + 2)];
+    s.wi1 = a.w32[min(4, s.cx1 + 2)];
+    s.we0 = a.w32[s.cx0 + 1];
+    s.we1 = a.w32[s.cx1 + 1];
 }
 
 // Row neighbours in the grid of row gy (2 inside, 1 on the first / last row).
@@ -198,13 +171,11 @@ __device__ __forceinline__ T cell_weight(const BlockState<T> &s, int q, int cy)
 
 // One half sweep of colour c over region rows [lo, hi) (rows interleaved by
 // warp, unrolled so that several rows' loads are in flight).  TRACK: mx takes
-// max |update| over the owned cells.  FP64: phi' = (1 - omega) phi + w sum -
-// w b (two FMAs); FP32: the reference's form v + w (sum - cnt v - rhs), whose
-// rounding stays at the size of the update (the two-FMA form rounds at the
-// size of phi twice, which at omega ~ 2 costs FP32 correction sweeps).
+// max |update| over the owned cells.  The reference's form v + w (sum - cnt v -
+// rhs), whose rounding stays at the size of the update (the two-FMA form
+// rounds at the size of phi twice, which at omega ~ 2 costs correction sweeps).
 template <typename T, bool TRACK>
-__device__ __forceinline__ void relax_half(const BlockState<T> &s, const BlocksArgs &a, int c, int lo, int hi, T omc,
-                                           T &mx)
+__device__ __forceinline__ void relax_half(const BlockState<T> &s, const BlocksArgs &a, int c, int lo, int hi, T &mx)
 {
     lo = max(lo, -s.oy);  // grid rows only: the others hold 0 and stay 0
     hi = min(hi, a.H - s.oy);
@@ -221,13 +192,8 @@ __device__ __forceinline__ void relax_half(const BlockState<T> &s, const BlocksA
         T *V = s.xrow(c, r) + s.k;
         const T v = *V;
         const T sum = (up + dn) + (mid + nb);
-        T vn;
-        if (sizeof(T) == 8) {
-            vn = bl_fma<T>(w, sum, bl_fma<T>(omc, v, -s.bsrow(c, r)[s.k]));
-        } else {
-            const T cnt = (T)((q ? s.cx1 : s.cx0) + cy);
-            vn = bl_fma<T>(w, bl_fma<T>(-cnt, v, sum) - s.burow(c, r)[s.k], v);
-        }
+        const T cnt = (T)((q ? s.cx1 : s.cx0) + cy);
+        const T vn = fmaf(w, fmaf(-cnt, v, sum) - s.burow(c, r)[s.k], v);
         const bool act = q ? s.act1 : s.act0;
         if (act) *V = vn;
         if (TRACK) {
@@ -307,17 +273,16 @@ __device__ void publish_own(const BlockState<T> &s, const BlocksArgs &a, T *dst)
     }
 }
 
-template <bool MIXED>
 __global__ void __launch_bounds__(kBlocksThreads, 1) k_sor_blocks(BlocksArgs a)
 {
-    using T = typename std::conditional<MIXED, float, double>::type;
+    using T = float;
     extern __shared__ __align__(16) unsigned char smem_b[];
     __shared__ int s_ok[8];
     __shared__ double s_dec[3];
     BlockState<T> s;
     block_setup<T>(s, a, smem_b);
     const int g = blockIdx.x;
-    T *xb0 = reinterpret_cast<T *>(a.xb);
+    T *xb0 = a.xb;
     T *xb1 = xb0 + (size_t)a.H * a.xs;
 
     // ---- load the region: planes zeroed, then the grid's cells
@@ -332,20 +297,13 @@ __global__ void __launch_bounds__(kBlocksThreads, 1) k_sor_blocks(BlocksArgs a)
             if (!(q ? s.act1 : s.act0)) continue;
             const int gx = s.ox + 2 * s.k + q, c = (q + gy) & 1;
             const size_t i = (size_t)gy * a.ld + gx;
-            T rhs;
-            if (MIXED) {
-                rhs = (T)a.r64[i];
-            } else {
-                rhs = (T)a.b[i];
-                s.xrow(c, r)[s.k] = (T)a.phi[i];
-            }
+            const T rhs = (T)a.r64[i];
             s.burow(c, r)[s.k] = rhs;
             s.bsrow(c, r)[s.k] = cell_weight(s, q, cy) * rhs;
         }
     }
     __syncthreads();
 
-    const T omc = (T)(1.0 - a.omega);
     const double bnorm = *(volatile const double *)&a.ctl->bnorm;
     const bool track = a.stop == PCD_STOP_MAX_UPDATE;
     unsigned ep = 0, checks = 0;
@@ -360,9 +318,7 @@ __global__ void __launch_bounds__(kBlocksThreads, 1) k_sor_blocks(BlocksArgs a)
         const bool check = sweeps > 0 && (sweeps % a.check_every == 0 || sweeps >= a.max_iter);
         if (check) {
             double v[3] = {0.0, 0.0, 0.0};
-            if (!MIXED && track) {
-                v[2] = (double)mx;
-            } else if (MIXED && track) {
+            if (track) {
                 v[2] = (double)mx;
             } else {
                 T acc = T(0), m = T(0);
@@ -396,28 +352,15 @@ __global__ void __launch_bounds__(kBlocksThreads, 1) k_sor_blocks(BlocksArgs a)
             const double ssum = s_dec[0], smax = s_dec[2];
             __syncthreads();
             bool end_cycle;
-            if (!MIXED) {
-                if (track) {
-                    last_max = smax;
-                    converged = last_max < a.tol;
-                } else {
-                    rel = bnorm > 0.0 ? sqrt(ssum) / bnorm : sqrt(ssum);
-                    rmax = smax;
-                    converged = rel <= a.tol;
-                }
-                if (converged || sweeps >= a.max_iter) break;
-                end_cycle = false;
+            if (track) {
+                last_max = smax;
+                end_cycle = last_max < a.tol;
             } else {
-                if (track) {
-                    last_max = smax;
-                    end_cycle = last_max < a.tol;
-                } else {
-                    const double est = sqrt(ssum);
-                    end_cycle = est <= a.drop * cyc0 || est <= 0.9 * a.tol * (bnorm > 0.0 ? bnorm : 1.0);
-                }
-                end_cycle = end_cycle || sweeps >= a.max_iter || sweeps - cyc_sweeps >= a.cycle_cap;
+                const double est = sqrt(ssum);
+                end_cycle = est <= a.drop * cyc0 || est <= 0.9 * a.tol * (bnorm > 0.0 ? bnorm : 1.0);
             }
-            if (MIXED && end_cycle) {
+            end_cycle = end_cycle || sweeps >= a.max_iter || sweeps - cyc_sweeps >= a.cycle_cap;
+            if (end_cycle) {
                 // ---- fold e into phi in FP64: r -= L e, phi += e, r32 = (float) r
                 double acc = 0.0, m = 0.0;
                 for (int r = s.h + s.warp; r < s.h + s.R; r += kBlocksThreads / 32) {
@@ -478,7 +421,7 @@ __global__ void __launch_bounds__(kBlocksThreads, 1) k_sor_blocks(BlocksArgs a)
                 converged = track ? (last_max < a.tol) : (rel <= a.tol);
                 if (converged || sweeps >= a.max_iter) break;
                 // the neighbours' new r32 (written before the barrier) and e = 0 everywhere
-                load_ring<T, true>(s, a, reinterpret_cast<const T *>(a.r32x));
+                load_ring<T, true>(s, a, a.r32x);
                 for (int i = threadIdx.x; i < 2 * s.ps; i += blockDim.x) s.X[i] = T(0);
                 __syncthreads();
             }
@@ -491,11 +434,11 @@ __global__ void __launch_bounds__(kBlocksThreads, 1) k_sor_blocks(BlocksArgs a)
         for (int t = 0; t < nsw; t++) {
             const int d = 2 * (nsw - t) - 1;
             const bool last = track && t == nsw - 1;
-            if (last) relax_half<T, true>(s, a, 0, s.h - d, s.h + s.R + d, omc, mx);
-            else relax_half<T, false>(s, a, 0, s.h - d, s.h + s.R + d, omc, mx);
+            if (last) relax_half<T, true>(s, a, 0, s.h - d, s.h + s.R + d, mx);
+            else relax_half<T, false>(s, a, 0, s.h - d, s.h + s.R + d, mx);
             __syncthreads();
-            if (last) relax_half<T, true>(s, a, 1, s.h - d + 1, s.h + s.R + d - 1, omc, mx);
-            else relax_half<T, false>(s, a, 1, s.h - d + 1, s.h + s.R + d - 1, omc, mx);
+            if (last) relax_half<T, true>(s, a, 1, s.h - d + 1, s.h + s.R + d - 1, mx);
+            else relax_half<T, false>(s, a, 1, s.h - d + 1, s.h + s.R + d - 1, mx);
             __syncthreads();
         }
         sweeps += nsw;
@@ -514,19 +457,6 @@ __global__ void __launch_bounds__(kBlocksThreads, 1) k_sor_blocks(BlocksArgs a)
         __syncthreads();
     }
 
-    // ---- results: the FP64 form writes its owned cells back (the mixed form
-    // updated phi at every cycle's end)
-    if (!MIXED) {
-        for (int r = s.h + s.warp; r < s.h + s.R; r += kBlocksThreads / 32) {
-            const int gy = s.oy + r;
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                if (!(q ? s.own1 : s.own0)) continue;
-                const int gx = s.ox + 2 * s.k + q, c = (q + gy) & 1;
-                a.phi[(size_t)gy * a.ld + gx] = (double)s.xrow(c, r)[s.k];
-            }
-        }
-    }
     if (g == 0 && threadIdx.x == 0 && ok) {
         volatile Ctl *c = a.ctl;
         c->sweeps = sweeps;
@@ -573,12 +503,11 @@ int blocks_plan(int dev, int W, int H, int K, bool mixed, BlocksPlan *plan)
     return PCD_OK;
 }
 
-int launch_blocks(BlocksArgs &a, bool mixed, size_t smem, cudaStream_t s)
+int launch_blocks(BlocksArgs &a, size_t smem, cudaStream_t s)
 {
-    void *fn = mixed ? (void *)k_sor_blocks<true> : (void *)k_sor_blocks<false>;
-    PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PCD_CUDA(cudaFuncSetAttribute(k_sor_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void *params[] = {&a};
-    PCD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(a.G), dim3(kBlocksThreads), params, smem, s));
+    PCD_CUDA(cudaLaunchCooperativeKernel((const void *)k_sor_blocks, dim3(a.G), dim3(kBlocksThreads), params, smem, s));
     count_launches(1);
     return PCD_OK;
 }
