@@ -25,11 +25,11 @@
 // (bounded) for what it has in flight and frees its tensor memory.
 #include <cuda.h>
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
 
 #include <mutex>
 
 #include "nn.cuh"
+#include "tensor_map.cuh"
 
 namespace pcd {
 namespace nn {
@@ -486,29 +486,12 @@ __global__ void __launch_bounds__(kTpThreads, tp_ctas_per_sm(BN))
     }
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against the driver library).
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
-{
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
-    return fn;
-}
-
 // A 2-D tensor map of a rows x cols BF16 matrix (row stride ld elements) with
 // a box of box_rows x box_cols (box_cols of 64: the 128-byte swizzle; of 32:
 // the 64-byte swizzle).
 int make_map(CUtensorMap *map, const void *base, int rows, int cols, int ld, int box_rows, int box_cols = kTcBK)
 {
-    auto fn = encode_fn();
+    auto fn = tensor_map_encoder();
     if (!fn) {
         set_error("tcgen05 gemm: cuTensorMapEncodeTiled is not available");
         return PCD_DEVICE_ERROR;
@@ -558,7 +541,7 @@ bool conv_box(int W, int H, int T, int box[3])
 // of conv_box (the 128-byte swizzle for 64 channels, the 64-byte for 32).
 int make_map4(CUtensorMap *map, const void *base, int C, int W, int H, int B, int ldx, int cwid, int T)
 {
-    auto fn = encode_fn();
+    auto fn = tensor_map_encoder();
     if (!fn) {
         set_error("tcgen05 conv: cuTensorMapEncodeTiled is not available");
         return PCD_DEVICE_ERROR;
@@ -715,7 +698,7 @@ int gemm_tc_prepare()
     PCD_TRY(tcp_attr<64>());
     PCD_TRY(tcp_attr<128>());
     PCD_TRY(tcp_attr<256>());
-    if (!encode_fn()) {
+    if (!tensor_map_encoder()) {
         set_error("tcgen05 gemm: cuTensorMapEncodeTiled is not available");
         return PCD_DEVICE_ERROR;
     }

@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "refresh.cuh"
+#include "sor_quads.cuh"
 
 namespace pcd {
 
@@ -70,8 +71,10 @@ __device__ void rf_sum_partials(const double *partials, int nblk, double (&v)[3]
     block_reduce<3, 4u>(v);
 }
 
+// FIRST: the start of a batch's solves (e = 0; zero: phi = 0 too, and written).
+template <bool FIRST>
 __global__ void __launch_bounds__(32 * kRefreshWarps)
-    k_refresh(const RefreshJob *__restrict__ jobs, RefreshJob one, int njobs, double tol)
+    k_refresh(const RefreshJob *__restrict__ jobs, RefreshJob one, int njobs, double tol, int zero)
 {
     RefreshJob J = one;
     if (jobs) {
@@ -87,12 +90,12 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
     if (rf_load(&ctl->done) || rf_load(&ctl->error) || rf_load(&ctl->nan_cells)) return;
     const int side = rf_load(&ctl->phi_side);
     const double *__restrict__ pin = side ? J.phi2 : J.phi;
-    double *__restrict__ pout = side ? J.phi : J.phi2;
+    double *__restrict__ pout = FIRST || side ? J.phi : J.phi2;
     const float *__restrict__ e = rf_load(&ctl->stream_out) ? J.e1 : J.e0;
-    const int W = J.W, H = J.H, ld = J.ld;
+    const int W = J.W, H = J.H, ld = J.ld, KQ = (W + 7) >> 3;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int strips = (W + kRefreshCols - 1) / kRefreshCols, pieces = (H + J.rows - 1) / J.rows;
-    double acc = 0.0;
+    double acc = 0.0, acc_b = 0.0;
     unsigned long long mbits = 0ull;
     for (int item = ((int)blockIdx.x - J.blk0) * kRefreshWarps + w; item < strips * pieces;
          item += J.nblk * kRefreshWarps) {
@@ -102,11 +105,12 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
         const int y0 = piece * J.rows, y1 = min(y0 + J.rows, H);
         const double c2 = (double)((x > 0) + (x < W - 1) + 2), c1 = c2 - 1.0, c0 = c2 - 2.0;
         const size_t at = in ? (size_t)x : 0;
+        const int col = quads::quad_column((int)at, KQ);  // in a row of e and r32
         auto load = [&](int y, double &p, float &ev) {
             const bool ok = in && y >= 0 && y < H;
             const size_t i = (size_t)(ok ? y : 0) * ld + at;
-            p = ok ? pin[i] : 0.0;
-            ev = ok ? e[i] : 0.f;
+            p = ok && !(FIRST && zero) ? pin[i] : 0.0;
+            ev = ok && !FIRST ? e[(long)y * 8 * KQ + col] : 0.f;
         };
         // rows y0 - 1, y0 and y0 + 1; then one row ahead of the one in hand
         double pa, pb, pc, bc;
@@ -132,9 +136,10 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
             const double r = fma(cnt, xc, bc) - sum;
             if (own) {
                 const size_t i = (size_t)y * ld + at;
-                pout[i] = xc;
-                J.r32[i] = (float)r;
+                if (!FIRST || zero) pout[i] = xc;
+                J.r32[(long)y * 8 * KQ + col] = -(float)r;
                 acc = fma(r, r, acc);
+                if (FIRST) acc_b = fma(bc, bc, acc_b);
                 mbits = max_abs_bits(mbits, r);
             }
             dp = d;
@@ -144,18 +149,19 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
             bc = bn;
         }
     }
-    double v[3] = {acc, 0.0, __longlong_as_double((long long)mbits)};
+    double v[3] = {acc, acc_b, __longlong_as_double((long long)mbits)};
     block_reduce<3, 4u>(v);
     if (threadIdx.x == 0) {
         double *p = J.partials + 3 * ((int)blockIdx.x - J.blk0);
         p[0] = v[0];
-        p[1] = 0.0;
+        p[1] = v[1];
         p[2] = v[2];
     }
     if (!rf_last_block(ctl, J.nblk)) return;
     rf_sum_partials(J.partials, J.nblk, v);
     if (threadIdx.x == 0) {
         volatile Ctl *c = ctl;
+        if (FIRST) c->bnorm = sqrt(v[1]);
         const double rn = sqrt(v[0]), bn = c->bnorm, rel = bn > 0.0 ? rn / bn : rn;
         c->rnorm = rn;
         c->rmax = v[2];
@@ -166,15 +172,16 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
             c->halt = 1;
         }
         if (c->halt) c->done = 1;
-        c->phi_side = side ^ 1;
+        if (!FIRST) c->phi_side = side ^ 1;
         c->stream_out = 0;
         c->blocks_done_r = 0;
         __threadfence();
     }
 }
 
-__global__ void __launch_bounds__(kStartThreads) k_phi_settle(RefreshJob J)
+__global__ void __launch_bounds__(kStartThreads) k_phi_settle(const RefreshJob *__restrict__ jobs, RefreshJob one)
 {
+    const RefreshJob &J = jobs ? jobs[blockIdx.z] : one;
     if (!rf_load(&J.ctl->phi_side)) return;
     for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < J.W; x += gridDim.x * blockDim.x)
         for (int y = blockIdx.y; y < J.H; y += gridDim.y) J.phi[(size_t)y * J.ld + x] = J.phi2[(size_t)y * J.ld + x];
@@ -183,14 +190,22 @@ __global__ void __launch_bounds__(kStartThreads) k_phi_settle(RefreshJob J)
 template <bool ZERO>
 __global__ void __launch_bounds__(kStartThreads)
     k_start(const double *__restrict__ b, double *__restrict__ phi, uint8_t *__restrict__ mask,
-            double *__restrict__ r64, float *__restrict__ r32, Ctl *ctl, double *partials, SolveArgs a, int test)
+            double *__restrict__ r64, float *__restrict__ r32, Ctl *ctl, double *partials, SolveArgs a, int in_quads,
+            int test)
 {
     const int W = a.W, H = a.H, ld = a.ld;
     double v[3] = {0.0, 0.0, 0.0};
     unsigned long long mbits = 0ull;
     int nans = 0;
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < W; x += gridDim.x * blockDim.x) {
+    const int KQ = (W + 7) >> 3;
+    const int last = in_quads ? 8 * KQ : W;
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < last; x += gridDim.x * blockDim.x) {
+        const int col = quads::quad_column(x, KQ);
         for (int y = blockIdx.y; y < H; y += gridDim.y) {
+            if (x >= W) {  // the rest of the last quads
+                r32[(long)y * 8 * KQ + col] = 0.f;
+                continue;
+            }
             const size_t i = (size_t)y * ld + x;
             const bool l = x > 0 && !is_nan_bits(b[i - 1]), u = y > 0 && !is_nan_bits(b[i - ld]);
             const bool rt = x < W - 1 && !is_nan_bits(b[i + 1]), d = y < H - 1 && !is_nan_bits(b[i + ld]);
@@ -209,7 +224,10 @@ __global__ void __launch_bounds__(kStartThreads)
                 r = bi - (sum - (double)((int)l + (int)u + (int)rt + (int)d) * phi[i]);
             }
             if (r64 && !nan) r64[i] = r;
-            if (r32) r32[i] = (float)r;
+            if (r32) {
+                if (in_quads) r32[(long)y * 8 * KQ + col] = -(float)r;
+                else r32[i] = (float)r;
+            }
             if (nan) {
                 nans++;
                 continue;
@@ -251,39 +269,49 @@ __global__ void __launch_bounds__(kStartThreads)
 
 }  // namespace
 
-int refresh_shape(int W, int H, int cap, int *rows)
+int refresh_shape(int W, int H, int cap, long warps, int *rows)
 {
     const int strips = ceil_div(W, kRefreshCols);
-    // a piece's two rows of overlap cost a quarter of a row's work each; the
-    // FP64 pipes want 4 warps an SM, and twice that to hide the loads
+    // a piece's two rows of overlap cost a quarter of a row's work each
     int r = 32;
-    while (r > 8 && (long)strips * ceil_div(H, r) < 152L * 2 * kRefreshWarps) r >>= 1;
+    while (r > 8 && (long)strips * ceil_div(H, r) < warps) r >>= 1;
     *rows = r;
     return std::max(1, std::min(cap, ceil_div((long)strips * ceil_div(H, r), kRefreshWarps)));
 }
 
 int launch_refresh(const RefreshJob *jobs, const RefreshJob &one, int njobs, int blocks, double tol, cudaStream_t s)
 {
-    k_refresh<<<blocks, 32 * kRefreshWarps, 0, s>>>(jobs, one, njobs, tol);
+    k_refresh<false><<<blocks, 32 * kRefreshWarps, 0, s>>>(jobs, one, njobs, tol, 0);
     PCD_LAUNCHED(1);
     return PCD_OK;
 }
 
-int launch_phi_settle(const RefreshJob &job, cudaStream_t s)
+int launch_first_refresh(const RefreshJob *jobs, int njobs, int blocks, double tol, bool zero, cudaStream_t s)
 {
-    const int gx = std::min(ceil_div(job.W, kStartThreads), 2432);
-    k_phi_settle<<<dim3(gx, std::max(1, std::min(job.H, 2432 / gx))), kStartThreads, 0, s>>>(job);
+    k_refresh<true><<<blocks, 32 * kRefreshWarps, 0, s>>>(jobs, RefreshJob{}, njobs, tol, zero ? 1 : 0);
+    PCD_LAUNCHED(1);
+    return PCD_OK;
+}
+
+int launch_phi_settle(const RefreshJob *jobs, const RefreshJob &one, int njobs, cudaStream_t s)
+{
+    const dim3 grid = jobs ? dim3(4, 64, njobs)
+                           : dim3(std::min(ceil_div(one.W, kStartThreads), 2432),
+                                  std::max(1, std::min(one.H, 2432 / ceil_div(one.W, kStartThreads))));
+    k_phi_settle<<<grid, kStartThreads, 0, s>>>(jobs, one);
     PCD_LAUNCHED(1);
     return PCD_OK;
 }
 
 int launch_start(const double *b, double *phi, uint8_t *mask, double *r64, float *r32, Ctl *ctl, double *partials,
-                 int max_partials, const SolveArgs &a, bool zero, bool test, cudaStream_t s)
+                 int max_partials, const SolveArgs &a, bool zero, bool quads, bool test, cudaStream_t s)
 {
-    const int gx = std::min(ceil_div(a.W, kStartThreads), max_partials);
+    const int gx = std::min(ceil_div(quads ? quads::quad_row_floats(a.W) : a.W, kStartThreads), max_partials);
     const dim3 grid(gx, std::max(1, std::min(a.H, max_partials / gx)));
-    if (zero) k_start<true><<<grid, kStartThreads, 0, s>>>(b, phi, mask, r64, r32, ctl, partials, a, test ? 1 : 0);
-    else k_start<false><<<grid, kStartThreads, 0, s>>>(b, phi, mask, r64, r32, ctl, partials, a, test ? 1 : 0);
+    if (zero) k_start<true><<<grid, kStartThreads, 0, s>>>(b, phi, mask, r64, r32, ctl, partials, a, quads ? 1 : 0,
+                                                      test ? 1 : 0);
+    else k_start<false><<<grid, kStartThreads, 0, s>>>(b, phi, mask, r64, r32, ctl, partials, a, quads ? 1 : 0,
+                                                      test ? 1 : 0);
     PCD_LAUNCHED(1);
     return PCD_OK;
 }

@@ -32,8 +32,10 @@
 #include "sor_cluster.cuh"
 #include "sor_blocks.cuh"
 #include "sor_blocks64.cuh"
+#include "sor_passes.cuh"
 #include "sor_resident.cuh"
 #include "refresh.cuh"
+#include "sor_quads.cuh"
 
 namespace pcd {
 
@@ -658,7 +660,7 @@ RefreshJob refresh_job(const SolverWorkspace &ws, const double *b, double *phi, 
     j.W = a.W;
     j.H = a.H;
     j.ld = a.ld;
-    j.nblk = refresh_shape(a.W, a.H, kResidualBlocksMax, &j.rows);
+    j.nblk = refresh_shape(a.W, a.H, kResidualBlocksMax, kRefreshFill, &j.rows);
     return j;
 }
 
@@ -692,12 +694,13 @@ int enqueue_chunk(SolverWorkspace &ws, const double *b, double *phi, const Solve
     }
     if (!MASKED && sched == PCD_SCHED_TILES) {
         // as the stream passes: pass k reads buffer k&1 and writes the other
+        TileMaps maps;
+        PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, sp.tile.rows + 4 * sp.tile.K, &maps));
         int k = 0;
         for (int done = 0; done < sweeps; k++) {
-            const float *ein = (k & 1) ? ws.e32b : ws.e32;
             float *eout = (k & 1) ? ws.e32 : ws.e32b;
             const int nsw = std::min(sp.tile_sweeps, sweeps - done);
-            PCD_TRY(launch_tile(sp.tile, ein, eout, ws.r32, ws.ctl, a, nsw, (k & 1) ? 0 : 1, track, k == 0, s));
+            PCD_TRY(launch_tile(sp.tile, (k & 1) ? maps.eb : maps.ea, eout, maps.r32, ws.ctl, a, nsw, (k & 1) ? 0 : 1, track, k == 0, s));
             done += nsw;
             n++;
         }
@@ -771,7 +774,7 @@ int get_chunk_graph(SolverWorkspace &ws, const double *b, double *phi, const Sol
 {
     std::vector<long long> key = {(long long)(uintptr_t)b, (long long)(uintptr_t)phi, a.W, a.H, a.ld, a.stop,
                                   a.max_iter, precision, masked, sweeps, sched, sp.G, sp.T, sp.R, sp.tma, sp.two,
-                                  sp.tile.K, sp.tile.L, sp.tile.NQ, sp.tile_sweeps};
+                                  sp.tile.K, sp.tile.grid, sp.tile_sweeps};
     long long tb, ob;
     std::memcpy(&tb, &a.tol, 8);
     std::memcpy(&ob, &a.omega, 8);
@@ -1232,7 +1235,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     const RefreshJob job = refresh_job(ws, b, phi, a);
 
     ResidentArgs ra{};
-    ra.W = a.W; ra.H = a.H; ra.ld = a.ld;
+    ra.W = a.W; ra.H = a.H;
     ra.e = ws.e32; ra.r32 = ws.r32; ra.ctl = ws.ctl;
     char *rx = static_cast<char *>(ws.rx);
     ra.xb = rx;
@@ -1274,7 +1277,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
             if (c.done || c.error || c.nan_cells) finished = true;
         }
     }
-    PCD_TRY(launch_phi_settle(job, s));
+    PCD_TRY(launch_phi_settle(nullptr, job, 1, s));
     PCD_CUDA(cudaEventRecord(ws.k1, s));
     PCD_CUDA(cudaEventRecord(ws.t1, s));
     PCD_CUDA(cudaMemcpyAsync(&ws.ctl_host[0], ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
@@ -1435,7 +1438,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         set_error("pcd solve: bad options");
         return PCD_BAD_ARG;
     }
-    PCD_TRY(ws.reserve((size_t)H * ld));
+    PCD_TRY(ws.reserve((size_t)H * std::max<size_t>(ld, quads::quad_row_floats(W))));
 
     SolveArgs a;
     a.W = W; a.H = H; a.ld = ld;
@@ -1450,17 +1453,25 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     const int precision = o.precision;
 
     PCD_CUDA(cudaEventRecord(ws.t0, s));
-    PCD_CUDA(cudaMemsetAsync(ws.ctl, 0, sizeof(Ctl), s));
     const int rblocks = grid_blocks((long)W * H);
+    const bool mixed = precision == PCD_PREC_MIXED;
     ResidentPlan rp;
     ResidentRule rule;
     const int resident = a.max_iter > 0 ? resident_rule(ws, a, o, &rp, &rule) : PCD_BAD_ARG;
     if (resident != PCD_OK && resident != PCD_BAD_ARG) return resident;
     // mask, initial FP64 residual and norms (valid with or without NaN cells);
-    // r64 for the mixed schedules that carry the residual on
-    PCD_TRY(launch_start(b, phi, ws.mask, precision == PCD_PREC_MIXED && resident != PCD_OK ? ws.r64 : nullptr,
-                         precision == PCD_PREC_MIXED ? ws.r32 : nullptr, ws.ctl, ws.partials, kResidualBlocksMax, a,
-                         !o.warm_start, a.stop == PCD_STOP_REL_RESIDUAL, s));
+    // r64 for the mixed schedules that carry the residual on; r32 in the layout
+    // of the schedule that will most likely run (NaN cells are not known yet)
+    bool r32_quads = false;
+    auto start = [&](bool in_quads) -> int {
+        r32_quads = in_quads;
+        PCD_CUDA(cudaMemsetAsync(ws.ctl, 0, sizeof(Ctl), s));
+        return launch_start(b, phi, ws.mask, mixed && resident != PCD_OK ? ws.r64 : nullptr, mixed ? ws.r32 : nullptr,
+                            ws.ctl, ws.partials, kResidualBlocksMax, a, !o.warm_start, in_quads,
+                            a.stop == PCD_STOP_REL_RESIDUAL, s);
+    };
+    PCD_TRY(start(mixed && (resident == PCD_OK ||
+                            ((o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_TILES) && W % 8 == 0))));
     if (resident == PCD_OK) {
         int nans = 0;
         const int st = solve_resident(ws, b, phi, a, o, rp, rule, stats, &nans, s);
@@ -1478,7 +1489,6 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
                              (long)W * H >= kTileMinCells;
     if (!done_already && !masked && (o.schedule == PCD_SCHED_BLOCKS || auto_blocks)) {
         BlocksPlan bp{};
-        const bool mixed = precision == PCD_PREC_MIXED;
         int st = PCD_BAD_ARG;
         if (o.block_sweeps < 0 || o.block_sweeps > 8) {
             set_error("pcd solve: block_sweeps must be 0 (auto) or 1..8");
@@ -1497,7 +1507,10 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     if (!done_already && !masked && precision == PCD_PREC_MIXED && a.stop == PCD_STOP_REL_RESIDUAL &&
         (o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_CLUSTER)) {
         ClusterPlan plan{};
-        if (cluster_plan(ws.dev, W, H, 4, &plan) == PCD_OK) return solve_cluster(ws, b, phi, a, o, plan, stats, s);
+        if (cluster_plan(ws.dev, W, H, 4, &plan) == PCD_OK) {
+            if (r32_quads) PCD_TRY(start(false));
+            return solve_cluster(ws, b, phi, a, o, plan, stats, s);
+        }
     }
     // FP32 sweeps beyond one cluster: the tile passes before the persistent
     // schedule (measured 2-3.5x faster from 64^2 to 1024^2)
@@ -1543,6 +1556,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     }
     // (r32, the first right-hand side of the FP32 sweeps, is the start's; the
     // tile passes start from 0 without reading it)
+    if (!done_already && mixed && r32_quads != (sched == PCD_SCHED_TILES)) PCD_TRY(start(!r32_quads));
     if (!done_already && precision == PCD_PREC_MIXED && sched != PCD_SCHED_TILES)
         PCD_CUDA(cudaMemsetAsync(ws.e32, 0, sizeof(float) * (size_t)H * ld, s));
     const bool stripes = sched == PCD_SCHED_STRIPES;
@@ -1579,10 +1593,10 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         if (launched >= 2) {
             const int prev = (int)((launched - 2) & 1);
             PCD_CUDA(cudaEventSynchronize(ws.ev[prev]));
-            if (flag_done(ws.ctl_host[prev])) finished = 1;
+            if (flag_done(ws.ctl_host[prev]) || ws.ctl_host[prev].error) finished = 1;
         }
     }
-    if (sched == PCD_SCHED_TILES && !done_already) PCD_TRY(launch_phi_settle(refresh_job(ws, b, phi, a), s));
+    if (sched == PCD_SCHED_TILES && !done_already) PCD_TRY(launch_phi_settle(nullptr, refresh_job(ws, b, phi, a), 1, s));
     PCD_CUDA(cudaEventRecord(ws.k1, s));
     // Final statistics (FP64 residual of the returned phi).
     if (precision != PCD_PREC_MIXED) {
@@ -1597,7 +1611,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     PCD_CUDA(cudaStreamSynchronize(s));
     const Ctl &c = ws.ctl_host[0];
     if (c.error) {
-        set_error("stream SOR: a bounded wait for a row copy gave up (status " + std::to_string(c.error) + ")");
+        set_error("stream or tile SOR: a bounded wait for a copy gave up (status " + std::to_string(c.error) + ")");
         return c.error;
     }
     if (stats) {
@@ -1620,137 +1634,30 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
 
 // ---------------------------------------------------------------------------
 // Batched tile solve: the grids of a batch share one tile pass per launch
-// (k_sor_tile_batch) and one FP64 refresh pair per chunk of passes, each
+// (k_tile_batch) and one FP64 refresh per chunk of passes, each
 // grid with its own control block, so a grid that has converged drops out
 // while the others go on.
 namespace {
 
-// One grid of the batched FP64 refresh: blocks [blk0, blk0 + nblk) of the
-// launch work on it.
-struct RefineJob {
-    const double *b;
-    double *phi;
-    float *e, *eb;       // the correction buffers (eb holds the latest when stream_out is set)
-    float *r32;
-    Ctl *ctl;
-    double *partials;    // 3 per block
-    int W, H, ld;
-    int blk0, nblk;
-};
-
-// Blocks per grid of the batched FP64 refresh: about 4 cells per thread, so
-// that the large grids' FP64 work spreads over every SM.
+// Most blocks of one grid in the batched FP64 refresh.
 constexpr int kBatchRefineBlocks = 1024;
-constexpr int kBatchRefineCellsPerBlock = 4 * kThreads;
-
-__device__ __forceinline__ int refine_job(const RefineJob *jobs, int njobs, int blk)
-{
-    int lo = 0, hi = njobs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&jobs[mid].blk0) <= blk) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ bool last_block_of(Ctl *ctl, int nblk)
-{
-    __shared__ bool is_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned t = atomicAdd(&ctl->blocks_done_r, 1u);
-        is_last = (t == (unsigned)nblk - 1u);
-    }
-    __syncthreads();
-    if (is_last) __threadfence();
-    return is_last;
-}
-
-// r = b - L(phi + e) in FP64 per grid (the latest correction buffer), r32 =
-// (float) r, norms and the relative-residual test by each grid's last block.
-__global__ void __launch_bounds__(kThreads)
-    k_batch_refine_residual(const RefineJob *__restrict__ jobs, int njobs, double tol, int with_b)
-{
-    const RefineJob &J = jobs[refine_job(jobs, njobs, blockIdx.x)];
-    Ctl *ctl = J.ctl;
-    if (vol_load(&ctl->done)) return;
-    const float *__restrict__ e = vol_load(&ctl->stream_out) ? J.eb : J.e;
-    const int lb = (int)blockIdx.x - J.blk0, W = J.W, H = J.H, ld = J.ld;
-    const long n = (long)W * H;
-    double v[3] = {0.0, 0.0, 0.0};
-    for (long t = (long)lb * blockDim.x + threadIdx.x; t < n; t += (long)J.nblk * blockDim.x) {
-        const int y = (int)(t / W), x = (int)(t - (long)y * W);
-        const long i = (long)y * ld + x;
-        const double bi = J.b[i];
-        // the neighbour sum in k_refine_residual's order; the count as an integer
-        double sum = 0.0;
-        int cnt = 0;
-        if (x > 0) { cnt++; sum += J.phi[i - 1] + (double)e[i - 1]; }
-        if (y > 0) { cnt++; sum += J.phi[i - ld] + (double)e[i - ld]; }
-        if (x < W - 1) { cnt++; sum += J.phi[i + 1] + (double)e[i + 1]; }
-        if (y < H - 1) { cnt++; sum += J.phi[i + ld] + (double)e[i + ld]; }
-        const double xi = J.phi[i] + (double)e[i];
-        const double r = bi - (sum - (double)cnt * xi);
-        J.r32[i] = (float)r;
-        if (isnan(bi)) continue;
-        v[0] += r * r;
-        v[1] += bi * bi;
-        v[2] = nan_skip_max(v[2], fabs(r));
-    }
-    block_reduce<3, 4u>(v);
-    if (threadIdx.x == 0) {
-        J.partials[3 * lb] = v[0];
-        J.partials[3 * lb + 1] = v[1];
-        J.partials[3 * lb + 2] = v[2];
-    }
-    if (last_block_of(ctl, J.nblk)) {
-        SolveArgs a{};
-        a.stop = PCD_STOP_REL_RESIDUAL;
-        a.tol = tol;
-        finalize_residual(ctl, J.partials, J.nblk, a, 1, with_b);
-    }
-}
-
-// phi += latest correction, e = 0 per grid; a halted grid is done.
-__global__ void __launch_bounds__(kThreads) k_batch_refine_update(const RefineJob *__restrict__ jobs, int njobs)
-{
-    const RefineJob &J = jobs[refine_job(jobs, njobs, blockIdx.x)];
-    Ctl *ctl = J.ctl;
-    if (vol_load(&ctl->done)) return;
-    const float *el = vol_load(&ctl->stream_out) ? J.eb : J.e;
-    const int lb = (int)blockIdx.x - J.blk0, W = J.W, ld = J.ld;
-    const long n = (long)W * J.H;
-    for (long t = (long)lb * blockDim.x + threadIdx.x; t < n; t += (long)J.nblk * blockDim.x) {
-        const int y = (int)(t / W), x = (int)(t - (long)y * W);
-        const long i = (long)y * ld + x;
-        J.phi[i] += (double)el[i];
-        J.e[i] = 0.0f;
-    }
-    if (last_block_of(ctl, J.nblk)) {
-        if (threadIdx.x == 0) {
-            volatile Ctl *c = ctl;
-            if (c->halt) c->done = 1;
-            c->stream_out = 0;
-            c->blocks_done_r = 0;
-            __threadfence();
-        }
-    }
-}
 
 }  // namespace
 
-int TileBatchWorkspace::reserve(size_t floats, int count)
+int TileBatchWorkspace::reserve(size_t cells, int count)
 {
-    if (floats > arena_floats) {
+    // per cell: the two corrections, the right-hand side, the second potential
+    if (cells > arena_cells) {
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
         graphs.clear();
         if (arena) cudaFree(arena);
+        if (phi2) cudaFree(phi2);
         arena = nullptr;
-        arena_floats = 0;
-        PCD_CUDA(cudaMalloc(&arena, floats * sizeof(float)));
-        arena_floats = floats;
+        phi2 = nullptr;
+        arena_cells = 0;
+        PCD_CUDA(cudaMalloc(&arena, 3 * cells * sizeof(float)));
+        PCD_CUDA(cudaMalloc(&phi2, cells * sizeof(double)));
+        arena_cells = cells;
     }
     if (count > cap) {
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
@@ -1766,7 +1673,7 @@ int TileBatchWorkspace::reserve(size_t floats, int count)
         PCD_CUDA(cudaMallocHost(&ctl_host, 2 * sizeof(Ctl) * count));
         PCD_CUDA(cudaMalloc(&partials, sizeof(double) * 3 * kBatchRefineBlocks * count));
         PCD_CUDA(cudaMalloc(&jobs, sizeof(TileJob) * count));
-        PCD_CUDA(cudaMalloc(&rjobs, sizeof(RefineJob) * count));
+        PCD_CUDA(cudaMalloc(&rjobs, sizeof(RefreshJob) * count));
         cap = count;
     }
     if (!t0) {
@@ -1784,6 +1691,7 @@ void TileBatchWorkspace::release()
     for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
     graphs.clear();
     if (arena) cudaFree(arena);
+    if (phi2) cudaFree(phi2);
     if (ctl) cudaFree(ctl);
     if (ctl_host) cudaFreeHost(ctl_host);
     if (partials) cudaFree(partials);
@@ -1820,10 +1728,12 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     }
     size_t smem = 0;
     int grid = 0;
-    PCD_TRY(tile_batch_config(dev, count, &smem, &grid));
+    bool narrow = false;
+    for (int i = 0; i < count; i++) narrow = narrow || inst[i].width == 8;
+    PCD_TRY(tile_batch_config(dev, count, narrow, &smem, &grid));
     size_t per = 0;
     for (int i = 0; i < count; i++) per += (size_t)inst[i].height * inst[i].ld;
-    PCD_TRY(ws.reserve(3 * per, count));
+    PCD_TRY(ws.reserve(per, count));
 
     // largest grids first: their refresh blocks are dispatched first
     std::vector<int> order(count);
@@ -1832,23 +1742,23 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         return (long)inst[x].width * inst[x].height > (long)inst[y].width * inst[y].height;
     });
     std::vector<TileJob> tj((size_t)count);
-    std::vector<RefineJob> rj((size_t)count);
-    size_t off = 0;
+    std::vector<RefreshJob> rj((size_t)count);
+    size_t off = 0, all_cells = 0;
+    for (int i = 0; i < count; i++) all_cells += (size_t)inst[i].width * inst[i].height;
     int tiles = 0, blocks = 0, maxdim = 0;
     for (int k = 0; k < count; k++) {
         const int i = order[k];
         const pcd_instance &q = inst[i];
         maxdim = std::max(maxdim, std::max(q.width, q.height));
         TileJob &t = tj[k];
-        RefineJob &r = rj[k];
+        RefreshJob &r = rj[k];
         t.ea = ws.arena + off;
         t.eb = ws.arena + per + off;
         t.r32 = ws.arena + 2 * per + off;
         t.ctl = ws.ctl + k;
         t.W = q.width;
         t.H = q.height;
-        t.ld = q.ld;
-        tile_counts(q.width, q.height, &t.ncol, &t.nrow);
+        PCD_TRY(tile_job_setup(&t));
         t.tile0 = tiles;
         t.max_iter = o.max_iterations;
         const double om = resolve_omega(o.omega, q.width, q.height);
@@ -1856,8 +1766,9 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         tiles += t.ncol * t.nrow;
         r.b = q.b;
         r.phi = q.phi;
-        r.e = t.ea;
-        r.eb = t.eb;
+        r.phi2 = ws.phi2 + off;
+        r.e0 = t.ea;
+        r.e1 = t.eb;
         r.r32 = ws.arena + 2 * per + off;
         r.ctl = t.ctl;
         r.partials = ws.partials + (size_t)3 * kBatchRefineBlocks * k;
@@ -1865,14 +1776,14 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         r.H = q.height;
         r.ld = q.ld;
         r.blk0 = blocks;
-        r.nblk = (int)std::min<long>(kBatchRefineBlocks,
-                                     ((long)q.width * q.height + kBatchRefineCellsPerBlock - 1) /
-                                         kBatchRefineCellsPerBlock);
+        // each grid's share of the warps that fill the chip
+        r.nblk = refresh_shape(q.width, q.height, kBatchRefineBlocks,
+                               (long)((double)kRefreshFill * q.width * q.height / (double)all_cells), &r.rows);
         blocks += r.nblk;
         off += (size_t)q.height * q.ld;
     }
     const TileJob *d_jobs = static_cast<const TileJob *>(ws.jobs);
-    const RefineJob *d_rjobs = static_cast<const RefineJob *>(ws.rjobs);
+    const RefreshJob *d_rjobs = static_cast<const RefreshJob *>(ws.rjobs);
     // sweeps between FP64 refreshes (passes of 4, the last one shorter):
     // refine_every, else 128 when the largest side is 1024 or more, down to
     // 32 when it is 256 or less
@@ -1881,21 +1792,14 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
 
     PCD_CUDA(cudaEventRecord(ws.t0, s));
     PCD_CUDA(cudaMemcpyAsync(ws.jobs, tj.data(), sizeof(TileJob) * count, cudaMemcpyHostToDevice, s));
-    PCD_CUDA(cudaMemcpyAsync(ws.rjobs, rj.data(), sizeof(RefineJob) * count, cudaMemcpyHostToDevice, s));
+    PCD_CUDA(cudaMemcpyAsync(ws.rjobs, rj.data(), sizeof(RefreshJob) * count, cudaMemcpyHostToDevice, s));
     PCD_CUDA(cudaMemsetAsync(ws.ctl, 0, sizeof(Ctl) * count, s));
     PCD_CUDA(cudaMemsetAsync(ws.counter, 0, sizeof(unsigned), s));
-    PCD_CUDA(cudaMemsetAsync(ws.arena, 0, sizeof(float) * per, s));
-    if (!o.warm_start)
-        for (int i = 0; i < count; i++)
-            PCD_CUDA(cudaMemset2DAsync(inst[i].phi, sizeof(double) * inst[i].ld, 0, sizeof(double) * inst[i].width,
-                                       inst[i].height, s));
     // first right-hand side, ||b|| and the stop test of the starting phi
-    k_batch_refine_residual<<<blocks, kThreads, 0, s>>>(d_rjobs, count, o.tol, 1);
-    k_batch_refine_update<<<blocks, kThreads, 0, s>>>(d_rjobs, count);
-    PCD_LAUNCHED(2);
+    PCD_TRY(launch_first_refresh(d_rjobs, count, blocks, o.tol, !o.warm_start, s));
 
     // one CUDA graph per batch signature: the chunk's passes and the refresh
-    std::vector<long long> key = {count, tiles, blocks, chunk, grid, (long long)smem,
+    std::vector<long long> key = {count, tiles, blocks, chunk, narrow, grid, (long long)smem,
                                   (long long)(uintptr_t)ws.jobs, (long long)(uintptr_t)ws.rjobs};
     {
         long long tb;
@@ -1911,10 +1815,9 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         PCD_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         int st = PCD_OK;
         for (int k = 0; k < passes && st == PCD_OK; k++)
-            st = launch_tile_batch(d_jobs, count, tiles, std::min(4, chunk - 4 * k), k & 1, grid, smem, ws.counter,
-                                   s);
-        k_batch_refine_residual<<<blocks, kThreads, 0, s>>>(d_rjobs, count, o.tol, 0);
-        k_batch_refine_update<<<blocks, kThreads, 0, s>>>(d_rjobs, count);
+            st = launch_tile_batch(d_jobs, count, tiles, std::min(4, chunk - 4 * k), k & 1, k == 0, narrow, grid, smem,
+                                   ws.counter, s);
+        if (st == PCD_OK) st = launch_refresh(d_rjobs, RefreshJob{}, count, blocks, o.tol, s);
         cudaError_t ce = cudaStreamEndCapture(s, &g);
         if (st != PCD_OK) {
             if (ce == cudaSuccess) cudaGraphDestroy(g);
@@ -1943,7 +1846,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     bool finished = false;
     auto all_done = [&](const Ctl *c) {
         for (int i = 0; i < count; i++)
-            if (!c[i].done) return false;
+            if (!c[i].done && !c[i].error) return false;
         return true;
     };
     while (!finished) {
@@ -1952,7 +1855,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
             return PCD_TIMEOUT;
         }
         PCD_CUDA(cudaGraphLaunch(exec, s));
-        count_launches(passes + 2);
+        count_launches(passes + 1);
         const int slot = (int)(launched & 1);
         PCD_CUDA(cudaMemcpyAsync(ws.ctl_host + (size_t)slot * count, ws.ctl, sizeof(Ctl) * count,
                                  cudaMemcpyDeviceToHost, s));
@@ -1964,9 +1867,15 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
             if (all_done(ws.ctl_host + (size_t)prev * count)) finished = true;
         }
     }
+    PCD_TRY(launch_phi_settle(d_rjobs, RefreshJob{}, count, s));
     PCD_CUDA(cudaEventRecord(ws.t1, s));
     PCD_CUDA(cudaMemcpyAsync(ws.ctl_host, ws.ctl, sizeof(Ctl) * count, cudaMemcpyDeviceToHost, s));
     PCD_CUDA(cudaStreamSynchronize(s));
+    for (int k = 0; k < count; k++)
+        if (ws.ctl_host[k].error) {
+            set_error("batched tile solve: a bounded wait for a copy gave up");
+            return ws.ctl_host[k].error;
+        }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ws.t0, ws.t1);
     int all = 1;

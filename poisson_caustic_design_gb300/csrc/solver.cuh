@@ -127,8 +127,9 @@ struct SolverWorkspace {
 // Workspace of the batched tile solve (every grid of a batch in one tile
 // pass per launch); grows on demand.
 struct TileBatchWorkspace {
-    float *arena = nullptr;     // [all e][all e'][all r32], each grid H x ld
-    size_t arena_floats = 0;
+    float *arena = nullptr;     // [all e][all e'][all r32], H x ld floats a grid
+    double *phi2 = nullptr;     // second potential, H x ld a grid
+    size_t arena_cells = 0;
     Ctl *ctl = nullptr;         // one control block per grid
     Ctl *ctl_host = nullptr;    // pinned, 2 slots of cap blocks
     double *partials = nullptr; // residual partials per grid
@@ -139,7 +140,7 @@ struct TileBatchWorkspace {
     cudaEvent_t ev[2] = {nullptr, nullptr};
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     std::map<std::vector<long long>, cudaGraphExec_t> graphs;
-    int reserve(size_t floats, int count);
+    int reserve(size_t cells, int count);
     void release();
 };
 

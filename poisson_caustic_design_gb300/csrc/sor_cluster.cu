@@ -456,24 +456,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sor_cluster_tb(ClusterAr
 }
 
 #include "sor_cluster_rr.cuh"
-#include "sor_tile_rr.cuh"
-
-template <int K, bool TRACK>
-const void *tile_kernel_k(int L, int NQ)
-{
-    if (L == 3 && NQ == 2) return (const void *)k_sor_tile_rr<K, 3, 2, TRACK>;
-    if (L == 4 && NQ == 1) return (const void *)k_sor_tile_rr<K, 4, 1, TRACK>;
-    return nullptr;
-}
-
-// The tile pass for K sweeps, L rows per warp and NQ quads per lane (nullptr
-// outside the compiled set).
-const void *tile_kernel(int K, int L, int NQ, bool track)
-{
-    if (K == 4) return track ? tile_kernel_k<4, true>(L, NQ) : tile_kernel_k<4, false>(L, NQ);
-    if (K == 2) return track ? tile_kernel_k<2, true>(L, NQ) : tile_kernel_k<2, false>(L, NQ);
-    return nullptr;
-}
 
 }  // namespace
 
@@ -577,111 +559,6 @@ int cluster_plan(int dev, int W, int H, int max_depth, ClusterPlan *plan)
         }
     }
     return PCD_BAD_ARG;
-}
-
-int tile_plan(int dev, int W, int H, int ld, int depth, TilePlan *plan)
-{
-    if (W < 8 || H < 1 || W % 8 != 0 || ld % 4 != 0) return PCD_BAD_ARG;
-    if (depth != 0 && depth != 2 && depth != 4) return PCD_BAD_ARG;
-    const int K = depth ? depth : 4;
-    int sms = 0, max_smem = 0;
-    PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PCD_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const int WQ = W / 8;
-    TilePlan best{};
-    long best_cost = 0;
-    // tiles of 16 L rows and 256 NQ columns; a tile costs about L NQ quad
-    // updates per thread and half sweep whatever its interior
-    const int forms[2][2] = {{3, 2}, {4, 1}};
-    for (const auto &f : forms) {
-        const int L = f[0], NQ = f[1];
-        const int N = kRRWarps * L - 4 * K;
-        if (N < 1) continue;
-        const int ncol = ceil_div(WQ, 32 * NQ - 2), nrow = ceil_div(H, N);
-        const long cost = (long)ncol * nrow * L * NQ;
-        if (best.K && cost >= best_cost) continue;
-        const size_t smem = tile_floats(L, NQ) * sizeof(float);
-        if (smem + 2048 > (size_t)max_smem) continue;
-        int bps = 1;
-        for (int tr = 0; tr < 2; tr++) {
-            const void *fn = tile_kernel(K, L, NQ, tr != 0);
-            if (!fn) {
-                bps = 0;
-                break;
-            }
-            int b = 0;
-            PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kRRThreads, smem));
-            bps = std::min(bps, b);
-        }
-        if (bps < 1) continue;
-        best.K = K;
-        best.L = L;
-        best.NQ = NQ;
-        best.ncol = ncol;
-        best.nrow = nrow;
-        best.grid = (int)std::min<long>((long)ncol * nrow, (long)sms * bps);
-        best.smem = smem;
-        best_cost = cost;
-    }
-    if (!best.K) return PCD_BAD_ARG;
-    *plan = best;
-    return PCD_OK;
-}
-
-int launch_tile(const TilePlan &p, const float *ein, float *eout, const float *r32, Ctl *ctl, const SolveArgs &a,
-                int nsw, int out_idx, bool track, bool zero, cudaStream_t s)
-{
-    const void *fn = tile_kernel(p.K, p.L, p.NQ, track);
-    if (!fn || nsw < 1 || nsw > p.K) {
-        set_error("tile SOR: no kernel for this plan");
-        return PCD_BAD_ARG;
-    }
-    using Fn = void (*)(const float *, float *, const float *, Ctl *, SolveArgs, int, int, int, int, int);
-    reinterpret_cast<Fn>(const_cast<void *>(fn))<<<p.grid, kRRThreads, p.smem, s>>>(ein, eout, r32, ctl, a, p.ncol,
-                                                                                    p.nrow, nsw, out_idx, zero ? 1 : 0);
-    return PCD_OK;
-}
-
-void tile_counts(int W, int H, int *ncol, int *nrow)
-{
-    constexpr int L = 4, NQ = 1, K = 4;
-    *ncol = ceil_div(W / 8, 32 * NQ - 2);
-    *nrow = ceil_div(H, kRRWarps * L - 4 * K);
-}
-
-int tile_batch_config(int dev, int njobs, size_t *smem, int *grid)
-{
-    if (njobs < 1 || njobs > kTileBatchJobsMax) {
-        set_error("batched tile pass: 1 to " + std::to_string(kTileBatchJobsMax) + " grids");
-        return PCD_BAD_ARG;
-    }
-    const void *fn = (const void *)k_sor_tile_batch<4, 4, 1>;
-    const size_t base = tile_floats(4, 1) * sizeof(float), per_job = sizeof(TileJob) + sizeof(int);
-    const size_t most = base + kTileBatchJobsMax * per_job, bytes = base + (size_t)njobs * per_job;
-    int sms = 0, bps = 0;
-    PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-    PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kRRThreads, bytes));
-    if (bps < 1) {
-        set_error("batched tile pass: the kernel does not fit on an SM");
-        return PCD_BAD_ARG;
-    }
-    *smem = bytes;
-    *grid = sms * bps;
-    return PCD_OK;
-}
-
-int launch_tile_batch(const TileJob *d_jobs, int njobs, int ntiles, int nsw, int par, int grid, size_t smem,
-                      unsigned *counter, cudaStream_t s)
-{
-    if (njobs < 1 || njobs > kTileBatchJobsMax || ntiles < 1 || nsw < 1 || nsw > 4) {
-        set_error("batched tile pass: bad arguments");
-        return PCD_BAD_ARG;
-    }
-    k_sor_tile_batch<4, 4, 1>
-        <<<std::min(grid, ntiles), kRRThreads, smem, s>>>(d_jobs, njobs, ntiles, nsw, par, counter);
-    return PCD_OK;
 }
 
 int launch_cluster(ClusterArgs &a, const ClusterPlan &p, cudaStream_t s)

@@ -47,7 +47,6 @@ struct RRState {
     float4 e[2][L][NQ];      // both colours of the warp's rows
     float2 waa[NQ], wla[NQ], war[NQ];  // weight pairs: (wa, wa), (wl, wa), (wa, wr)
     bool act[NQ], eL[NQ], eR[NQ];
-    bool own[NQ];            // tile passes: quad in the tile's interior columns
     float w4, w3, w2, w1;
     int lane, w, H, ybase, R;
     unsigned edge_s, r_s;    // shared addresses of slot 4 * lane of edge row 0 / -r32 row 0
@@ -81,10 +80,9 @@ struct RRState {
     }
 
     // Half sweep of colour CC over plane rows [lo, hi); P = parity of the
-    // grid row of the warp's first row.  TR: mx takes the largest |update| of
-    // the cells of plane rows [olo, ohi) in quads marked own.
-    template <int CC, int P, bool TR = false>
-    __device__ __forceinline__ void half(int lo, int hi, float *mx = nullptr, int olo = 0, int ohi = 0)
+    // grid row of the warp's first row.
+    template <int CC, int P>
+    __device__ __forceinline__ void half(int lo, int hi)
     {
         constexpr int OC = 1 - CC;
         float4 eu[NQ], ed[NQ];
@@ -127,7 +125,6 @@ struct RRState {
                     const float4 d = j + 1 < L ? e[OC][j + 1 < L ? j + 1 : j][i] : ed[i];
                     const float4 nv =
                         quad_ghost_q(q, v, rh, u, d, e[OC][j][i], ex, q ? wla[i] : waa[i], q ? waa[i] : war[i]);
-                    if (TR && own[i] && lr0 + j >= olo && lr0 + j < ohi) *mx = fmaxf(*mx, quad_max_change(v, nv));
                     e[CC][j][i] = nv;
                 }
             }
@@ -159,7 +156,6 @@ struct RRState {
                     const float we = !on ? 0.f : edge ? (brd ? (two ? w2 : w1) : w3) : a;
                     const float2 wA = make_float2(q ? we : a, a), wB = make_float2(a, q ? a : we);
                     const float4 nv = quad_ghost_q(q, v, rh, u, d, e[OC][j][i], ex, wA, wB);
-                    if (TR && on && own[i] && lr >= olo && lr < ohi) *mx = fmaxf(*mx, quad_max_change(v, nv));
                     e[CC][j][i] = nv;
                 }
             }

@@ -52,12 +52,6 @@ __device__ __forceinline__ float4 quad_ghost_q(int q, const float4 &v, const flo
     return make_float4(nA.x, nA.y, nB.x, nB.y);
 }
 
-// Largest |nv - v| over the quad (a NaN change does not raise it).
-__device__ __forceinline__ float quad_max_change(const float4 &v, const float4 &nv)
-{
-    return fmaxf(fmaxf(fabsf(nv.x - v.x), fabsf(nv.y - v.y)), fmaxf(fabsf(nv.z - v.z), fabsf(nv.w - v.w)));
-}
-
 // Sum of squares of r32 - L v over the quad (ghost neighbours; nrh is -r32).
 __device__ __forceinline__ float quad_ghost_res2(int q, const float4 &v, const float4 &nrh, const float4 &u,
                                                 const float4 &d, const float4 &m, float ex)
@@ -79,6 +73,22 @@ __device__ __forceinline__ float quad_ghost_res2(int q, const float4 &v, const f
 struct Quad {
     float2 a, b;
 };
+
+// The layout of a grid in HBM that the tiles read and write (the correction and
+// minus its right-hand side): a row is KQ = ceil(W / 8) quads of its cells at
+// even columns, then KQ quads of those at odd ones, a quad's floats in the order
+// (a, b).  A lane's quad is one aligned 16-byte access, 16 lanes one run of 256
+// bytes, and the quad lands in whole register pairs.  (From a row-major grid a
+// lane read 32 bytes in two half-used accesses, and the registers of those
+// loads, two cells of which make a pair, stayed tied to the sweep loop: 2700
+// instructions a warp and tile pass against 1700.)
+__host__ __device__ inline long quad_row_floats(int W) { return 8l * ((W + 7) / 8); }
+// the float of cell (x, y) in its row: column x
+__host__ __device__ inline int quad_column(int x, int KQ)
+{
+    const int t = (x >> 1) & 3;
+    return ((x & 1) * KQ + (x >> 3)) * 4 + ((t & 1) << 1 | t >> 1);
+}
 
 __device__ __forceinline__ Quad quad_zero() { return {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
 __device__ __forceinline__ Quad ldsq(unsigned p)
@@ -114,6 +124,7 @@ __device__ __forceinline__ Quad quad_defect(int q, const Quad &v, const Quad &nr
     return {__fadd2_rn(__ffma2_rn(ca, v.a, s.a), nrh.a), __fadd2_rn(__ffma2_rn(cb, v.b, s.b), nrh.b)};
 }
 
+// Largest |nv - v| over the quad (a NaN change does not raise it).
 __device__ __forceinline__ float quad_max_change(const Quad &v, const Quad &nv)
 {
     return fmaxf(fmaxf(fabsf(nv.a.x - v.a.x), fabsf(nv.a.y - v.a.y)),

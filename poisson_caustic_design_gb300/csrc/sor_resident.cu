@@ -9,22 +9,10 @@
 // sweeps ends inside the halo, whose values are recomputed with the owner's
 // arithmetic and thrown away at the next exchange.
 //
-// Layout: a lane holds L consecutive rows of one lane column (eight cells: one
-// quad of each colour, sor_quads.cuh).  CL lanes side by side make a tile row,
-// so a warp holds 32 / CL groups of L rows.  Horizontal neighbours come by
-// shuffle from the next lane, vertical ones from the lane's own registers and,
-// between groups, from the groups' edge rows in shared memory (double-buffered
-// by colour: one block barrier a half sweep).
-//
-// Exchange: every 32-bit value travels in a 64-bit word together with the
-// epoch it belongs to; the reader polls the words themselves.  No fence, no
-// flag and no second trip stand between a neighbour's store and this CTA's
-// use: a microbenchmark of fence + flag + poll + load needed 4-5 us for the
-// same exchange (sor_blocks.cu pays it).  Words are double-buffered by epoch
-// parity: a CTA overwrites epoch n's word with epoch n + 2 only after it read
-// its neighbours' epoch n + 1, which they publish after reading epoch n.
-// A 64-bit relaxed access is single-copy atomic, so value and epoch are never
-// torn; a vector of two is two such accesses.
+// The lanes' part of a tile is sor_tile.cuh's, the exchange's words those of
+// words.cuh, double-buffered by epoch parity: a CTA overwrites epoch n's word
+// with epoch n + 2 only after it read its neighbours' epoch n + 1, which they
+// publish after reading epoch n.
 //
 // Two ways to end a launch:
 //   cycle   an FP32 estimate of ||r32 - L e|| every check_every sweeps, its
@@ -43,74 +31,29 @@
 // sor_cluster_rr.cuh): 16 half sweeps of about 470 cycles (64 instructions a
 // warp; shuffle, edge row, five dependent packed operations, block barrier)
 // and about 2900 cycles of exchange a round; 1.15-1.2 us at 1024^2 against
-// 5.7 of the tile passes.  Measured on the way: a quad held as consecutive
-// cells needs three packed registers a half sum (35 instructions a quad
-// against 24); -r32 in registers doubles the two-row form's instructions by
-// register moves; a separate update for the border rows set the pace of the
-// grid (0.59 against 0.72 us on one tile); 16-byte exchange accesses fetch
+// 5.7 of the tile passes of that time.  Measured on the way: a separate update
+// for the border rows set the pace of the
+// grid (0.72 against 0.59 us on one tile); 16-byte exchange accesses fetch
 // each sector twice (1.48 against 1.15 us a sweep at 1024^2); publishing each
 // colour as it becomes final gains nothing.
 #include <algorithm>
 
 #include "sor_resident.cuh"
-#include "sor_quads.cuh"
+#include "sor_tile.cuh"
+#include "words.cuh"
 
 namespace pcd {
 
 namespace {
 
-using namespace quads;
-
-__device__ __forceinline__ unsigned long long rs_word(float v, unsigned ep)
-{
-    return (unsigned long long)__float_as_uint(v) | ((unsigned long long)ep << 32);
-}
-
-// Four words, one 32-byte sector: a quad in one access (two 16-byte ones fetch
-// the sector twice, and the words of a halo fill the SM's L2 port as it is).
-struct Words {
-    unsigned long long x, y, z, w;
-};
-
-__device__ __forceinline__ void rs_st4(Words *p, const Words &v)
-{
-    asm volatile("st.relaxed.gpu.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v.x), "l"(v.y), "l"(v.z), "l"(v.w)
-                 : "memory");
-}
-
-__device__ __forceinline__ Words rs_ld4(const Words *p)
-{
-    Words v;
-    asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
-                 : "=l"(v.x), "=l"(v.y), "=l"(v.z), "=l"(v.w)
-                 : "l"(p)
-                 : "memory");
-    return v;
-}
-
-__device__ __forceinline__ unsigned long long rs_ld1(const unsigned long long *p)
-{
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void rs_st1(unsigned long long *p, unsigned long long v)
-{
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
+using namespace tile;
+using namespace words;
 
 __device__ __forceinline__ unsigned rs_ld_acquire(const unsigned *p)
 {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
-}
-
-__device__ __forceinline__ bool rs_fresh(const Words &v, unsigned ep)
-{
-    return (unsigned)(v.x >> 32) == ep && (unsigned)(v.y >> 32) == ep && (unsigned)(v.z >> 32) == ep &&
-           (unsigned)(v.w >> 32) == ep;
 }
 
 __device__ __forceinline__ Quad rs_quad(const Words &v)
@@ -121,193 +64,16 @@ __device__ __forceinline__ Quad rs_quad(const Words &v)
 
 __device__ __forceinline__ Words rs_words(const Quad &q, unsigned ep)
 {
-    return {rs_word(q.a.x, ep), rs_word(q.a.y, ep), rs_word(q.b.x, ep), rs_word(q.b.y, ep)};
-}
-
-// One more unsuccessful poll: false once the poll budget is spent (then
-// PCD_TIMEOUT is recorded) or another CTA recorded an error.
-__device__ __forceinline__ bool rs_again(const ResidentArgs &a, long long &it)
-{
-    if ((++it & 63) == 0) {
-        if (*(volatile const int *)&a.ctl->error) return false;
-        if (it > a.spin_limit) {
-            atomicCAS(&a.ctl->error, 0, PCD_TIMEOUT);
-            return false;
-        }
-    }
-    return true;
+    return {word(__float_as_uint(q.a.x), ep), word(__float_as_uint(q.a.y), ep), word(__float_as_uint(q.b.x), ep),
+            word(__float_as_uint(q.b.y), ep)};
 }
 
 // Most warps of a CTA: as few as the tiles need, for the registers that L rows
 // of both colours take (512 threads of 128 registers spill from L = 4 on).
 __host__ __device__ constexpr int rs_warps(int L) { return L == 2 ? 16 : 12; }
 
-template <int K, int L, int CL, bool RAG>
-struct Tile {
-    static constexpr int G = 32 / CL;              // row groups of a warp
-    static constexpr int NS = RAG ? 2 : 1;         // weight sets of a row: one per parity where lanes differ
-    static_assert(L % 2 == 0, "groups start on even grid rows");
-
-    Quad e[2][L];
-    // Per row: weight omega / cnt (0 outside the grid), as pairs.
-    //   whole lane columns: wa both horizontal neighbours, wb the pair with
-    //   the grid's first or last cell
-    //   RAG: wa / wb of the quad's pairs by parity, and the coefficient of the
-    //   cell's own value (-3 in a last column inside its lane, whose right
-    //   neighbour reads 0)
-    float2 wa[NS][L], wb[NS][L], ca[2], cb[2];
-    bool own, zl, zr;
-    bool brd, gin;           // warp with the grid's first or last row; group with a row of the grid
-    int cl, gi, lr0, y0, H, nvalid;
-    int wlo, whi;            // plane rows of the warp's groups
-    unsigned edge_own, edge_up, edge_dn, edge_c;  // shared addresses; edge_c: bytes from colour 0 to 1
-    unsigned r_s, r_c;       // -r32 planes: shared address of the first row, bytes between colours
-
-    // w4, w3, w2: omega / cnt
-    __device__ __forceinline__ void setup_weights(bool act, int R, float w4, float w3, float w2)
-    {
-#pragma unroll
-        for (int j = 0; j < L; j++) {
-            const int y = y0 + j;
-            const bool in = act && lr0 + j < R && y >= 0 && y < H, mid = y > 0 && y < H - 1;
-            const float wi = !in ? 0.f : mid ? w4 : w3, we = !in ? 0.f : mid ? w3 : w2;
-            if (RAG) {
-#pragma unroll
-                for (int q = 0; q < NS; q++) {
-                    float w[4];
-#pragma unroll
-                    for (int t = 0; t < 4; t++) {
-                        const int off = 2 * t + 1 - q, last = nvalid - 1;
-                        const bool edge = (off == 0 && zl) || (off == 7 && zr) || (off == last && nvalid < 8);
-                        w[t] = off > last ? 0.f : edge ? we : wi;
-                    }
-                    wa[q][j] = make_float2(w[0], w[2]);
-                    wb[q][j] = make_float2(w[1], w[3]);
-                }
-            } else {
-                wa[0][j] = make_float2(wi, wi);
-                wb[0][j] = zl ? make_float2(we, wi) : zr ? make_float2(wi, we) : make_float2(wi, wi);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            auto c = [&](int t) { return RAG && nvalid < 8 && 2 * t + 1 - q == nvalid - 1 ? -3.f : -4.f; };
-            ca[q] = make_float2(c(0), c(2));
-            cb[q] = make_float2(c(1), c(3));
-        }
-    }
-    __device__ __forceinline__ float2 weight_a(int q, int j) const { return RAG ? wa[RAG ? q : 0][j] : q && zl ? wb[0][j] : wa[0][j]; }
-    __device__ __forceinline__ float2 weight_b(int q, int j) const { return RAG ? wb[RAG ? q : 0][j] : !q && zr ? wb[0][j] : wa[0][j]; }
-
-    // Publishes the group's edge rows of colour CC.  The grid's first and last
-    // row also go, as the other colour, into the rows just outside the grid:
-    // a missing vertical neighbour takes the cell's own value.  (Those rows
-    // weigh 0, and groups outside the grid publish nothing, so nobody else
-    // writes them.)  Every warp runs the same update; a separate form for the
-    // border rows would set the pace of the whole grid.
-    template <int CC>
-    __device__ __forceinline__ void put_edges()
-    {
-        constexpr int OC = 1 - CC;
-        if (brd) {
-#pragma unroll
-            for (int j = 0; j < L; j++) {
-                if (y0 + j == 0) {
-                    if (j > 0) e[OC][j > 0 ? j - 1 : 0] = e[CC][j];
-                    else stsq(edge_up + (OC ? edge_c : 0u), e[CC][j]);
-                }
-                if (y0 + j == H - 1) {
-                    if (j + 1 < L) e[OC][j + 1 < L ? j + 1 : j] = e[CC][j];
-                    else stsq(edge_dn + (OC ? edge_c : 0u), e[CC][j]);
-                }
-            }
-        }
-        if (gin) {
-            const unsigned a = edge_own + (CC ? edge_c : 0u);
-            stsq(a, e[CC][0]);
-            stsq(a + 16u * CL, e[CC][L - 1]);
-        }
-    }
-
-    // the other colour's cell beyond the lane's eight columns, or beyond the
-    // grid the cell's own value
-    __device__ __forceinline__ float beyond(int q, const Quad &m, const Quad &v) const
-    {
-        const float x = q ? __shfl_up_sync(0xffffffffu, m.b.y, 1) : __shfl_down_sync(0xffffffffu, m.a.x, 1);
-        return (q ? zl : zr) ? (q ? v.a.x : v.b.y) : x;
-    }
-
-    __device__ __forceinline__ Quad rhs(int c, int j) const
-    {
-        return ldsq(r_s + (c ? r_c : 0u) + 16u * (unsigned)(CL * j));
-    }
-
-    // The negated residual of row j's quad of colour CC.
-    template <int CC>
-    __device__ __forceinline__ Quad defect(int j, const Quad &eu, const Quad &ed) const
-    {
-        constexpr int OC = 1 - CC;
-        const int q = 1 - ((j ^ CC) & 1);  // the group's first row is even
-        const Quad &v = e[CC][j], &m = e[OC][j];
-        const float ex = beyond(q, m, v);
-        return quad_defect(q, v, rhs(CC, j), j > 0 ? e[OC][j > 0 ? j - 1 : 0] : eu,
-                           j + 1 < L ? e[OC][j + 1 < L ? j + 1 : j] : ed, m, ex, RAG ? ca[q] : make_float2(-4.f, -4.f),
-                           RAG ? cb[q] : make_float2(-4.f, -4.f));
-    }
-
-    // Half sweep of colour CC.  TR: mx takes the largest |update| of the tile's
-    // own cells (plane rows [olo, ohi)).
-    template <int CC, bool TR>
-    __device__ __forceinline__ void half(float &mx, int olo, int ohi)
-    {
-        constexpr int OC = 1 - CC;
-        const Quad eu = ldsq(edge_up + (OC ? edge_c : 0u));
-        const Quad ed = ldsq(edge_dn + (OC ? edge_c : 0u));
-#pragma unroll
-        for (int j = 0; j < L; j++) {
-            const int q = 1 - ((j ^ CC) & 1);
-            const Quad t = defect<CC>(j, eu, ed), v = e[CC][j];
-            const Quad nv = {__ffma2_rn(weight_a(q, j), t.a, v.a), __ffma2_rn(weight_b(q, j), t.b, v.b)};
-            if (TR && own && lr0 + j >= olo && lr0 + j < ohi) mx = fmaxf(mx, quad_max_change(v, nv));
-            e[CC][j] = nv;
-        }
-        put_edges<CC>();
-    }
-
-    template <int CC>
-    __device__ __forceinline__ float residual_of(int olo, int ohi) const
-    {
-        constexpr int OC = 1 - CC;
-        float acc = 0.f;
-        const Quad eu = ldsq(edge_up + (OC ? edge_c : 0u));
-        const Quad ed = ldsq(edge_dn + (OC ? edge_c : 0u));
-#pragma unroll
-        for (int j = 0; j < L; j++) {
-            const int o = (j ^ CC) & 1;  // offset of the quad's first cell
-            Quad r = defect<CC>(j, eu, ed);
-            if (RAG) {
-                r.a.x = o < nvalid ? r.a.x : 0.f;
-                r.b.x = o + 2 < nvalid ? r.b.x : 0.f;
-                r.a.y = o + 4 < nvalid ? r.a.y : 0.f;
-                r.b.y = o + 6 < nvalid ? r.b.y : 0.f;
-            }
-            const float s2 = fmaf(r.a.x, r.a.x, fmaf(r.b.x, r.b.x, fmaf(r.a.y, r.a.y, r.b.y * r.b.y)));
-            acc += own && lr0 + j >= olo && lr0 + j < ohi ? s2 : 0.f;
-        }
-        return acc;
-    }
-    // Sum of (r32 - L e)^2 over the lane's own cells of plane rows [olo, ohi).
-    __device__ __forceinline__ float residual(int olo, int ohi) const
-    {
-        return residual_of<0>(olo, ohi) + residual_of<1>(olo, ohi);
-    }
-};
-
-// Shared memory of a CTA: the groups' edge rows and, for each colour, one
-// row above the first group and one below the last, the -r32 planes, the landing planes of the halo quads (the same
-// shape, only halo places written) and the table of the halo quads.
-__host__ __device__ inline size_t rs_edge_quads(int CL, int NG) { return (size_t)4 * (NG + 1) * CL; }
-__host__ __device__ inline size_t rs_plane_quads(int L, int CL, int NG) { return (size_t)2 * NG * L * CL; }
+// Shared memory of a CTA: the tile's, the landing planes of the halo quads (the
+// -r32 planes' shape, only halo places written) and the table of the halo quads.
 // halo quads of a tile with n own rows: the rows above and below, then the
 // lane columns left and right of the own rows
 __host__ __device__ inline int rs_halo_quads(int K, int CL, int n)
@@ -316,15 +82,15 @@ __host__ __device__ inline int rs_halo_quads(int K, int CL, int n)
 }
 inline size_t rs_smem(int K, int L, int CL, int NG, int n, bool exchange)
 {
-    size_t b = (rs_edge_quads(CL, NG) + rs_plane_quads(L, CL, NG)) * sizeof(Quad);
-    if (exchange) b += rs_plane_quads(L, CL, NG) * sizeof(Quad) + (size_t)rs_halo_quads(K, CL, n) * sizeof(uint2);
+    size_t b = (edge_quads(CL, NG) + plane_quads(L, CL, NG)) * sizeof(Quad);
+    if (exchange) b += plane_quads(L, CL, NG) * sizeof(Quad) + (size_t)rs_halo_quads(K, CL, n) * sizeof(uint2);
     return b;
 }
 
 template <int K, int L, int CL, bool RAG>
 __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentArgs a)
 {
-    using T = Tile<K, L, CL, RAG>;
+    using T = Tile<L, CL, RAG>;
     constexpr int HK = 2 * K, HL = HK / 8;  // halo rows, halo lane columns
     static_assert(K % 4 == 0, "the halo is a whole number of lane columns");
     extern __shared__ __align__(16) float smem_f[];
@@ -354,10 +120,7 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
     const int ybase = yb - hr, qbase = qb - hl;
 
     T st;
-    st.cl = lane & (CL - 1);
-    const int h = lane / CL;
-    st.gi = w * T::G + h;
-    st.lr0 = st.gi * L;
+    st.place(smem_f, a.NG);
     st.y0 = ybase + st.lr0;
     const int q = qbase + st.cl;
     const bool act = st.cl < nq + 2 * hl && q >= 0 && q < a.KQ;
@@ -366,24 +129,16 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
     st.nvalid = min(8, a.W - 8 * q);
     st.zr = q == a.KQ - 1 && st.nvalid == 8;
     st.H = a.H;
-    st.setup_weights(act, R, a.w32[4], a.w32[3], a.w32[2]);
+    st.setup_weights(act, R, a.w32);
     st.gin = st.y0 < a.H && st.y0 + L > 0;
     st.brd = __any_sync(0xffffffffu, st.gin && (st.y0 <= 0 || st.y0 + L >= a.H));
-    st.wlo = w * T::G * L;
-    st.whi = (w + 1) * T::G * L;
-    const unsigned edge_s = (unsigned)__cvta_generic_to_shared(smem_f);
-    const unsigned grow = 16u * CL;  // bytes of one edge row
-    st.edge_c = 2u * ((unsigned)a.NG + 1u) * grow;
-    st.edge_own = edge_s + (unsigned)(st.gi * 2) * grow + 16u * st.cl;
-    st.edge_up = edge_s + (unsigned)(st.gi > 0 ? 2 * st.gi - 1 : 2 * a.NG) * grow + 16u * st.cl;
-    st.edge_dn = edge_s + (unsigned)(st.gi < a.NG - 1 ? 2 * st.gi + 2 : 2 * a.NG + 1) * grow + 16u * st.cl;
-    for (unsigned z = threadIdx.x; z < rs_edge_quads(CL, a.NG); z += NT) stsq(edge_s + 16u * z, quad_zero());
-    Quad *rp = reinterpret_cast<Quad *>(smem_f) + rs_edge_quads(CL, a.NG);
-    st.r_c = (unsigned)(a.NG * L) * grow;
-    st.r_s = (unsigned)__cvta_generic_to_shared(rp) + (unsigned)st.lr0 * grow + 16u * st.cl;
-    Quad *land = rp + rs_plane_quads(L, CL, a.NG);
-    uint2 *table = reinterpret_cast<uint2 *>(land + rs_plane_quads(L, CL, a.NG));
-    const unsigned land_s = st.r_s + 2u * st.r_c;  // the lane's place in the landing planes
+    for (unsigned z = threadIdx.x; z < edge_quads(CL, a.NG); z += NT) reinterpret_cast<Quad *>(smem_f)[z] = quad_zero();
+    Quad *rp = reinterpret_cast<Quad *>(smem_f) + edge_quads(CL, a.NG);
+    Quad *land = rp + plane_quads(L, CL, a.NG);
+    uint2 *table = reinterpret_cast<uint2 *>(land + plane_quads(L, CL, a.NG));
+    constexpr unsigned grow = 16u * CL;  // bytes of a plane's row
+    // the lane's place in the landing planes, which are one of each colour
+    const unsigned land_s = st.r_s + 2u * st.r_c;
     const unsigned xplane = (unsigned)a.H * (unsigned)a.KQ;  // exchange quads of one colour
     // rows of the lane that go out (pub) and come in (imp) at an exchange
     unsigned pub = 0, imp = 0;
@@ -428,27 +183,11 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
     // ---- -r32 of the tile and its halo; e = 0
 #pragma unroll
     for (int j = 0; j < L; j++) {
-        const int lr = st.lr0 + j, y = st.y0 + j, par = y & 1;
-        float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A;
-        if (lr < R && y >= 0 && y < a.H && act) {
-            const float *p = a.r32 + (size_t)y * a.ld + 8 * q;
-            if (a.vec && st.nvalid == 8) {
-                A = *reinterpret_cast<const float4 *>(p);
-                B = *reinterpret_cast<const float4 *>(p + 4);
-            } else {
-                float t[8];
-#pragma unroll
-                for (int k = 0; k < 8; k++) t[k] = k < st.nvalid ? p[k] : 0.f;
-                A = make_float4(t[0], t[1], t[2], t[3]);
-                B = make_float4(t[4], t[5], t[6], t[7]);
-            }
-        }
-        const Quad ev = {make_float2(-A.x, -B.x), make_float2(-A.z, -B.z)};
-        const Quad od = {make_float2(-A.y, -B.y), make_float2(-A.w, -B.w)};
-        // colour c holds the cells at offsets ((y & 1) ^ c) + 2 t
-        stsq(st.r_s + grow * (unsigned)j, par ? od : ev);
-        stsq(st.r_s + st.r_c + grow * (unsigned)j, par ? ev : od);
+        const int lr = st.lr0 + j, y = st.y0 + j;
+        const bool in = lr < R && y >= 0 && y < a.H && act;
+        st.copy_row(st.r_s, j, a.r32 + (in ? (long)y * 8 * a.KQ : 0), q, a.KQ, in);
     }
+    st.copies_wait();
     const double bnorm = ((volatile const Ctl *)ctl)->bnorm;
     const double rstart = ((volatile const Ctl *)ctl)->rnorm;
     if (threadIdx.x == 0) {
@@ -464,17 +203,7 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
         for (int j = 0; j < L; j++) {
             const int lr = st.lr0 + j, y = st.y0 + j;
             if (!st.own || lr < hr || lr >= hr + n) continue;
-            const Quad ev = (y & 1) ? st.e[1][j] : st.e[0][j], od = (y & 1) ? st.e[0][j] : st.e[1][j];
-            float *p = a.e + (size_t)y * a.ld + 8 * q;
-            if (a.vec && st.nvalid == 8) {
-                *reinterpret_cast<float4 *>(p) = make_float4(ev.a.x, od.a.x, ev.b.x, od.b.x);
-                *reinterpret_cast<float4 *>(p + 4) = make_float4(ev.a.y, od.a.y, ev.b.y, od.b.y);
-            } else {
-                const float t[8] = {ev.a.x, od.a.x, ev.b.x, od.b.x, ev.a.y, od.a.y, ev.b.y, od.b.y};
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                    if (k < st.nvalid) p[k] = t[k];
-            }
+            st.store_row(j, a.e + (long)y * 8 * a.KQ, q, a.KQ);
         }
     };
 
@@ -549,7 +278,7 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
                         x = warp_sum_f(x);
                         if (lane == 0) {
                             if (G == 1) s_tot = x;
-                            else if (!(a.withhold && g == 0)) rs_st1(a.part + (size_t)(ck & 1) * G + g, rs_word(x, ck));
+                            else if (!(a.withhold && g == 0)) st1(a.part + (size_t)(ck & 1) * G + g, word(__float_as_uint(x), ck));
                         }
                     }
                     to_post = false;
@@ -564,10 +293,10 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
                 for (int t = threadIdx.x; t < G; t += NT) {
                     const unsigned long long *p = a.part + (size_t)(ck & 1) * G + t;
                     long long it = 0;
-                    unsigned long long v = rs_ld1(p);
+                    unsigned long long v = ld1(p);
                     while ((unsigned)(v >> 32) != ck && !failed) {
-                        if (!rs_again(a, it)) failed = true;
-                        v = rs_ld1(p);
+                        if (!again(&a.ctl->error, a.spin_limit, it)) failed = true;
+                        v = ld1(p);
                     }
                     s_vals[t] = __uint_as_float((unsigned)v);
                 }
@@ -581,8 +310,8 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
 #pragma unroll
                     for (int j = 0; j < L; j++, p += a.KQ)
                         if (pub >> j & 1u) {
-                            rs_st4(p, rs_words(st.e[0][j], ep));
-                            rs_st4(p + xplane, rs_words(st.e[1][j], ep));
+                            st4(p, rs_words(st.e[0][j], ep));
+                            st4(p + xplane, rs_words(st.e[1][j], ep));
                         }
                 }
                 // ---- halo quads in
@@ -601,18 +330,18 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
                         Words v[U];
 #pragma unroll
                         for (int u = 0; u < U; u++)
-                            if (at[u].x != ~0u) v[u] = rs_ld4(xb + at[u].x);
+                            if (at[u].x != ~0u) v[u] = ld4(xb + at[u].x);
 #pragma unroll
                         for (int u = 0; u < U; u++)
                             if (at[u].x != ~0u) {
-                                if (rs_fresh(v[u], ep)) {
+                                if (fresh(v[u], ep)) {
                                     land[at[u].y] = rs_quad(v[u]);
                                     at[u].x = ~0u;
                                 } else {
                                     any = true;
                                 }
                             }
-                        if (any && !rs_again(a, it)) failed = true;
+                        if (any && !again(&a.ctl->error, a.spin_limit, it)) failed = true;
                     }
                 }
                 __syncthreads();
@@ -670,7 +399,7 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
             if (threadIdx.x == 0) {
                 long long it = 0;
                 while (rs_ld_acquire(a.bar) < (unsigned)G && !failed)
-                    if (!rs_again(a, it)) failed = true;
+                    if (!again(&a.ctl->error, a.spin_limit, it)) failed = true;
             }
             if (__syncthreads_or(failed)) { failed = true; break; }
         } else {
@@ -822,7 +551,6 @@ int launch_resident(ResidentArgs &a, const ResidentPlan &p, cudaStream_t s)
     a.TY = p.TY;
     a.NG = p.NG;
     a.R = p.R;
-    a.vec = a.ld % 4 == 0;
     PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
     void *params[] = {&a};
     if (p.TX * p.TY == 1) PCD_CUDA(cudaLaunchKernel(fn, dim3(1), dim3(32 * p.NW), params, p.smem, s));

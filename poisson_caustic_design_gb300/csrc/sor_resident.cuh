@@ -10,12 +10,12 @@ constexpr int kResidentChecksMax = 512;  // tracked sweeps of one launch
 constexpr int kResidentCtasMax = 256;
 
 struct ResidentArgs {
-    int W, H, ld;
+    int W, H;
     int KQ;              // lane columns of the grid (8 cells each)
     int TX, TY;          // tile columns x tile rows = CTAs
     int NG, R;           // row groups of a CTA, most rows of any tile (halo included)
-    float *e;            // FP32 correction, out
-    const float *r32;    // FP32 right-hand side
+    float *e;            // FP32 correction, out (in the layout of sor_quads.cuh, as r32)
+    const float *r32;    // minus the FP32 right-hand side
     Ctl *ctl;
     void *xb;            // exchange words: [2 parities][2 colours][H][KQ] x 32 bytes
     unsigned long long *part;  // residual partials: [2][CTAs] words
@@ -29,7 +29,6 @@ struct ResidentArgs {
     int gran;            // max-update stop: tracked every gran sweeps; 0: not tracked
     double tol, drop;
     float w32[5];
-    int vec;             // rows 16-byte aligned
     long long spin_limit;
     int withhold;        // failure test: CTA 0 never publishes
 };

@@ -1,0 +1,73 @@
+"""FP32 tile passes over grids in HBM, at the edges of their tiles (80 or 88
+written rows, 14 lane columns of 8 cells): the launch-per-half-sweep kernels'
+iterates, in a single solve and in a batch."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import poisson_caustic_design_gb300 as pcd
+
+    c = pcd.Context(0)
+    yield c
+    c.close()
+
+
+def _problem(n, m):
+    import torch
+
+    import poisson_caustic_design_gb300 as pcd
+
+    b = pcd.inputs.poisson_rhs(max(n, m), 4, "binary" if n % 16 else "gaussian", m=max(n, m))[:m, :n]
+    b = b - b.mean()
+    start = 1e-2 * np.add.outer(np.cos(np.arange(m) / 7.0), np.sin(np.arange(n) / 5.0))
+    return torch.from_numpy(np.ascontiguousarray(b)).cuda(), torch.from_numpy(start).cuda()
+
+
+def _agree(x, ref):
+    """FP32 rounding of the corrections, the other schedules' tolerance."""
+    return bool((x - ref).abs().max() < 1e-5 * ref.abs().max())
+
+
+@pytest.mark.parametrize("n", [8, 16, 112, 120, 128, 232])
+@pytest.mark.parametrize("m", [1, 2, 15, 80, 81, 89, 161])
+@pytest.mark.parametrize("check_every,sweeps", [(4, 1), (4, 43), (2, 37)])
+def test_tile_edges(ctx, n, m, check_every, sweeps):
+    import poisson_caustic_design_gb300 as pcd
+
+    b, start = _problem(n, m)
+    out = {}
+    for sched in (1, 6):
+        phi = start.clone()
+        st = ctx.solve_device(b, phi, pcd.SolveOptions(
+            stop=pcd.STOP_REL_RESIDUAL, tol=0.0, max_iterations=sweeps, precision=pcd.PREC_MIXED, omega=1.8,
+            warm_start=1, schedule=sched, check_every=check_every if sched == 6 else 0, refine_every=16))
+        assert st["sweeps"] == sweeps and st["schedule_used"] == sched
+        out[sched] = phi
+    assert _agree(out[6], out[1])
+
+
+@pytest.mark.parametrize("zero_start", [False, True])
+@pytest.mark.parametrize("narrow", [False, True])
+def test_batch_tile_edges(ctx, zero_start, narrow):
+    """Grids of unlike sizes in one batch, up to the sweep cap in the middle of
+    a pass, are the single solves."""
+    import torch
+
+    import poisson_caustic_design_gb300 as pcd
+
+    sizes = [(80, 112), (81, 120), (2, 16), (161, 232), (96, 128), (300, 1016)] + [(33, 8)] * narrow
+    probs = [_problem(n, m) for m, n in sizes]
+    o = dict(stop=pcd.STOP_REL_RESIDUAL, tol=1e-14, max_iterations=43, precision=pcd.PREC_MIXED, omega=1.8,
+             refine_every=16)
+    phis = [torch.full_like(s, 7.0) if zero_start else s.clone() for _, s in probs]
+    stats, _ = pcd.solver.batch_solve(ctx, [b for b, _ in probs], phis,
+                                      pcd.SolveOptions(warm_start=0 if zero_start else 1, **o))
+    for (b, s), phi, st in zip(probs, phis, stats):
+        assert st["sweeps"] == 43
+        ref = torch.zeros_like(s) if zero_start else s.clone()
+        ctx.solve_device(b, ref, pcd.SolveOptions(schedule=1, warm_start=1, **o))
+        assert _agree(phi, ref)
