@@ -644,6 +644,25 @@ int launch_stripes(T *phi, const T *rhs, Ctl *ctl, const SolveArgs &a, int R, in
     return PCD_OK;
 }
 
+// Polls of a tagged word before a wait gives up: each is an L2 trip, together
+// about two seconds.
+constexpr long long kWordPolls = 1ll << 21;
+
+// The tagged words' buffer, zeroed: tags start at 1 in every solve, and no word
+// of an earlier one may match.
+int reserve_words(SolverWorkspace &ws, size_t need, cudaStream_t s)
+{
+    if (need > ws.rx_bytes) {
+        if (ws.rx) cudaFree(ws.rx);
+        ws.rx = nullptr;
+        ws.rx_bytes = 0;
+        PCD_CUDA(cudaMalloc(&ws.rx, need));
+        ws.rx_bytes = need;
+    }
+    PCD_CUDA(cudaMemsetAsync(ws.rx, 0, need, s));
+    return PCD_OK;
+}
+
 // The FP64 refresh of a single solve: the potential alternates between phi and
 // the workspace's r64.
 RefreshJob refresh_job(const SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a)
@@ -693,17 +712,11 @@ int enqueue_chunk(SolverWorkspace &ws, const double *b, double *phi, const Solve
         sweeps = 0;
     }
     if (!MASKED && sched == PCD_SCHED_TILES) {
-        // as the stream passes: pass k reads buffer k&1 and writes the other
         TileMaps maps;
-        PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, sp.tile.rows + 4 * sp.tile.K, &maps));
-        int k = 0;
-        for (int done = 0; done < sweeps; k++) {
-            float *eout = (k & 1) ? ws.e32 : ws.e32b;
-            const int nsw = std::min(sp.tile_sweeps, sweeps - done);
-            PCD_TRY(launch_tile(sp.tile, (k & 1) ? maps.eb : maps.ea, eout, maps.r32, ws.ctl, a, nsw, (k & 1) ? 0 : 1, track, k == 0, s));
-            done += nsw;
-            n++;
-        }
+        PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, sp.tile.ncol, sp.tile.rows, 2 * sp.tile.K, &maps));
+        unsigned *done = static_cast<unsigned *>(ws.rx);
+        PCD_TRY(launch_tile(sp.tile, maps, ws.ctl, done, done + (size_t)sp.tile.ncol * sp.tile.nrow, a, sp.tile_sweeps,
+                            sweeps, ws.wait_limit > 0 ? ws.wait_limit : kWordPolls, ws.withhold_flag, s, &n));
         PCD_TRY(launch_refresh(nullptr, refresh_job(ws, b, phi, a), 1, refresh_job(ws, b, phi, a).nblk,
                                a.stop == PCD_STOP_REL_RESIDUAL ? a.tol : -1.0, s));
         *nodes = n + 1;
@@ -774,7 +787,8 @@ int get_chunk_graph(SolverWorkspace &ws, const double *b, double *phi, const Sol
 {
     std::vector<long long> key = {(long long)(uintptr_t)b, (long long)(uintptr_t)phi, a.W, a.H, a.ld, a.stop,
                                   a.max_iter, precision, masked, sweeps, sched, sp.G, sp.T, sp.R, sp.tma, sp.two,
-                                  sp.tile.K, sp.tile.grid, sp.tile_sweeps};
+                                  sp.tile.K, sp.tile.grid, sp.tile.rows, sp.tile_sweeps,
+                                  (long long)(uintptr_t)ws.rx, ws.wait_limit, ws.withhold_flag};
     long long tb, ob;
     std::memcpy(&tb, &a.tol, 8);
     std::memcpy(&ob, &a.omega, 8);
@@ -842,24 +856,6 @@ int cached_plan(SolverWorkspace &ws, std::vector<int> key, Plan *out, Make make)
 
 enum { kPlanResident, kPlanCluster, kPlanTile, kPlanPersist, kPlanBlocks, kPlanBlocks64 };
 
-// Polls of a tagged word before a wait gives up: each is an L2 trip, together
-// about two seconds.
-constexpr long long kWordPolls = 1ll << 21;
-
-// The tagged words' buffer, zeroed: tags start at 1 in every solve, and no word
-// of an earlier one may match.
-int reserve_words(SolverWorkspace &ws, size_t need, cudaStream_t s)
-{
-    if (need > ws.rx_bytes) {
-        if (ws.rx) cudaFree(ws.rx);
-        ws.rx = nullptr;
-        ws.rx_bytes = 0;
-        PCD_CUDA(cudaMalloc(&ws.rx, need));
-        ws.rx_bytes = need;
-    }
-    PCD_CUDA(cudaMemsetAsync(ws.rx, 0, need, s));
-    return PCD_OK;
-}
 
 // One cooperative launch per solve (sor_persist.cu), bracketed by the FP64
 // residual kernels that supply ||b|| / r64 before and the exact statistics after.
@@ -1544,7 +1540,9 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         if (tile_plan(ws.dev, W, H, ld, sp.tile_sweeps <= 2 ? 2 : 4, &sp.tile) == PCD_OK) sched = PCD_SCHED_TILES;
     }
     if (sched == PCD_SCHED_TILES) {
-        // chosen above
+        // a word a tile, and one a pass (at least one sweep)
+        if (!done_already)
+            PCD_TRY(reserve_words(ws, sizeof(unsigned) * ((size_t)sp.tile.ncol * sp.tile.nrow + mixed_chunk(a, o)), s));
     } else if (!masked && precision == PCD_PREC_MIXED &&
                (o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_STREAM ||
                 o.schedule == PCD_SCHED_PERSISTENT || o.schedule == PCD_SCHED_CLUSTER ||
@@ -1611,7 +1609,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     PCD_CUDA(cudaStreamSynchronize(s));
     const Ctl &c = ws.ctl_host[0];
     if (c.error) {
-        set_error("stream or tile SOR: a bounded wait for a copy gave up (status " + std::to_string(c.error) + ")");
+        set_error("stream or tile SOR: a bounded device wait gave up (status " + std::to_string(c.error) + ")");
         return c.error;
     }
     if (stats) {
@@ -1644,7 +1642,7 @@ constexpr int kBatchRefineBlocks = 1024;
 
 }  // namespace
 
-int TileBatchWorkspace::reserve(size_t cells, int count)
+int TileBatchWorkspace::reserve(size_t cells, int count, int tiles)
 {
     // per cell: the two corrections, the right-hand side, the second potential
     if (cells > arena_cells) {
@@ -1681,7 +1679,15 @@ int TileBatchWorkspace::reserve(size_t cells, int count)
         PCD_CUDA(cudaEventCreate(&t1));
         PCD_CUDA(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
         PCD_CUDA(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
-        PCD_CUDA(cudaMalloc(&counter, sizeof(unsigned)));
+    }
+    if (tiles > sync_tiles) {
+        for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+        graphs.clear();
+        if (sync) cudaFree(sync);
+        sync = nullptr;
+        sync_tiles = 0;
+        PCD_CUDA(cudaMalloc(&sync, sizeof(unsigned) * (2 + (size_t)tiles)));
+        sync_tiles = tiles;
     }
     return PCD_OK;
 }
@@ -1697,7 +1703,7 @@ void TileBatchWorkspace::release()
     if (partials) cudaFree(partials);
     if (jobs) cudaFree(jobs);
     if (rjobs) cudaFree(rjobs);
-    if (counter) cudaFree(counter);
+    if (sync) cudaFree(sync);
     for (cudaEvent_t *e : {&t0, &t1, &ev[0], &ev[1]})
         if (*e) cudaEventDestroy(*e);
     *this = TileBatchWorkspace();
@@ -1733,7 +1739,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     PCD_TRY(tile_batch_config(dev, count, narrow, &smem, &grid));
     size_t per = 0;
     for (int i = 0; i < count; i++) per += (size_t)inst[i].height * inst[i].ld;
-    PCD_TRY(ws.reserve(per, count));
+    PCD_TRY(ws.reserve(per, count, 0));
 
     // largest grids first: their refresh blocks are dispatched first
     std::vector<int> order(count);
@@ -1782,25 +1788,26 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         blocks += r.nblk;
         off += (size_t)q.height * q.ld;
     }
+    PCD_TRY(ws.reserve(per, count, tiles));
     const TileJob *d_jobs = static_cast<const TileJob *>(ws.jobs);
     const RefreshJob *d_rjobs = static_cast<const RefreshJob *>(ws.rjobs);
     // sweeps between FP64 refreshes (passes of 4, the last one shorter):
     // refine_every, else 128 when the largest side is 1024 or more, down to
     // 32 when it is 256 or less
     const int chunk = o.refine_every > 0 ? o.refine_every : 4 * std::max(8, std::min(32, maxdim / 32));
-    const int passes = (chunk + 3) / 4;
 
     PCD_CUDA(cudaEventRecord(ws.t0, s));
     PCD_CUDA(cudaMemcpyAsync(ws.jobs, tj.data(), sizeof(TileJob) * count, cudaMemcpyHostToDevice, s));
     PCD_CUDA(cudaMemcpyAsync(ws.rjobs, rj.data(), sizeof(RefreshJob) * count, cudaMemcpyHostToDevice, s));
     PCD_CUDA(cudaMemsetAsync(ws.ctl, 0, sizeof(Ctl) * count, s));
-    PCD_CUDA(cudaMemsetAsync(ws.counter, 0, sizeof(unsigned), s));
+    PCD_CUDA(cudaMemsetAsync(ws.sync, 0, sizeof(unsigned) * (2 + (size_t)tiles), s));
     // first right-hand side, ||b|| and the stop test of the starting phi
     PCD_TRY(launch_first_refresh(d_rjobs, count, blocks, o.tol, !o.warm_start, s));
 
-    // one CUDA graph per batch signature: the chunk's passes and the refresh
+    // one CUDA graph per batch signature: the chunk's sweeps and the refresh
     std::vector<long long> key = {count, tiles, blocks, chunk, narrow, grid, (long long)smem,
-                                  (long long)(uintptr_t)ws.jobs, (long long)(uintptr_t)ws.rjobs};
+                                  (long long)(uintptr_t)ws.jobs, (long long)(uintptr_t)ws.rjobs,
+                                  (long long)(uintptr_t)ws.sync};
     {
         long long tb;
         std::memcpy(&tb, &o.tol, 8);
@@ -1813,10 +1820,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     } else {
         cudaGraph_t g;
         PCD_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        int st = PCD_OK;
-        for (int k = 0; k < passes && st == PCD_OK; k++)
-            st = launch_tile_batch(d_jobs, count, tiles, std::min(4, chunk - 4 * k), k & 1, k == 0, narrow, grid, smem,
-                                   ws.counter, s);
+        int st = launch_tile_batch(d_jobs, count, tiles, chunk, narrow, grid, smem, ws.sync, ws.sync + 2, kWordPolls, s);
         if (st == PCD_OK) st = launch_refresh(d_rjobs, RefreshJob{}, count, blocks, o.tol, s);
         cudaError_t ce = cudaStreamEndCapture(s, &g);
         if (st != PCD_OK) {
@@ -1855,7 +1859,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
             return PCD_TIMEOUT;
         }
         PCD_CUDA(cudaGraphLaunch(exec, s));
-        count_launches(passes + 1);
+        count_launches(2);
         const int slot = (int)(launched & 1);
         PCD_CUDA(cudaMemcpyAsync(ws.ctl_host + (size_t)slot * count, ws.ctl, sizeof(Ctl) * count,
                                  cudaMemcpyDeviceToHost, s));
@@ -1873,7 +1877,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     PCD_CUDA(cudaStreamSynchronize(s));
     for (int k = 0; k < count; k++)
         if (ws.ctl_host[k].error) {
-            set_error("batched tile solve: a bounded wait for a copy gave up");
+            set_error("batched tile solve: a bounded device wait gave up");
             return ws.ctl_host[k].error;
         }
     float ms = 0.f;

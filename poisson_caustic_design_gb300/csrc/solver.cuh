@@ -29,7 +29,8 @@ struct Ctl {
     int error;                   // PCD_TIMEOUT when a bounded device wait gave up
     int stream_out;              // ping-pong buffer holding the latest FP32 correction
     int phi_side;                // refreshes: 1 while the potential sits in the second buffer
-    unsigned int res_epoch;      // resident sweeps: halo exchanges of this solve so far
+    unsigned int res_epoch;      // resident sweeps: halo exchanges of this solve so far; tile passes: passes
+    int redo;                    // tile passes: sweeps up to the pass that met the max-update stop
     unsigned int res_checks;     // resident sweeps: residual estimates of this solve so far
     unsigned long long maxbits;  // running max |delta| of the current sweep
     double last_max;             // max |delta| of the last full sweep
@@ -107,7 +108,8 @@ struct SolverWorkspace {
     void *bx = nullptr;
     size_t bx_bytes = 0;
     // the resident sweeps' exchange words, and behind them the residual
-    // partials, tracked maxima and barrier counter (all zeroed per solve)
+    // partials, tracked maxima and barrier counter; or the last pass of each
+    // tile (all zeroed per solve)
     void *rx = nullptr;
     size_t rx_bytes = 0;
     // launch plans by grid size and kind (host arithmetic and device queries
@@ -135,12 +137,14 @@ struct TileBatchWorkspace {
     double *partials = nullptr; // residual partials per grid
     void *jobs = nullptr;       // TileJob[cap] (device)
     void *rjobs = nullptr;      // refine descriptors [cap] (device)
-    unsigned *counter = nullptr; // last-CTA counter of the batched pass
+    // batched tile passes: finished CTAs, epoch, and each tile's last pass
+    unsigned *sync = nullptr;
+    int sync_tiles = 0;
     int cap = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     std::map<std::vector<long long>, cudaGraphExec_t> graphs;
-    int reserve(size_t cells, int count);
+    int reserve(size_t cells, int count, int tiles);
     void release();
 };
 

@@ -18,13 +18,15 @@ struct TilePlan {
     size_t smem = 0;
 };
 
-// A grid's arrays as the passes' bulk copies see them: boxes of one plane (the
-// cells in even or in odd columns) of a tile's rows x lane columns.
+// A grid's arrays as the passes' TMA copies see them, boxes of one plane (the
+// cells in even or in odd columns): the two corrections and minus their right-hand
+// side as read, a tile's rows and lane columns with their halo, and the
+// corrections as written, without it (lane columns: KQ / ncol, and one more).
 struct TileMaps {
-    CUtensorMap ea, eb, r32;
+    CUtensorMap in[2], out[2][2], r32;
 };
-// rows: of a tile, halo included.
-int tile_maps(const float *ea, const float *eb, const float *r32, int W, int H, int rows, TileMaps *m);
+// Tiles of `rows` written rows and `halo` more on each side, ncol tile columns.
+int tile_maps(float *ea, float *eb, const float *r32, int W, int H, int ncol, int rows, int halo, TileMaps *m);
 
 // One grid of a batched tile pass (4 sweeps at most).
 struct TileJob {
@@ -47,21 +49,24 @@ constexpr int kTileBatchJobsMax = 1024;
 // Dynamic shared memory of the batched pass for njobs grids (narrow: some of
 // them 8 cells wide) and its persistent grid.
 int tile_batch_config(int dev, int njobs, bool narrow, size_t *smem, int *grid);
-// One batched pass of nsw <= 4 sweeps over ntiles tiles of njobs grids
-// (d_jobs on the device, tile0 ascending); parity par reads ea (0) or eb, zero:
-// the corrections start from 0.
-// counter: a device word that is zero between passes.
-int launch_tile_batch(const TileJob *d_jobs, int njobs, int ntiles, int nsw, int par, bool zero, bool narrow, int grid,
-                      size_t smem, unsigned *counter, cudaStream_t s);
+// `sweeps` sweeps (fewer at a grid's sweep cap) in passes of four over ntiles
+// tiles of njobs grids (d_jobs on the device, tile0 ascending), the corrections
+// starting from 0 in ea.  Cooperative.  sync (two words), done (one a tile):
+// zero before a solve's first launch; limit: polls before a wait gives up.
+int launch_tile_batch(const TileJob *d_jobs, int njobs, int ntiles, int sweeps, bool narrow, int grid, size_t smem,
+                      unsigned *sync, unsigned *done, long long limit, cudaStream_t s);
 
 // The plan for a W x H grid with leading dimension ld (W a multiple of 8, ld
 // of 4); depth = sweeps per pass (2 or 4; 0: 4).  PCD_BAD_ARG when no form
 // applies.
 int tile_plan(int dev, int W, int H, int ld, int depth, TilePlan *plan);
-// One pass of nsw <= K sweeps from ein into eout (fewer at the sweep cap);
-// track: the pass reports the largest |update| of its last sweep; zero: the
-// correction starts at 0 and ein is not read.
-int launch_tile(const TilePlan &p, const CUtensorMap &ein, float *eout, const CUtensorMap &r32, Ctl *ctl,
-                const SolveArgs &a, int nsw, int out_idx, bool track, bool zero, cudaStream_t s);
+// `sweeps` sweeps (fewer at the sweep cap), nsw <= K in a pass, of a correction that
+// starts from 0; the result ping-pongs between the maps' buffers
+// (Ctl::stream_out).  Cooperative.  The max-update stop is tested for every pass
+// (gmax: a word a pass, zero between launches), in a second launch that stops
+// where it was met.  done: a word a tile, zero before a solve's first launch;
+// limit: polls before a wait gives up; withhold: tile 0 is never reported done.
+int launch_tile(const TilePlan &p, const TileMaps &maps, Ctl *ctl, unsigned *done, unsigned *gmax, const SolveArgs &a,
+                int nsw, int sweeps, long long limit, int withhold, cudaStream_t s, int *launches);
 
 }  // namespace pcd

@@ -71,3 +71,41 @@ def test_batch_tile_edges(ctx, zero_start, narrow):
         ref = torch.zeros_like(s) if zero_start else s.clone()
         ctx.solve_device(b, ref, pcd.SolveOptions(schedule=1, warm_start=1, **o))
         assert _agree(phi, ref)
+
+
+@pytest.mark.parametrize("n,m", [(2048, 1500), (1600, 900), (1024, 704), (120, 89)])
+@pytest.mark.parametrize("sweeps,refine_every", [(43, 41), (96, 32)])
+def test_passes_without_a_barrier(ctx, n, m, sweeps, refine_every):
+    """Launches of many passes, whose tiles wait only for their neighbours'
+    last pass: more tiles than SMs (361, 180) and fewer (81, 4)."""
+    import poisson_caustic_design_gb300 as pcd
+
+    b, start = _problem(n, m)
+    out = {}
+    for sched in (1, 6):
+        phi = start.clone()
+        st = ctx.solve_device(b, phi, pcd.SolveOptions(
+            stop=pcd.STOP_REL_RESIDUAL, tol=0.0, max_iterations=sweeps, precision=pcd.PREC_MIXED, omega=-1.0,
+            warm_start=1, schedule=sched, refine_every=refine_every))
+        assert st["sweeps"] == sweeps and st["schedule_used"] == sched
+        out[sched] = phi
+    assert _agree(out[6], out[1])
+
+
+def test_tile_wait_runs_out():
+    """With the first tile's passes never reported its neighbours' waits run
+    out: the solve returns PCD_TIMEOUT and the context solves normally
+    afterwards."""
+    import poisson_caustic_design_gb300 as pcd
+
+    c = pcd.Context(0)
+    b, start = _problem(512, 512)
+    o = pcd.SolveOptions(stop=pcd.STOP_REL_RESIDUAL, tol=1e-6, precision=pcd.PREC_MIXED, omega=-1.0, schedule=6)
+    L = pcd.solver._lib.load()
+    assert L.pcd_ctx_set_wait_limit(c.handle, 2000, 1) == 0
+    with pytest.raises(pcd.PCDError) as err:
+        c.solve_device(b, start.clone(), o)
+    assert err.value.status == 4
+    assert L.pcd_ctx_set_wait_limit(c.handle, 0, 0) == 0
+    assert c.solve_device(b, start.clone(), o)["converged"]
+    c.close()
