@@ -1,23 +1,27 @@
 // refresh.cu -- the FP64 passes of a solve (sm_103a).
 //
-// This part runs one FP64 operation per SM and half clock (1/56 of the FP32
-// rate), so these passes are bound by the number of FP64 instructions, not by
-// memory: 24 bytes read and 12 written a cell take 80 us at 4096^2, eight FP64
-// operations a cell 240.
+// This part runs an FP64 operation of a warp every 16 clocks of an SM (1/56 of
+// the FP32 rate), so these passes are bound by the number of FP64 instructions,
+// not by memory: 20 bytes read and 12 written a cell take 80 us at 4096^2, six
+// FP64 operations a cell 190.
 //
 // k_refresh folds the FP32 correction into the potential and renews the
 // residual in one pass:  xi = phi + e,  r = b - (sum of neighbours - cnt xi).
 // A warp walks down a strip of 30 columns (lanes 1 to 30; lanes 0 and 31 the
 // columns beside it).  With D(x, y) = xi(x+1, y) + xi(x, y+1) the neighbour sum
 // of (x, y) is D(x-1, y-1) + D(x, y), so a cell costs two additions for it
-// instead of three, one shuffle each way, and xi is formed once:  widen e, add,
-// D, D + D, multiply-add, subtract, multiply-add for the norm, narrow r.  (One
-// thread a cell forming xi of all five cells and counting neighbours in FP64
-// took about 24.)  Cells outside the grid read 0.
+// instead of three, one shuffle each way, and xi is formed once:  add, D, D + D,
+// multiply-add, subtract, multiply-add for the norm (the conversions run beside
+// them).  4096^2: 308 us, 2048^2: 88, the pipe 81% busy; 386 and 122 when the
+// compiler formed the neighbour counts in FP64 for every row, the largest |r| was
+// compared as 64-bit words and pieces of 8, 16 or 32 rows left SMs idle at the
+// end.  (One thread a cell forming xi of all five cells took about 24
+// operations.)  Cells outside the grid read 0.
 //
 // xi goes to the other of two buffers, because a neighbouring strip may still
 // need the old phi; the control block says which one holds the potential.
 #include <algorithm>
+#include <cmath>
 
 #include "refresh.cuh"
 #include "sor_quads.cuh"
@@ -26,7 +30,9 @@ namespace pcd {
 
 namespace {
 
-constexpr int kRefreshWarps = 4;      // warps of a block: one or two blocks fill the FP64 pipes of an SM
+constexpr int kRefreshWarps = 4;      // warps of a block
+constexpr int kRefreshResident = 4;   // blocks of an SM (4096^2: 305 us, with eight 330)
+constexpr int kRefreshSms = 152;
 constexpr int kRefreshCols = 30;      // columns a warp owns
 constexpr int kStartThreads = 256;
 
@@ -43,6 +49,15 @@ __device__ __forceinline__ unsigned long long max_abs_bits(unsigned long long m,
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
     return b > m && b <= 0x7ff0000000000000ull ? b : m;
+}
+
+// The same on words.
+__device__ __forceinline__ void max_abs_words(unsigned &mhi, unsigned &mlo, double r)
+{
+    const unsigned hi = (unsigned)__double2hiint(r) & 0x7fffffffu, lo = (unsigned)__double2loint(r);
+    const bool more = hi > mhi || (hi == mhi && lo > mlo), number = hi < 0x7ff00000u || (hi == 0x7ff00000u && lo == 0u);
+    mhi = more && number ? hi : mhi;
+    mlo = more && number ? lo : mlo;
 }
 
 __device__ __forceinline__ bool rf_last_block(Ctl *ctl, int nblk)
@@ -93,24 +108,40 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
     double *__restrict__ pout = FIRST || side ? J.phi : J.phi2;
     const float *__restrict__ e = rf_load(&ctl->stream_out) ? J.e1 : J.e0;
     const int W = J.W, H = J.H, ld = J.ld, KQ = (W + 7) >> 3;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     const int strips = (W + kRefreshCols - 1) / kRefreshCols, pieces = (H + J.rows - 1) / J.rows;
     double acc = 0.0, acc_b = 0.0;
-    unsigned long long mbits = 0ull;
+    unsigned mhi = 0u, mlo = 0u;  // the largest |r|'s words
     for (int item = ((int)blockIdx.x - J.blk0) * kRefreshWarps + w; item < strips * pieces;
          item += J.nblk * kRefreshWarps) {
         const int piece = item / strips, strip = item - piece * strips;
         const int x = strip * kRefreshCols + lane - 1;
         const bool in = x >= 0 && x < W, own = in && lane >= 1 && lane <= kRefreshCols;
-        const int y0 = piece * J.rows, y1 = min(y0 + J.rows, H);
-        const double c2 = (double)((x > 0) + (x < W - 1) + 2), c1 = c2 - 1.0, c0 = c2 - 2.0;
-        const size_t at = in ? (size_t)x : 0;
-        const int col = quads::quad_column((int)at, KQ);  // in a row of e and r32
+        const int y0 = piece * J.rows, y1 = min(y0 + J.rows, H), yb = max(y0 - 1, 0);
+        // neighbours of a cell with both vertical ones, with one and with none,
+        // as the high words of doubles
+        const int nh = (x > 0) + (x < W - 1);
+        const int c2 = nh == 2 ? 0x40100000 : nh ? 0x40080000 : 0x40000000;
+        const int c1 = nh == 2 ? 0x40080000 : nh ? 0x40000000 : 0x3ff00000;
+        const int c0 = nh == 2 ? 0x40000000 : nh ? 0x3ff00000 : 0;
+        // places as byte offsets in 32 bits from the piece's first row (28% fewer
+        // instructions than 64-bit indices)
+        const unsigned at = in ? (unsigned)x : 0u, row = (unsigned)ld * 8u, row32 = 32u * (unsigned)KQ;
+        const unsigned col = (unsigned)quads::quad_column((int)at, KQ) * 4u;
+        const size_t base = (size_t)yb * ld, base32 = (size_t)yb * 8 * KQ;
+        const char *p_in = reinterpret_cast<const char *>(pin + base), *p_b = reinterpret_cast<const char *>(J.b + base);
+        const char *p_e = reinterpret_cast<const char *>(e + base32);
+        char *p_out = reinterpret_cast<char *>(pout + base), *p_r = reinterpret_cast<char *>(J.r32 + base32);
         auto load = [&](int y, double &p, float &ev) {
             const bool ok = in && y >= 0 && y < H;
-            const size_t i = (size_t)(ok ? y : 0) * ld + at;
-            p = ok && !(FIRST && zero) ? pin[i] : 0.0;
-            ev = ok && !FIRST ? e[(long)y * 8 * KQ + col] : 0.f;
+            const unsigned k = (unsigned)(y - yb);
+            p = 0.0;
+            ev = 0.f;
+            if (ok && !(FIRST && zero)) p = *reinterpret_cast<const double *>(p_in + (k * row + at * 8u));
+            if (ok && !FIRST) ev = *reinterpret_cast<const float *>(p_e + (k * row32 + col));
+        };
+        auto load_b = [&](int y) {
+            return *reinterpret_cast<const double *>(p_b + ((unsigned)(y - yb) * row + at * 8u));
         };
         // rows y0 - 1, y0 and y0 + 1; then one row ahead of the one in hand
         double pa, pb, pc, bc;
@@ -118,7 +149,7 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
         load(y0 - 1, pa, ea);
         load(y0, pb, eb);
         load(y0 + 1, pc, ec);
-        bc = own ? J.b[(size_t)y0 * ld + at] : 0.0;
+        bc = own ? load_b(y0) : 0.0;
         const double xa = pa + (double)ea;
         double xc = pb + (double)eb;
         // D(x, y0 - 1)
@@ -127,20 +158,20 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
             double pn, bn = 0.0;
             float en;
             load(y + 2, pn, en);
-            if (own && y + 1 < y1) bn = J.b[(size_t)(y + 1) * ld + at];
+            if (own && y + 1 < y1) bn = load_b(y + 1);
             const double xn = pc + (double)ec;
             const double d = __shfl_down_sync(0xffffffffu, xc, 1) + xn;
             const double sum = __shfl_up_sync(0xffffffffu, dp, 1) + d;
             const bool top = y > 0, bot = y < H - 1;
-            const double cnt = top && bot ? c2 : top || bot ? c1 : c0;
+            const double cnt = __hiloint2double(top && bot ? c2 : top || bot ? c1 : c0, 0);
             const double r = fma(cnt, xc, bc) - sum;
             if (own) {
-                const size_t i = (size_t)y * ld + at;
-                if (!FIRST || zero) pout[i] = xc;
-                J.r32[(long)y * 8 * KQ + col] = -(float)r;
+                const unsigned k = (unsigned)(y - yb);
+                if (!FIRST || zero) *reinterpret_cast<double *>(p_out + (k * row + at * 8u)) = xc;
+                *reinterpret_cast<float *>(p_r + (k * row32 + col)) = -(float)r;
                 acc = fma(r, r, acc);
                 if (FIRST) acc_b = fma(bc, bc, acc_b);
-                mbits = max_abs_bits(mbits, r);
+                max_abs_words(mhi, mlo, r);
             }
             dp = d;
             xc = xn;
@@ -149,6 +180,7 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
             bc = bn;
         }
     }
+    const unsigned long long mbits = ((unsigned long long)mhi << 32) | mlo;
     double v[3] = {acc, acc_b, __longlong_as_double((long long)mbits)};
     block_reduce<3, 4u>(v);
     if (threadIdx.x == 0) {
@@ -269,14 +301,30 @@ __global__ void __launch_bounds__(kStartThreads)
 
 }  // namespace
 
-int refresh_shape(int W, int H, int cap, long warps, int *rows)
+int refresh_shape(int W, int H, int cap, double share, int *rows)
 {
+    // An SM's time is that of its warps' FP64 instructions, six a row and five
+    // for the rows of overlap, on one pipe; with fewer than twelve warps on it,
+    // their latency.  All blocks are resident at once, so the fullest SM counts.
     const int strips = ceil_div(W, kRefreshCols);
-    // a piece's two rows of overlap cost a quarter of a row's work each
-    int r = 32;
-    while (r > 8 && (long)strips * ceil_div(H, r) < warps) r >>= 1;
-    *rows = r;
-    return std::max(1, std::min(cap, ceil_div((long)strips * ceil_div(H, r), kRefreshWarps)));
+    const double sms = std::max(1.0, kRefreshSms * share);
+    double best = 0.0;
+    int best_rows = 0, best_blocks = 1;
+    for (int r = 4; r <= std::max(4, H); r += r < 32 ? 1 : r / 16) {
+        const int blocks = ceil_div((long)strips * ceil_div(H, r), kRefreshWarps);
+        if (blocks > kRefreshResident * sms || blocks > cap) continue;
+        const double t = std::max(12.0, kRefreshWarps * std::ceil(blocks / sms)) * (6 * r + 5);
+        if (best_rows && t >= best) continue;
+        best = t;
+        best_rows = r;
+        best_blocks = blocks;
+    }
+    if (!best_rows) {  // more strips than warps
+        best_rows = std::max(32, H);
+        best_blocks = std::max(1, std::min<int>(cap, (int)(kRefreshResident * sms)));
+    }
+    *rows = best_rows;
+    return best_blocks;
 }
 
 int launch_refresh(const RefreshJob *jobs, const RefreshJob &one, int njobs, int blocks, double tol, cudaStream_t s)

@@ -19,10 +19,9 @@ struct RefreshJob {
     int rows;                // rows of a strip piece
 };
 
-// Blocks of a W x H grid's refresh (at most cap), in about `warps` pieces or
-// more, and the rows of a piece.
-constexpr int kRefreshFill = 1216;  // warps that fill the chip: two a scheduler
-int refresh_shape(int W, int H, int cap, long warps, int *rows);
+// Blocks of a W x H grid's refresh (at most cap) on `share` of the chip, and the
+// rows of a piece.
+int refresh_shape(int W, int H, int cap, double share, int *rows);
 // For every job whose solve is not done: phi += e in FP64, r = b - L phi, -r in
 // FP32 to r32, the norms, and (tol >= 0) the relative-residual stop test; a solve
 // that has halted is then done.  jobs: on the device, or nullptr for the single

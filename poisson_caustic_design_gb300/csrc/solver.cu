@@ -679,7 +679,7 @@ RefreshJob refresh_job(const SolverWorkspace &ws, const double *b, double *phi, 
     j.W = a.W;
     j.H = a.H;
     j.ld = a.ld;
-    j.nblk = refresh_shape(a.W, a.H, kResidualBlocksMax, kRefreshFill, &j.rows);
+    j.nblk = refresh_shape(a.W, a.H, kResidualBlocksMax, 1.0, &j.rows);
     return j;
 }
 
@@ -1782,9 +1782,8 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         r.H = q.height;
         r.ld = q.ld;
         r.blk0 = blocks;
-        // each grid's share of the warps that fill the chip
         r.nblk = refresh_shape(q.width, q.height, kBatchRefineBlocks,
-                               (long)((double)kRefreshFill * q.width * q.height / (double)all_cells), &r.rows);
+                               (double)q.width * q.height / (double)all_cells, &r.rows);
         blocks += r.nblk;
         off += (size_t)q.height * q.ld;
     }
