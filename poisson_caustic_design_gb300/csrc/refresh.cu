@@ -73,6 +73,17 @@ __device__ __forceinline__ bool rf_last_block(Ctl *ctl, int nblk)
     return is_last;
 }
 
+// The control block into host memory, one thread (the end of the launch, which
+// the host waits for, makes it visible).
+__device__ void rf_report(const Ctl *ctl, Ctl *report)
+{
+    static_assert(sizeof(Ctl) % 8 == 0, "copied in 64-bit words");
+    const volatile unsigned long long *from = reinterpret_cast<const volatile unsigned long long *>(ctl);
+    volatile unsigned long long *to = reinterpret_cast<volatile unsigned long long *>(report);
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(Ctl) / 8); k++) to[k] = from[k];
+}
+
 // Sums the blocks' partials in a fixed order (every thread of the block
 // calls); thread 0 has the result.
 __device__ void rf_sum_partials(const double *partials, int nblk, double (&v)[3])
@@ -102,8 +113,16 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
         J = jobs[lo];
     }
     Ctl *ctl = J.ctl;
-    if (rf_load(&ctl->done) || rf_load(&ctl->error) || rf_load(&ctl->nan_cells)) return;
     const int side = rf_load(&ctl->phi_side);
+    if (rf_load(&ctl->done) || rf_load(&ctl->error) || rf_load(&ctl->nan_cells)) {
+        if (!J.report) return;
+        if ((int)blockIdx.x == J.blk0 && threadIdx.x == 0) rf_report(ctl, J.report);
+        if (side)
+            for (int y = (int)blockIdx.x - J.blk0; y < J.H; y += J.nblk)
+                for (int x = threadIdx.x; x < J.W; x += blockDim.x)
+                    J.phi[(size_t)y * J.ld + x] = J.phi2[(size_t)y * J.ld + x];
+        return;
+    }
     const double *__restrict__ pin = side ? J.phi2 : J.phi;
     double *__restrict__ pout = FIRST || side ? J.phi : J.phi2;
     const float *__restrict__ e = rf_load(&ctl->stream_out) ? J.e1 : J.e0;
@@ -208,12 +227,13 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
         c->stream_out = 0;
         c->blocks_done_r = 0;
         __threadfence();
+        if (J.report) rf_report(ctl, J.report);
     }
 }
 
-__global__ void __launch_bounds__(kStartThreads) k_phi_settle(const RefreshJob *__restrict__ jobs, RefreshJob one)
+__global__ void __launch_bounds__(kStartThreads) k_phi_settle(const RefreshJob *__restrict__ jobs)
 {
-    const RefreshJob &J = jobs ? jobs[blockIdx.z] : one;
+    const RefreshJob &J = jobs[blockIdx.z];
     if (!rf_load(&J.ctl->phi_side)) return;
     for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < J.W; x += gridDim.x * blockDim.x)
         for (int y = blockIdx.y; y < J.H; y += gridDim.y) J.phi[(size_t)y * J.ld + x] = J.phi2[(size_t)y * J.ld + x];
@@ -341,12 +361,9 @@ int launch_first_refresh(const RefreshJob *jobs, int njobs, int blocks, double t
     return PCD_OK;
 }
 
-int launch_phi_settle(const RefreshJob *jobs, const RefreshJob &one, int njobs, cudaStream_t s)
+int launch_phi_settle(const RefreshJob *jobs, int njobs, cudaStream_t s)
 {
-    const dim3 grid = jobs ? dim3(4, 64, njobs)
-                           : dim3(std::min(ceil_div(one.W, kStartThreads), 2432),
-                                  std::max(1, std::min(one.H, 2432 / ceil_div(one.W, kStartThreads))));
-    k_phi_settle<<<grid, kStartThreads, 0, s>>>(jobs, one);
+    k_phi_settle<<<dim3(4, 64, njobs), kStartThreads, 0, s>>>(jobs);
     PCD_LAUNCHED(1);
     return PCD_OK;
 }

@@ -17,6 +17,9 @@ struct RefreshJob {
     int W, H, ld;
     int blk0, nblk;
     int rows;                // rows of a strip piece
+    // a single solve's launches leave their control block here (host memory), and
+    // one behind the solve's last brings the potential back into phi
+    Ctl *report;
 };
 
 // Blocks of a W x H grid's refresh (at most cap) on `share` of the chip, and the
@@ -30,8 +33,8 @@ int launch_refresh(const RefreshJob *jobs, const RefreshJob &one, int njobs, int
 // The same for the starts of a batch: e is 0 (zero: so is phi), the norms
 // include ||b||, and phi stays where it is.
 int launch_first_refresh(const RefreshJob *jobs, int njobs, int blocks, double tol, bool zero, cudaStream_t s);
-// The potential back into job.phi.
-int launch_phi_settle(const RefreshJob *jobs, const RefreshJob &one, int njobs, cudaStream_t s);
+// A batch's potentials back into phi.
+int launch_phi_settle(const RefreshJob *jobs, int njobs, cudaStream_t s);
 
 // The start of a solve: the neighbour-validity mask and the number of NaN
 // cells of b; zero: phi = 0; r = b - L phi in FP64 over the valid cells with

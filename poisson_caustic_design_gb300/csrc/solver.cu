@@ -440,8 +440,6 @@ struct StreamPlan {
     size_t smem = 0;
     int two = 0;          // two sweeps per pass (k_sweep2_tma) available
     size_t smem2 = 0;
-    TilePlan tile;        // register-resident tile passes (schedule TILES)
-    int tile_sweeps = 0;  // sweeps per tile pass (between stop tests)
 };
 
 int stream_plan(int dev, int W, int H, int ld, bool allow_tma, StreamPlan *p)
@@ -711,17 +709,6 @@ int enqueue_chunk(SolverWorkspace &ws, const double *b, double *phi, const Solve
         }
         sweeps = 0;
     }
-    if (!MASKED && sched == PCD_SCHED_TILES) {
-        TileMaps maps;
-        PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, sp.tile.ncol, sp.tile.rows, 2 * sp.tile.K, &maps));
-        unsigned *done = static_cast<unsigned *>(ws.rx);
-        PCD_TRY(launch_tile(sp.tile, maps, ws.ctl, done, done + (size_t)sp.tile.ncol * sp.tile.nrow, a, sp.tile_sweeps,
-                            sweeps, ws.wait_limit > 0 ? ws.wait_limit : kWordPolls, ws.withhold_flag, s, &n));
-        PCD_TRY(launch_refresh(nullptr, refresh_job(ws, b, phi, a), 1, refresh_job(ws, b, phi, a).nblk,
-                               a.stop == PCD_STOP_REL_RESIDUAL ? a.tol : -1.0, s));
-        *nodes = n + 1;
-        return PCD_OK;
-    }
     if (!MASKED && sched == PCD_SCHED_STREAM) {
         // launch k reads buffer k&1 and writes the other (two sweeps per
         // launch where the plan allows, a single sweep for an odd rest); the
@@ -786,9 +773,7 @@ int get_chunk_graph(SolverWorkspace &ws, const double *b, double *phi, const Sol
                     const StreamPlan &sp)
 {
     std::vector<long long> key = {(long long)(uintptr_t)b, (long long)(uintptr_t)phi, a.W, a.H, a.ld, a.stop,
-                                  a.max_iter, precision, masked, sweeps, sched, sp.G, sp.T, sp.R, sp.tma, sp.two,
-                                  sp.tile.K, sp.tile.grid, sp.tile.rows, sp.tile_sweeps,
-                                  (long long)(uintptr_t)ws.rx, ws.wait_limit, ws.withhold_flag};
+                                  a.max_iter, precision, masked, sweeps, sched, sp.G, sp.T, sp.R, sp.tma, sp.two};
     long long tb, ob;
     std::memcpy(&tb, &a.tol, 8);
     std::memcpy(&ob, &a.omega, 8);
@@ -1215,6 +1200,58 @@ int resident_rule(SolverWorkspace &ws, const SolveArgs &a, const pcd_solve_opts 
     return PCD_OK;
 }
 
+// A mixed-precision solve's chunks: launch(): one chunk of FP32 sweeps; after each
+// the FP64 refresh.  Chunk i + 1 is launched before chunk i's control block is
+// inspected, and does nothing but bring the potential home where the solve is
+// done.  The refresh leaves the control block in host memory itself: a copy
+// between it and the next chunk's launch took 9 us.
+template <typename Launch>
+int run_chunks(SolverWorkspace &ws, RefreshJob job, const SolveArgs &a, long max_launches, int sched,
+               const char *what, pcd_solve_stats *stats, int *nans, cudaStream_t s, Launch launch)
+{
+    PCD_CUDA(cudaEventRecord(ws.k0, s));
+    const Ctl *last = nullptr;
+    for (long launched = 0; !last; launched++) {
+        if (launched >= max_launches) {
+            set_error(std::string(what) + ": launch budget exceeded without a done flag");
+            return PCD_TIMEOUT;
+        }
+        PCD_TRY(launch());
+        const int slot = (int)(launched & 1);
+        job.report = &ws.ctl_host[slot];
+        PCD_TRY(launch_refresh(nullptr, job, 1, job.nblk, a.stop == PCD_STOP_REL_RESIDUAL ? a.tol : -1.0, s));
+        PCD_CUDA(cudaEventRecord(ws.ev[slot], s));
+        if (launched < 1) continue;
+        PCD_CUDA(cudaEventSynchronize(ws.ev[slot ^ 1]));
+        const Ctl &c = ws.ctl_host[slot ^ 1];
+        if (c.done || c.error || c.nan_cells) last = &c;
+    }
+    PCD_CUDA(cudaEventRecord(ws.k1, s));
+    PCD_CUDA(cudaEventRecord(ws.t1, s));
+    PCD_CUDA(cudaStreamSynchronize(s));
+    const Ctl &c = *last;
+    *nans = c.nan_cells;
+    if (c.error) {
+        set_error(std::string(what) + ": a bounded device wait gave up (status " + std::to_string(c.error) + ")");
+        return c.error;
+    }
+    if (stats) {
+        stats->sweeps = c.sweeps;
+        stats->converged = c.converged;
+        stats->rel_residual = c.rel;
+        stats->max_residual = c.rmax;
+        stats->last_max_update = c.last_max;
+        stats->residual_checks = c.checks;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ws.t0, ws.t1);
+        stats->device_ms = ms;
+        cudaEventElapsedTime(&ms, ws.k0, ws.k1);
+        stats->sweep_ms = ms;
+        stats->schedule_used = sched;
+    }
+    return c.converged ? PCD_OK : PCD_NOT_CONVERGED;
+}
+
 // Mixed precision on resident tiles: launches of [FP32 sweeps, FP64 residual
 // refresh, phi += e] until the stop test passes.  The next launch is enqueued
 // before the previous one's control block is read; a launch after the stop
@@ -1228,7 +1265,6 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     const size_t part_at = plan.xb_bytes, gmax_at = part_at + 2 * (size_t)G * sizeof(unsigned long long);
     const size_t bar_at = gmax_at + kResidentChecksMax * sizeof(unsigned), need = bar_at + 64;
     PCD_TRY(reserve_words(ws, need, s));
-    const RefreshJob job = refresh_job(ws, b, phi, a);
 
     ResidentArgs ra{};
     ra.W = a.W; ra.H = a.H;
@@ -1251,54 +1287,28 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     ra.spin_limit = ws.wait_limit > 0 ? ws.wait_limit : kWordPolls;
     ra.withhold = ws.withhold_flag;
 
-    PCD_CUDA(cudaEventRecord(ws.k0, s));
     const long max_launches = rule.cycle ? (long)a.max_iter + 4 : (long)a.max_iter / std::max(1, rule.chunk) + 3;
-    long launched = 0;
-    bool finished = false;
-    while (!finished) {
-        if (launched >= max_launches) {
-            set_error("resident SOR: launch budget exceeded without a done flag");
-            return PCD_TIMEOUT;
-        }
-        PCD_TRY(launch_resident(ra, plan, s));
-        PCD_TRY(launch_refresh(nullptr, job, 1, job.nblk, a.stop == PCD_STOP_REL_RESIDUAL ? a.tol : -1.0, s));
-        const int slot = (int)(launched & 1);
-        PCD_CUDA(cudaMemcpyAsync(&ws.ctl_host[slot], ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-        PCD_CUDA(cudaEventRecord(ws.ev[slot], s));
-        launched++;
-        if (launched >= 2) {
-            const int prev = (int)((launched - 2) & 1);
-            PCD_CUDA(cudaEventSynchronize(ws.ev[prev]));
-            const Ctl &c = ws.ctl_host[prev];
-            if (c.done || c.error || c.nan_cells) finished = true;
-        }
-    }
-    PCD_TRY(launch_phi_settle(nullptr, job, 1, s));
-    PCD_CUDA(cudaEventRecord(ws.k1, s));
-    PCD_CUDA(cudaEventRecord(ws.t1, s));
-    PCD_CUDA(cudaMemcpyAsync(&ws.ctl_host[0], ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-    PCD_CUDA(cudaStreamSynchronize(s));
-    const Ctl &c = ws.ctl_host[0];
-    *nans = c.nan_cells;
-    if (c.error) {
-        set_error("resident SOR: a bounded device wait gave up (status " + std::to_string(c.error) + ")");
-        return c.error;
-    }
-    if (stats) {
-        stats->sweeps = c.sweeps;
-        stats->converged = c.converged;
-        stats->rel_residual = c.rel;
-        stats->max_residual = c.rmax;
-        stats->last_max_update = c.last_max;
-        stats->residual_checks = c.checks;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, ws.t0, ws.t1);
-        stats->device_ms = ms;
-        cudaEventElapsedTime(&ms, ws.k0, ws.k1);
-        stats->sweep_ms = ms;
-        stats->schedule_used = rule.sched;
-    }
-    return c.converged ? PCD_OK : PCD_NOT_CONVERGED;
+    return run_chunks(ws, refresh_job(ws, b, phi, a), a, max_launches, rule.sched, "resident SOR", stats, nans, s,
+                      [&] { return launch_resident(ra, plan, s); });
+}
+
+// Tile passes over a grid in HBM (sor_tile.cu); nsw sweeps a pass, the last
+// one's update tested by the max-update stop.
+int solve_tiles(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const TilePlan &plan, int nsw,
+                int chunk, pcd_solve_stats *stats, cudaStream_t s)
+{
+    // a word a tile, and one a pass
+    const size_t tiles = (size_t)plan.ncol * plan.nrow;
+    PCD_TRY(reserve_words(ws, sizeof(unsigned) * (tiles + chunk), s));
+    unsigned *done = static_cast<unsigned *>(ws.rx);
+    TileMaps maps;
+    PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, plan.ncol, plan.rows, 2 * plan.K, &maps));
+    int nans = 0;
+    return run_chunks(ws, refresh_job(ws, b, phi, a), a, (long)a.max_iter / chunk + 3, PCD_SCHED_TILES, "tile SOR",
+                      stats, &nans, s, [&] {
+                          return launch_tile(plan, maps, ws.ctl, done, done + tiles, a, nsw, chunk,
+                                             ws.wait_limit > 0 ? ws.wait_limit : kWordPolls, ws.withhold_flag, s);
+                      });
 }
 
 }  // namespace
@@ -1533,16 +1543,20 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     StreamPlan sp;
     if (!masked && precision == PCD_PREC_MIXED && o.schedule != PCD_SCHED_STREAM &&
         o.schedule != PCD_SCHED_LAUNCHES && o.schedule != PCD_SCHED_STRIPES) {
-        // register-resident tile passes (4096^2 FP32 sweep: 26 us against the
-        // stream pass's 40 us); check_every: sweeps per pass (stop tests
-        // after every pass), 4 at most
-        sp.tile_sweeps = o.check_every > 0 ? std::min(o.check_every, 4) : 4;
-        if (tile_plan(ws.dev, W, H, ld, sp.tile_sweeps <= 2 ? 2 : 4, &sp.tile) == PCD_OK) sched = PCD_SCHED_TILES;
+        // register-resident tile passes; check_every: sweeps per pass (stop
+        // tests after every pass), 4 at most
+        const int nsw = o.check_every > 0 ? std::min(o.check_every, 4) : 4;
+        TilePlan tp;
+        if (tile_plan(ws.dev, W, H, ld, nsw <= 2 ? 2 : 4, &tp) == PCD_OK) {
+            sched = PCD_SCHED_TILES;
+            if (!done_already) {
+                if (!r32_quads) PCD_TRY(start(true));
+                return solve_tiles(ws, b, phi, a, tp, nsw, mixed_chunk(a, o), stats, s);
+            }
+        }
     }
     if (sched == PCD_SCHED_TILES) {
-        // a word a tile, and one a pass (at least one sweep)
-        if (!done_already)
-            PCD_TRY(reserve_words(ws, sizeof(unsigned) * ((size_t)sp.tile.ncol * sp.tile.nrow + mixed_chunk(a, o)), s));
+        // nothing left to sweep
     } else if (!masked && precision == PCD_PREC_MIXED &&
                (o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_STREAM ||
                 o.schedule == PCD_SCHED_PERSISTENT || o.schedule == PCD_SCHED_CLUSTER ||
@@ -1552,10 +1566,9 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     } else if (!masked && H >= 3 && W <= 2 * kRowCellsMax * kStripeThreads && o.schedule != PCD_SCHED_LAUNCHES) {
         sched = PCD_SCHED_STRIPES;
     }
-    // (r32, the first right-hand side of the FP32 sweeps, is the start's; the
-    // tile passes start from 0 without reading it)
-    if (!done_already && mixed && r32_quads != (sched == PCD_SCHED_TILES)) PCD_TRY(start(!r32_quads));
-    if (!done_already && precision == PCD_PREC_MIXED && sched != PCD_SCHED_TILES)
+    // (r32, the first right-hand side of the FP32 sweeps, is the start's)
+    if (!done_already && mixed && r32_quads) PCD_TRY(start(false));
+    if (!done_already && precision == PCD_PREC_MIXED)
         PCD_CUDA(cudaMemsetAsync(ws.e32, 0, sizeof(float) * (size_t)H * ld, s));
     const bool stripes = sched == PCD_SCHED_STRIPES;
     if (stripes && ws.stripe_resident == 0) {
@@ -1594,7 +1607,6 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
             if (flag_done(ws.ctl_host[prev]) || ws.ctl_host[prev].error) finished = 1;
         }
     }
-    if (sched == PCD_SCHED_TILES && !done_already) PCD_TRY(launch_phi_settle(nullptr, refresh_job(ws, b, phi, a), 1, s));
     PCD_CUDA(cudaEventRecord(ws.k1, s));
     // Final statistics (FP64 residual of the returned phi).
     if (precision != PCD_PREC_MIXED) {
@@ -1609,7 +1621,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     PCD_CUDA(cudaStreamSynchronize(s));
     const Ctl &c = ws.ctl_host[0];
     if (c.error) {
-        set_error("stream or tile SOR: a bounded device wait gave up (status " + std::to_string(c.error) + ")");
+        set_error("stream SOR: a bounded device wait gave up (status " + std::to_string(c.error) + ")");
         return c.error;
     }
     if (stats) {
@@ -1870,7 +1882,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
             if (all_done(ws.ctl_host + (size_t)prev * count)) finished = true;
         }
     }
-    PCD_TRY(launch_phi_settle(d_rjobs, RefreshJob{}, count, s));
+    PCD_TRY(launch_phi_settle(d_rjobs, count, s));
     PCD_CUDA(cudaEventRecord(ws.t1, s));
     PCD_CUDA(cudaMemcpyAsync(ws.ctl_host, ws.ctl, sizeof(Ctl) * count, cudaMemcpyDeviceToHost, s));
     PCD_CUDA(cudaStreamSynchronize(s));

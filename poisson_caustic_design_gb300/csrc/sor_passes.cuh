@@ -67,6 +67,6 @@ int tile_plan(int dev, int W, int H, int ld, int depth, TilePlan *plan);
 // where it was met.  done: a word a tile, zero before a solve's first launch;
 // limit: polls before a wait gives up; withhold: tile 0 is never reported done.
 int launch_tile(const TilePlan &p, const TileMaps &maps, Ctl *ctl, unsigned *done, unsigned *gmax, const SolveArgs &a,
-                int nsw, int sweeps, long long limit, int withhold, cudaStream_t s, int *launches);
+                int nsw, int sweeps, long long limit, int withhold, cudaStream_t s);
 
 }  // namespace pcd

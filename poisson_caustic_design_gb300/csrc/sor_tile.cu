@@ -679,7 +679,7 @@ int tile_maps(float *ea, float *eb, const float *r32, int W, int H, int ncol, in
 }
 
 int launch_tile(const TilePlan &p, const TileMaps &maps, Ctl *ctl, unsigned *done, unsigned *gmax, const SolveArgs &a,
-                int nsw, int sweeps, long long limit, int withhold, cudaStream_t s, int *launches)
+                int nsw, int sweeps, long long limit, int withhold, cudaStream_t s)
 {
     if (nsw < 1 || nsw > p.K || sweeps < 1) {
         set_error("tile SOR: more sweeps than the plan's halo holds");
@@ -690,12 +690,12 @@ int launch_tile(const TilePlan &p, const TileMaps &maps, Ctl *ctl, unsigned *don
     void *params[] = {const_cast<TileMaps *>(&maps), &ctl, &done, const_cast<SolveArgs *>(&a), &ncol, &nrow, &rows, &hk,
                       &nsw, &sweeps, &again, &gmax, &limit, &withhold};
     PCD_CUDA(cudaLaunchCooperativeKernel(tile_kernel(track, a.W == 8), dim3(p.grid), dim3(kTBlock), params, p.smem, s));
-    *launches = 1;
+    count_launches(1);
     if (track && sweeps > nsw) {
         again = 1;
         PCD_CUDA(cudaLaunchCooperativeKernel(tile_kernel(false, a.W == 8), dim3(p.grid), dim3(kTBlock), params, p.smem,
                                              s));
-        *launches = 2;
+        count_launches(1);
     }
     return PCD_OK;
 }
