@@ -1139,6 +1139,10 @@ struct ResidentRule {
     int sched = PCD_SCHED_TILES; // what the solve reports
 };
 
+// Grids that the tile passes take under any schedule.  Others (AUTO alone) keep
+// the stop tests of the schedules that they had before.
+bool tile_grid(int W, int ld) { return W >= 8 && W % 8 == 0 && ld % 4 == 0; }
+
 // FP32 sweeps between FP64 refreshes of the chunked mixed schedules.
 int mixed_chunk(const SolveArgs &a, const pcd_solve_opts &o)
 {
@@ -1179,8 +1183,9 @@ int resident_rule(SolverWorkspace &ws, const SolveArgs &a, const pcd_solve_opts 
     }
     const int depth = o.check_every > 0 && o.check_every <= 2 ? 2 : 4;
     TilePlan tp{};
-    st = cached_plan(ws, {kPlanTile, W, H, a.ld % 4, depth}, &tp,
-                     [&](TilePlan *p) { return tile_plan(ws.dev, W, H, a.ld, depth, p); });
+    st = tile_grid(W, a.ld) ? cached_plan(ws, {kPlanTile, W, H, depth}, &tp,
+                                          [&](TilePlan *p) { return tile_plan(ws.dev, W, H, depth, p); })
+                            : PCD_BAD_ARG;
     if (st != PCD_OK && st != PCD_BAD_ARG) return st;
     if (st == PCD_OK && (long)W * H >= kTileMinCells) {
         r.chunk = mixed_chunk(a, o);
@@ -1292,10 +1297,11 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
                       [&] { return launch_resident(ra, plan, s); });
 }
 
-// Tile passes over a grid in HBM (sor_tile.cu); nsw sweeps a pass, the last
-// one's update tested by the max-update stop.
+// Tile passes over a grid in HBM (sor_tile.cu), nsw sweeps a pass; the update of a
+// pass's last sweep is tested by the max-update stop, for each pass or for a chunk's
+// last.
 int solve_tiles(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const TilePlan &plan, int nsw,
-                int chunk, pcd_solve_stats *stats, cudaStream_t s)
+                int chunk, bool each, int sched, pcd_solve_stats *stats, cudaStream_t s)
 {
     // a word a tile, and one a pass
     const size_t tiles = (size_t)plan.ncol * plan.nrow;
@@ -1304,9 +1310,9 @@ int solve_tiles(SolverWorkspace &ws, const double *b, double *phi, const SolveAr
     TileMaps maps;
     PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, plan.ncol, plan.rows, 2 * plan.K, &maps));
     int nans = 0;
-    return run_chunks(ws, refresh_job(ws, b, phi, a), a, (long)a.max_iter / chunk + 3, PCD_SCHED_TILES, "tile SOR",
+    return run_chunks(ws, refresh_job(ws, b, phi, a), a, (long)a.max_iter / chunk + 3, sched, "tile SOR",
                       stats, &nans, s, [&] {
-                          return launch_tile(plan, maps, ws.ctl, done, done + tiles, a, nsw, chunk,
+                          return launch_tile(plan, maps, ws.ctl, done, done + tiles, a, nsw, chunk, each,
                                              ws.wait_limit > 0 ? ws.wait_limit : kWordPolls, ws.withhold_flag, s);
                       });
 }
@@ -1476,8 +1482,8 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
                             ws.ctl, ws.partials, kResidualBlocksMax, a, !o.warm_start, in_quads,
                             a.stop == PCD_STOP_REL_RESIDUAL, s);
     };
-    PCD_TRY(start(mixed && (resident == PCD_OK ||
-                            ((o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_TILES) && W % 8 == 0))));
+    PCD_TRY(start(mixed && (resident == PCD_OK || o.schedule == PCD_SCHED_AUTO ||
+                            (o.schedule == PCD_SCHED_TILES && W % 8 == 0))));
     if (resident == PCD_OK) {
         int nans = 0;
         const int st = solve_resident(ws, b, phi, a, o, rp, rule, stats, &nans, s);
@@ -1522,7 +1528,35 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     // schedule (measured 2-3.5x faster from 64^2 to 1024^2)
     TilePlan tp_probe;
     const bool prefer_tiles = precision == PCD_PREC_MIXED && o.schedule != PCD_SCHED_PERSISTENT &&
-                              (long)W * H >= kTileMinCells && tile_plan(ws.dev, W, H, ld, 4, &tp_probe) == PCD_OK;
+                              (long)W * H >= kTileMinCells && tile_grid(W, ld) &&
+                              tile_plan(ws.dev, W, H, 4, &tp_probe) == PCD_OK;
+    // AUTO beyond the chip's registers: widths and rows that the tile passes do not
+    // take under their own name run on them, too, with the stop tests, and under
+    // the name, of the schedule whose place they take: the persistent bands (chunks
+    // of 32 or 16 sweeps, tested at their ends), else the stream passes (two
+    // sweeps or one), else the stripes (every sweep).  1500^2: 3.2 us a sweep with
+    // its refreshes, the stream passes 22.9; 9.1 and 24.5 to the max-update stop.
+    TilePlan tp;
+    if (!done_already && !masked && mixed && !prefer_tiles && o.schedule == PCD_SCHED_AUTO && W >= 16 && H >= 16 &&
+        (long)W * H >= kTileMinCells) {
+        int G = 0, chunk = mixed_chunk(a, o), nsw = 1, name = PCD_SCHED_STRIPES;
+        size_t smem = 0;
+        StreamPlan probe;
+        const bool bands = persist_grid(ws.dev, W, H, true, &G, &smem) == PCD_OK;
+        if (bands) {
+            name = PCD_SCHED_PERSISTENT;
+            chunk = o.check_every > 0 ? o.check_every : (a.stop == PCD_STOP_MAX_UPDATE ? 16 : 32);
+            if (o.refine_every > 0 && o.refine_every < chunk) chunk = o.refine_every;
+        } else if (stream_plan(ws.dev, W, H, ld, true, &probe) == PCD_OK) {
+            name = PCD_SCHED_STREAM;
+            if (probe.two) nsw = 2;
+        }
+        if (bands || a.stop != PCD_STOP_MAX_UPDATE) nsw = 4;
+        if (tile_plan(ws.dev, W, H, nsw <= 2 ? 2 : 4, &tp) == PCD_OK) {
+            if (!r32_quads) PCD_TRY(start(true));
+            return solve_tiles(ws, b, phi, a, tp, nsw, chunk, !bands, name, stats, s);
+        }
+    }
     if (!done_already && !masked && !prefer_tiles &&
         (o.schedule == PCD_SCHED_AUTO || o.schedule == PCD_SCHED_PERSISTENT || o.schedule == PCD_SCHED_CLUSTER)) {
         int G = 0;
@@ -1546,12 +1580,11 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         // register-resident tile passes; check_every: sweeps per pass (stop
         // tests after every pass), 4 at most
         const int nsw = o.check_every > 0 ? std::min(o.check_every, 4) : 4;
-        TilePlan tp;
-        if (tile_plan(ws.dev, W, H, ld, nsw <= 2 ? 2 : 4, &tp) == PCD_OK) {
+        if (tile_grid(W, ld) && tile_plan(ws.dev, W, H, nsw <= 2 ? 2 : 4, &tp) == PCD_OK) {
             sched = PCD_SCHED_TILES;
             if (!done_already) {
                 if (!r32_quads) PCD_TRY(start(true));
-                return solve_tiles(ws, b, phi, a, tp, nsw, mixed_chunk(a, o), stats, s);
+                return solve_tiles(ws, b, phi, a, tp, nsw, mixed_chunk(a, o), true, PCD_SCHED_TILES, stats, s);
             }
         }
     }

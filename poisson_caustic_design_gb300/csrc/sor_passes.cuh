@@ -56,17 +56,16 @@ int tile_batch_config(int dev, int njobs, bool narrow, size_t *smem, int *grid);
 int launch_tile_batch(const TileJob *d_jobs, int njobs, int ntiles, int sweeps, bool narrow, int grid, size_t smem,
                       unsigned *sync, unsigned *done, long long limit, cudaStream_t s);
 
-// The plan for a W x H grid with leading dimension ld (W a multiple of 8, ld
-// of 4); depth = sweeps per pass (2 or 4; 0: 4).  PCD_BAD_ARG when no form
-// applies.
-int tile_plan(int dev, int W, int H, int ld, int depth, TilePlan *plan);
+// The plan for a W x H grid (W >= 8); depth = sweeps per pass (2 or 4; 0: 4).
+// PCD_BAD_ARG when no form applies.
+int tile_plan(int dev, int W, int H, int depth, TilePlan *plan);
 // `sweeps` sweeps (fewer at the sweep cap), nsw <= K in a pass, of a correction that
 // starts from 0; the result ping-pongs between the maps' buffers
 // (Ctl::stream_out).  Cooperative.  The max-update stop is tested for every pass
-// (gmax: a word a pass, zero between launches), in a second launch that stops
-// where it was met.  done: a word a tile, zero before a solve's first launch;
+// (each; a second launch stops where it was met) or for the last one (gmax: a word
+// a pass, zero between launches).  done: a word a tile, zero before a solve's first launch;
 // limit: polls before a wait gives up; withhold: tile 0 is never reported done.
 int launch_tile(const TilePlan &p, const TileMaps &maps, Ctl *ctl, unsigned *done, unsigned *gmax, const SolveArgs &a,
-                int nsw, int sweeps, long long limit, int withhold, cudaStream_t s);
+                int nsw, int sweeps, bool each, long long limit, int withhold, cudaStream_t s);
 
 }  // namespace pcd

@@ -50,11 +50,12 @@ constexpr int kTBlock = kTThreads + 128, kTRegsSweep = 152, kTRegsProduce = 56;
 static_assert(kTThreads * kTRegsSweep + 128 * kTRegsProduce <= kTBlock * 128, "registers of the launch");
 
 constexpr int kTGroups = kTWarps * (32 / kTCL), kTRows = kTGroups * kTL;  // 96
-// NARROW: one lane column wide (8 cells), whose lane has both the grid's first
-// and its last column; the form with every cell's own weights.
+// RAG: the form with every cell's own weights, for the last tile column of a grid
+// whose last lane column is not whole, or also the first (8 cells wide).
 // UNI: a tile all of whose rows have both vertical neighbours.
-template <bool NARROW, bool UNI>
-using TileT = Tile<kTL, kTCL, NARROW, UNI>;
+template <bool RAG, bool UNI>
+using TileT = Tile<kTL, kTCL, RAG, UNI>;
+inline bool ragged(int W) { return W % 8 != 0 || W == 8; }
 
 // edge rows, two sets of -r32 planes (this tile's and the next one's), the next
 // tile's correction; and the written part of the last tile's (the written lane
@@ -265,22 +266,22 @@ __device__ __forceinline__ void tile_drain(const void *smem, TileShared *sh, int
 }
 
 // kr <= hk / 2 sweeps on the tile in the landing planes and plane set `set`.
-template <bool TRACK, bool NARROW, bool UNI>
+template <bool TRACK, bool RAG, bool UNI>
 __device__ __forceinline__ bool tile_sweeps(float *smem, TileShared *sh, const TileItem &it, int W, int H, int hk,
                                             int n, const float *w32, float &mx)
 {
     const TileGeom g = it.g;
     const int kr = it.kr;
-    TileT<NARROW, UNI> st;
+    TileT<RAG, UNI> st;
     st.place(smem, kTGroups);
-    const int q = g.qbase + st.cl, KQ = W >> 3;
+    const int q = g.qbase + st.cl, KQ = (W + 7) >> 3;
     const bool act = st.cl < g.nq + 2 && q >= 0 && q < KQ;
     st.y0 = g.ybase + st.lr0;
     st.H = H;
     st.own = st.cl >= 1 && st.cl <= g.nq;
     st.zl = q == 0;
-    st.zr = q == KQ - 1;
-    st.nvalid = 8;
+    st.nvalid = RAG ? min(8, W - 8 * q) : 8;
+    st.zr = q == KQ - 1 && st.nvalid == 8;
     st.gin = st.y0 < H && st.y0 + kTL > 0;
     st.brd = __any_sync(0xffffffffu, st.gin && (st.y0 <= 0 || st.y0 + kTL >= H));
     st.setup_weights(act, kTRows, w32);
@@ -327,7 +328,7 @@ __device__ __forceinline__ bool tile_sweeps(float *smem, TileShared *sh, const T
 
 // The sweeping warps: tile after tile, as they land.  grid(it, W, H, w32): the
 // grid of a tile; gmax: each pass's largest |update| (TRACK).
-template <bool TRACK, bool NARROW, typename Grid>
+template <bool TRACK, bool RAGGED, typename Grid>
 __device__ __forceinline__ void tile_consume(float *smem, TileShared *sh, int hk, int *error, unsigned *gmax, Grid grid)
 {
     const unsigned full = shared_at(&sh->full);
@@ -353,10 +354,12 @@ __device__ __forceinline__ void tile_consume(float *smem, TileShared *sh, int hk
         int W, H;
         grid(it, W, H, w32);
         float mx = 0.f;
-        if (!NARROW && it.g.ybase > 0 && it.g.ybase + kTRows < H)
-            fine = tile_sweeps<TRACK, NARROW, true>(smem, sh, it, W, H, hk, n, w32, mx);
+        if (RAGGED && it.g.qbase + it.g.nq + 2 >= (W + 7) >> 3)
+            fine = tile_sweeps<TRACK, RAGGED, false>(smem, sh, it, W, H, hk, n, w32, mx);
+        else if (it.g.ybase > 0 && it.g.ybase + kTRows < H)
+            fine = tile_sweeps<TRACK, false, true>(smem, sh, it, W, H, hk, n, w32, mx);
         else
-            fine = tile_sweeps<TRACK, NARROW, false>(smem, sh, it, W, H, hk, n, w32, mx);
+            fine = tile_sweeps<TRACK, false, false>(smem, sh, it, W, H, hk, n, w32, mx);
         if (TRACK) {
             const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
             if ((threadIdx.x & 31) == 0 && m) atomicMax(gmax + it.pass, m);
@@ -388,14 +391,15 @@ __device__ __forceinline__ int tile_neighbour(int t, int ncol, int nrow)
 }
 
 // `sweeps` sweeps from 0 in ea, nsw in a pass (fewer in the last one and at the
-// sweep cap).  TRACK: the max-update stop after every pass.  Where a pass that is
+// sweep cap).  TRACK: the max-update stop, after every pass or (!each) after the
+// launch's last one.  Where a pass that is
 // not the launch's last one meets it, the launch has run too far: it leaves the
 // sweeps up to that pass in ctl->redo, and a launch with `again` (one without
 // TRACK) runs these, the first time's bits.
-template <bool TRACK, bool NARROW>
+template <bool TRACK, bool RAGGED>
 __global__ void __launch_bounds__(kTBlock, 1)
     k_tile_pass(const __grid_constant__ TileMaps maps, Ctl *ctl, unsigned *done, const __grid_constant__ SolveArgs a, int ncol, int nrow, int N, int hk, int nsw,
-                int sweeps, int again, unsigned *gmax, long long limit, int withhold)
+                int sweeps, int again, int each, unsigned *gmax, long long limit, int withhold)
 {
     if (*(volatile const int *)&ctl->halt || *(volatile const int *)&ctl->error) return;
     const int total = again ? *(volatile const int *)&ctl->redo
@@ -405,7 +409,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
     __shared__ TileShared sh;
     tile_begin(smem_f, &sh);
     const unsigned base = *(volatile const unsigned *)&ctl->res_epoch;
-    const int ntiles = ncol * nrow, KQ = a.W >> 3, passes = (total + nsw - 1) / nsw;
+    const int ntiles = ncol * nrow, KQ = (a.W + 7) >> 3, passes = (total + nsw - 1) / nsw;
     if (threadIdx.x >= kTThreads) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTRegsProduce));
         const int role = ((int)threadIdx.x - kTThreads) >> 5;
@@ -437,7 +441,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
                                        [&](const TileItem &it) { return &maps.out[it.side ? 0 : 1][it.wide]; });
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTRegsSweep));
-        tile_consume<TRACK, NARROW>(smem_f, &sh, hk, &ctl->error, gmax,
+        tile_consume<TRACK, RAGGED>(smem_f, &sh, hk, &ctl->error, gmax,
                                     [&](const TileItem &, int &W, int &H, const float *&w32) {
                                         W = a.W;
                                         H = a.H;
@@ -456,7 +460,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
     if (!s_last) return;
     __threadfence();
     if (TRACK) {
-        for (int p = threadIdx.x; p < passes; p += kTBlock)
+        for (int p = (each ? 0 : passes - 1) + (int)threadIdx.x; p < passes; p += kTBlock)
             if ((double)__uint_as_float(__ldcg(gmax + p)) < a.tol) atomicMin(&s_first, p);
         __syncthreads();
     }
@@ -509,7 +513,7 @@ __host__ __device__ inline int batch_rows(int H)
 // the end of the launch); the CTA that finishes last closes it for every
 // job that ran (sweep count, sweep cap, ping-pong side) and resets the counter.
 // sync: finished CTAs, epoch of done[].
-template <bool NARROW>
+template <bool RAGGED>
 __global__ void __launch_bounds__(kTBlock, 1)
     k_tile_batch(const TileJob *__restrict__ jobs, int njobs, int ntiles, int sweeps, unsigned *sync, unsigned *done,
                  long long limit)
@@ -575,7 +579,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
                                        [&](const TileItem &it) { return &jobs[it.job].maps.out[it.side ? 0 : 1][it.wide]; });
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTRegsSweep));
-        tile_consume<false, NARROW>(smem_f, &sh, hk, &jobs[0].ctl->error, nullptr,
+        tile_consume<false, RAGGED>(smem_f, &sh, hk, &jobs[0].ctl->error, nullptr,
                                     [&](const TileItem &it, int &W, int &H, const float *&w32) {
                                         const TileJob &J = jobs[it.job];
                                         W = J.W;
@@ -607,9 +611,9 @@ __global__ void __launch_bounds__(kTBlock, 1)
     }
 }
 
-const void *tile_kernel(bool track, bool narrow)
+const void *tile_kernel(bool track, bool rag)
 {
-    if (narrow) return track ? (const void *)k_tile_pass<true, true> : (const void *)k_tile_pass<false, true>;
+    if (rag) return track ? (const void *)k_tile_pass<true, true> : (const void *)k_tile_pass<false, true>;
     return track ? (const void *)k_tile_pass<true, false> : (const void *)k_tile_pass<false, false>;
 }
 
@@ -620,19 +624,19 @@ const void *batch_kernel(bool narrow)
 
 }  // namespace
 
-int tile_plan(int dev, int W, int H, int ld, int depth, TilePlan *plan)
+int tile_plan(int dev, int W, int H, int depth, TilePlan *plan)
 {
-    if (W < 8 || H < 1 || W % 8 != 0 || ld % 4 != 0) return PCD_BAD_ARG;
+    if (W < 8 || H < 1) return PCD_BAD_ARG;
     if (depth != 0 && depth != 2 && depth != 4) return PCD_BAD_ARG;
     TilePlan p;
     p.K = depth ? depth : kTilePassSweeps;
-    p.ncol = ceil_div(W / 8, kTCL - 2);
+    p.ncol = ceil_div(ceil_div(W, 8), kTCL - 2);
     p.nrow = ceil_div(H, kTRows - 4 * p.K);
     p.smem = tile_smem();
     int sms = 0, bps = 0;
     PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     for (bool track : {false, true}) {
-        const void *fn = tile_kernel(track, W == 8);
+        const void *fn = tile_kernel(track, ragged(W));
         PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
         PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kTBlock, p.smem));
         if (bps < 1) return PCD_BAD_ARG;
@@ -658,7 +662,7 @@ int tile_maps(float *ea, float *eb, const float *r32, int W, int H, int ncol, in
         set_error("tile SOR: cuTensorMapEncodeTiled is not available");
         return PCD_DEVICE_ERROR;
     }
-    const cuuint64_t KQ = (cuuint64_t)W / 8;
+    const cuuint64_t KQ = ((cuuint64_t)W + 7) / 8;
     const cuuint64_t dims[3] = {4 * KQ, 2, (cuuint64_t)H}, strides[2] = {16 * KQ, 32 * KQ};
     auto encode = [&](CUtensorMap *map, const float *base, int quads, int box_rows) {
         const cuuint32_t box[3] = {4 * (cuuint32_t)quads, 1, (cuuint32_t)box_rows}, estr[3] = {1, 1, 1};
@@ -679,21 +683,21 @@ int tile_maps(float *ea, float *eb, const float *r32, int W, int H, int ncol, in
 }
 
 int launch_tile(const TilePlan &p, const TileMaps &maps, Ctl *ctl, unsigned *done, unsigned *gmax, const SolveArgs &a,
-                int nsw, int sweeps, long long limit, int withhold, cudaStream_t s)
+                int nsw, int sweeps, bool each, long long limit, int withhold, cudaStream_t s)
 {
     if (nsw < 1 || nsw > p.K || sweeps < 1) {
         set_error("tile SOR: more sweeps than the plan's halo holds");
         return PCD_BAD_ARG;
     }
     const bool track = a.stop == PCD_STOP_MAX_UPDATE;
-    int ncol = p.ncol, nrow = p.nrow, rows = p.rows, hk = 2 * p.K, again = 0;
+    int ncol = p.ncol, nrow = p.nrow, rows = p.rows, hk = 2 * p.K, again = 0, every = each ? 1 : 0;
     void *params[] = {const_cast<TileMaps *>(&maps), &ctl, &done, const_cast<SolveArgs *>(&a), &ncol, &nrow, &rows, &hk,
-                      &nsw, &sweeps, &again, &gmax, &limit, &withhold};
-    PCD_CUDA(cudaLaunchCooperativeKernel(tile_kernel(track, a.W == 8), dim3(p.grid), dim3(kTBlock), params, p.smem, s));
+                      &nsw, &sweeps, &again, &every, &gmax, &limit, &withhold};
+    PCD_CUDA(cudaLaunchCooperativeKernel(tile_kernel(track, ragged(a.W)), dim3(p.grid), dim3(kTBlock), params, p.smem, s));
     count_launches(1);
-    if (track && sweeps > nsw) {
+    if (track && each && sweeps > nsw) {
         again = 1;
-        PCD_CUDA(cudaLaunchCooperativeKernel(tile_kernel(false, a.W == 8), dim3(p.grid), dim3(kTBlock), params, p.smem,
+        PCD_CUDA(cudaLaunchCooperativeKernel(tile_kernel(false, ragged(a.W)), dim3(p.grid), dim3(kTBlock), params, p.smem,
                                              s));
         count_launches(1);
     }

@@ -109,3 +109,46 @@ def test_tile_wait_runs_out():
     assert L.pcd_ctx_set_wait_limit(c.handle, 0, 0) == 0
     assert c.solve_device(b, start.clone(), o)["converged"]
     c.close()
+
+
+# wider than the chip's registers hold, not a whole number of lane columns or of
+# 16-byte rows: the last tile column in a whole and in a partial lane column, one
+# cell to seven in it
+RAGGED = [(1801, 1201, 1801), (1802, 1203, 1804), (1998, 1700, 2000), (2047, 1900, 2048), (1912, 1207, 1913),
+          (4103, 600, 4104)]
+
+
+def _auto(ctx, n, m, ld, sched, **kw):
+    import torch
+
+    import poisson_caustic_design_gb300 as pcd
+
+    b0, start = _problem(n, m)
+    b = torch.zeros((m, ld), dtype=torch.float64, device="cuda")[:, :n]
+    phi = torch.zeros((m, ld), dtype=torch.float64, device="cuda")[:, :n]
+    b.copy_(b0)
+    phi.copy_(start)
+    st = ctx.solve_device(b, phi, pcd.SolveOptions(precision=pcd.PREC_MIXED, omega=-1.0, schedule=sched, **kw))
+    return st, phi
+
+
+@pytest.mark.parametrize("n,m,ld", RAGGED)
+@pytest.mark.parametrize("sweeps", [3, 75])
+def test_ragged_grids_match_launch_schedule(ctx, n, m, ld, sweeps):
+    ref = _auto(ctx, n, m, ld, 1, stop=1, tol=0.0, max_iterations=sweeps, refine_every=32)
+    got = _auto(ctx, n, m, ld, 0, stop=1, tol=0.0, max_iterations=sweeps, refine_every=32)
+    assert got[0]["sweeps"] == ref[0]["sweeps"] == sweeps
+    assert _agree(got[1], ref[1])
+
+
+@pytest.mark.parametrize("n,m,ld", RAGGED[:4])
+@pytest.mark.parametrize("stop,tol,check_every", [(0, 2e-2, 0), (0, 2e-2, 3), (1, 0.3, 0)])
+def test_ragged_grids_keep_their_stop_tests(ctx, n, m, ld, stop, tol, check_every):
+    """AUTO's sweeps end where those of the schedule would that takes the grid
+    otherwise: stream passes, or stripes."""
+    ref = _auto(ctx, n, m, ld, 2, stop=stop, tol=tol, max_iterations=20000, check_every=check_every)
+    assert ref[0]["schedule_used"] in (4, 5) and ref[0]["converged"]
+    got = _auto(ctx, n, m, ld, 0, stop=stop, tol=tol, max_iterations=20000, check_every=check_every)
+    assert got[0]["converged"] and got[0]["schedule_used"] == ref[0]["schedule_used"]
+    assert got[0]["sweeps"] == ref[0]["sweeps"]
+    assert _agree(got[1] - got[1].mean(), ref[1] - ref[1].mean())
