@@ -41,12 +41,12 @@ TOL = 1e-6
 METRIC = "OT solve wall-time to residual 1e-6 at 512²: learned+mixed vs plain GPU"
 UNIT = "ms/solve"
 SEEDS = [(s, "gaussian" if s % 2 == 0 else "binary") for s in range(8)]
-# DRAM bytes (read + write) of one k_sor_cluster_rr launch of the autotuned
-# headline solve, ncu (profiles/k_sor_cluster_rr_512_autotuned.md)
-CLUSTER_DRAM_BYTES_PER_LAUNCH = 2.183e6
+# DRAM bytes (read + write) of one k_sor_resident launch of a 512^2 solve, ncu
+# (profiles/solver_kernels.md)
+RESIDENT_DRAM_BYTES_PER_LAUNCH = 3.237e6
 # FP64 operations per cell-sweep of the block schedule's update and the
 # measured FP64 FMA rate of this part (dependent-free FMA loop, all SMs)
-FP64_OPS_PER_CELL = 5
+FP64_OPS_PER_CELL = 4
 FP64_OPS_PER_S = 0.60e12
 
 
@@ -719,28 +719,27 @@ def run_ours(args, rank, world, local, pg):
     if e2e_ms:
         print("e2e samples (ms): " + " ".join(f"{t:.2f}" for t in e2e_ms), file=sys.stderr, flush=True)
 
-    # roofline of the dominant kernel of the headline step: the FP32 cluster
-    # sweep kernel (k_sor_cluster_rr, one launch per FP32 cycle).  Algorithmic
-    # bytes per cell-sweep: 12 (read e, read r32, write e in FP32); a launch
-    # runs sweeps / cycles sweeps (cycles = FP64 residual evaluations - 1 on
-    # the cluster schedule), over the sweep kernels' device time (CUDA events
-    # on the context stream around the cycle loop).
+    # roofline of the dominant kernel of the headline step: the resident FP32
+    # sweeps (k_sor_resident, one launch per FP32 cycle).  Algorithmic bytes per
+    # cell-sweep: 12 (read e, read r32, write e in FP32); a launch runs sweeps /
+    # cycles sweeps (cycles = FP64 residual evaluations - 1), over the sweep
+    # kernels' device time (CUDA events on the context stream around the cycle
+    # loop, the FP64 refreshes with it).
     hm = results[headline]
     cells = N_GRID * N_GRID
     alg_bytes = 12.0 * cells * hm["sweeps"]
     achieved = alg_bytes / (hm["sweep_ms"] * 1e-3) / 1e9
     peak, peak_src = measured_hbm_peak()
     cycles = max(1.0, hm["residual_checks"] - 1.0)
-    # DRAM bytes per k_sor_cluster_rr launch of the autotuned headline
-    # configuration, from one ncu capture: the band load of e and r32 only --
-    # the grid stays on the cluster for the whole launch
+    # DRAM bytes per k_sor_resident launch, from one ncu capture: the load of
+    # r32 and the store of e only -- the grid stays on chip for the whole launch
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": CLUSTER_DRAM_BYTES_PER_LAUNCH, "traffic_unit": "bytes per launch (ncu)",
+            "traffic": RESIDENT_DRAM_BYTES_PER_LAUNCH, "traffic_unit": "bytes per launch (ncu)",
             "alg_bytes_per_launch": alg_bytes / cycles, "sweeps_per_launch": hm["sweeps"] / cycles,
-            "peak_source": peak_src, "kernel": "k_sor_cluster_rr (FP32 sweeps)", "alg_bytes_per_solve": alg_bytes,
-            "note": "the 512^2 working set stays on one 16-CTA cluster for a whole FP32 cycle (e in registers, "
-                    "r32 in shared memory): the kernel is bound by FP32 issue, block and cluster barriers, not "
-                    "HBM; DRAM traffic per launch is the band load and store (ncu summary under profiles/)"}
+            "peak_source": peak_src, "kernel": "k_sor_resident (FP32 sweeps)", "alg_bytes_per_solve": alg_bytes,
+            "note": "the 512^2 working set stays on all SMs for a whole FP32 cycle (e in registers, r32 in shared "
+                    "memory): the kernel is bound by the latency of block barriers and of halo words through L2, "
+                    "not HBM; DRAM traffic per launch is the load and store (ncu summary under profiles/)"}
     # the plain FP64 form's sweep kernel (the block schedule at 512^2) is bound
     # by the FP64 pipe: reported against the measured FP64 FMA rate of this part
     if "plain_fp64" in results:
@@ -749,7 +748,7 @@ def run_ours(args, rank, world, local, pg):
         roof["plain_fp64_sweep"] = {"us_per_sweep": us, "schedule": pf["schedule"],
                                     "alg_gbs": 24.0 * cells / (us * 1e-6) / 1e9,
                                     "fp64_issue_bound_us": FP64_OPS_PER_CELL * cells / FP64_OPS_PER_S * 1e6,
-                                    "note": "5 FP64 operations per cell-sweep over the measured 0.60 TFMA/s "
+                                    "note": "4 FP64 operations per cell-sweep over the measured 0.60 TFMA/s "
                                             "FP64 rate of this part"}
 
     # batched configuration: 64 instances, sizes uniform in {64..1024}^2,
@@ -837,7 +836,7 @@ def run_ours(args, rank, world, local, pg):
                    "l2": "flushed before every solve (512 MiB write)", "instances": len(SEEDS),
                    "autotuned": not args.no_autotune,
                    "schedule": {1: "launches", 2: "persistent", 3: "cluster", 4: "stripes",
-                                5: "stream"}.get(hm["schedule"], "?")},
+                                5: "stream", 6: "resident"}.get(hm["schedule"], "?")},
         "forms": {k: {**v, "err_vs_exact_fp64": acc.get(k)} for k, v in results.items()},
         "speedup_plain_over_mixed": (results["plain_fp64"]["ms"] / results["mixed"]["ms"]
                                      if "plain_fp64" in results else None),

@@ -98,9 +98,11 @@ typedef enum {
                                   to about two million cells; reported as PCD_SCHED_TILES, with
                                   the stop tests of the schedule they stand for: the cluster's
                                   estimate cycles, the tile passes' or the persistent bands'
-                                  chunks), else tile passes (grids of at least 64 x 64 cells),
-                                  else persistent, else stream; FP64: blocks, else persistent,
-                                  else stripes; else launches, as the grid allows */
+                                  chunks), else tile passes (widths that are not a multiple of 8
+                                  with the stop tests, and under the name, of the persistent,
+                                  stream or stripe schedule); grids below 64 x 64 cells or 16
+                                  on a side: persistent, else stream; FP64: blocks, else
+                                  persistent, else stripes; else launches, as the grid allows */
     PCD_SCHED_LAUNCHES = 1,    /* one kernel per half sweep, CUDA-graph chunks (any grid) */
     PCD_SCHED_PERSISTENT = 2,  /* one cooperative launch per solve, bands in shared memory
                                   (no NaN cells, band fits on chip) */
@@ -114,17 +116,14 @@ typedef enum {
     PCD_SCHED_STREAM = 5,      /* mixed precision, grids in HBM without NaN cells, ld a multiple
                                   of 4, W <= 4096: passes of one or two sweeps from one FP32
                                   correction buffer into another (row window in registers,
-                                  stripe edges recomputed, no boundary pass); AUTO picks it for
-                                  FP32 sweeps when neither the on-chip schedules nor the tile
-                                  passes apply */
+                                  stripe edges recomputed, no boundary pass) */
     PCD_SCHED_TILES = 6,       /* mixed precision, grids in HBM without NaN cells, width a multiple
                                   of 8, ld of 4: passes of up to 4 FP32 sweeps from one correction
                                   buffer into another, each tile of the grid held in registers
-                                  for the whole pass (halo recomputed); check_every = sweeps per
-                                  pass, i.e. between stop tests (1..4, 0 = 4), so the max |delta|
-                                  stop may come up to 3 sweeps after the first passing sweep;
-                                  AUTO picks it for FP32 sweeps when the cluster schedule does
-                                  not apply */
+                                  for the whole pass (halo recomputed), all passes of a chunk in
+                                  one cooperative launch; check_every = sweeps per pass, i.e.
+                                  between stop tests (1..4, 0 = 4), so the max |delta| stop may
+                                  come up to 3 sweeps after the first passing sweep */
     PCD_SCHED_BLOCKS = 7       /* grids without NaN cells: one cooperative launch per solve on
                                   2-D blocks (one per SM), each kept in shared memory with a
                                   halo of 2K cells, K red-black sweeps between exchanges of
