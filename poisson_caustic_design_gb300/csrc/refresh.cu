@@ -43,15 +43,8 @@ __device__ __forceinline__ bool is_nan_bits(double v)
     return ((unsigned long long)__double_as_longlong(v) << 1) > 0xffe0000000000000ull;
 }
 
-// Running max of |r| on the bit patterns (they order like the values; NaN
-// does not raise it), off the FP64 pipe.
-__device__ __forceinline__ unsigned long long max_abs_bits(unsigned long long m, double r)
-{
-    const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
-    return b > m && b <= 0x7ff0000000000000ull ? b : m;
-}
-
-// The same on words.
+// Running max of |r| on its words (they order like the values; NaN does not raise
+// it), off the FP64 pipe.
 __device__ __forceinline__ void max_abs_words(unsigned &mhi, unsigned &mlo, double r)
 {
     const unsigned hi = (unsigned)__double2hiint(r) & 0x7fffffffu, lo = (unsigned)__double2loint(r);
@@ -84,17 +77,67 @@ __device__ void rf_report(const Ctl *ctl, Ctl *report)
     for (int k = 0; k < (int)(sizeof(Ctl) / 8); k++) to[k] = from[k];
 }
 
-// Sums the blocks' partials in a fixed order (every thread of the block
-// calls); thread 0 has the result.
-__device__ void rf_sum_partials(const double *partials, int nblk, double (&v)[3])
+// The norms of a pass: sums of r^2 and b^2 and the largest |r|'s words.
+struct Norms {
+    double rr = 0.0, bb = 0.0;
+    unsigned hi = 0u, lo = 0u;
+    __device__ __forceinline__ double rmax() const { return __hiloint2double((int)hi, (int)lo); }
+};
+
+// The block's norms in thread 0, in a fixed order (every thread calls).  FP64
+// instructions are what it would wait for: five a sum and warp, none for the
+// maximum, and no sum that is not asked for.  (Three FP64 reductions, and
+// partials loaded one after the other: 23 us a 512^2 refresh, now 17.)
+template <bool BB>
+__device__ __forceinline__ void rf_block_norms(Norms &v)
 {
-    v[0] = v[1] = v[2] = 0.0;
-    for (int k = threadIdx.x; k < nblk; k += blockDim.x) {
-        v[0] += __ldcg(partials + 3 * k);
-        v[1] += __ldcg(partials + 3 * k + 1);
-        v[2] = nan_skip_max(v[2], __ldcg(partials + 3 * k + 2));
+    __shared__ Norms part[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+    v.rr = warp_sum(v.rr);
+    if (BB) v.bb = warp_sum(v.bb);
+    const unsigned hi = __reduce_max_sync(0xffffffffu, v.hi);
+    v.lo = __reduce_max_sync(0xffffffffu, v.hi == hi ? v.lo : 0u);
+    v.hi = hi;
+    __syncthreads();
+    if (lane == 0) part[w] = v;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int k = 1; k < nw; k++) {
+        const Norms &p = part[k];
+        v.rr += p.rr;
+        if (BB) v.bb += p.bb;
+        if (p.hi > v.hi || (p.hi == v.hi && p.lo > v.lo)) {
+            v.hi = p.hi;
+            v.lo = p.lo;
+        }
     }
-    block_reduce<3, 4u>(v);
+}
+
+// The blocks' norms (three doubles each) in thread 0 of the last block, in a fixed
+// order.
+template <bool BB>
+__device__ __forceinline__ Norms rf_all_norms(const double *partials, int nblk)
+{
+    Norms v;
+    for (int k0 = threadIdx.x; k0 < nblk; k0 += 4 * blockDim.x) {
+        double r[4], b[4], m[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = k0 + u * (int)blockDim.x;
+            const bool in = k < nblk;
+            r[u] = in ? __ldcg(partials + 3 * k) : 0.0;
+            b[u] = BB && in ? __ldcg(partials + 3 * k + 1) : 0.0;
+            m[u] = in ? __ldcg(partials + 3 * k + 2) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            v.rr += r[u];
+            if (BB) v.bb += b[u];
+            max_abs_words(v.hi, v.lo, m[u]);
+        }
+    }
+    rf_block_norms<BB>(v);
+    return v;
 }
 
 // FIRST: the start of a batch's solves (e = 0; zero: phi = 0 too, and written).
@@ -129,8 +172,7 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
     const int W = J.W, H = J.H, ld = J.ld, KQ = (W + 7) >> 3;
     const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     const int strips = (W + kRefreshCols - 1) / kRefreshCols, pieces = (H + J.rows - 1) / J.rows;
-    double acc = 0.0, acc_b = 0.0;
-    unsigned mhi = 0u, mlo = 0u;  // the largest |r|'s words
+    Norms v;
     for (int item = ((int)blockIdx.x - J.blk0) * kRefreshWarps + w; item < strips * pieces;
          item += J.nblk * kRefreshWarps) {
         const int piece = item / strips, strip = item - piece * strips;
@@ -188,9 +230,9 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
                 const unsigned k = (unsigned)(y - yb);
                 if (!FIRST || zero) *reinterpret_cast<double *>(p_out + (k * row + at * 8u)) = xc;
                 *reinterpret_cast<float *>(p_r + (k * row32 + col)) = -(float)r;
-                acc = fma(r, r, acc);
-                if (FIRST) acc_b = fma(bc, bc, acc_b);
-                max_abs_words(mhi, mlo, r);
+                v.rr = fma(r, r, v.rr);
+                if (FIRST) v.bb = fma(bc, bc, v.bb);
+                max_abs_words(v.hi, v.lo, r);
             }
             dp = d;
             xc = xn;
@@ -199,23 +241,22 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
             bc = bn;
         }
     }
-    const unsigned long long mbits = ((unsigned long long)mhi << 32) | mlo;
-    double v[3] = {acc, acc_b, __longlong_as_double((long long)mbits)};
-    block_reduce<3, 4u>(v);
+    rf_block_norms<FIRST>(v);
     if (threadIdx.x == 0) {
         double *p = J.partials + 3 * ((int)blockIdx.x - J.blk0);
-        p[0] = v[0];
-        p[1] = v[1];
-        p[2] = v[2];
+        p[0] = v.rr;
+        p[1] = v.bb;
+        p[2] = v.rmax();
     }
     if (!rf_last_block(ctl, J.nblk)) return;
-    rf_sum_partials(J.partials, J.nblk, v);
+    const double bnorm = FIRST ? 0.0 : *(const volatile double *)&ctl->bnorm;
+    v = rf_all_norms<FIRST>(J.partials, J.nblk);
     if (threadIdx.x == 0) {
         volatile Ctl *c = ctl;
-        if (FIRST) c->bnorm = sqrt(v[1]);
-        const double rn = sqrt(v[0]), bn = c->bnorm, rel = bn > 0.0 ? rn / bn : rn;
+        const double rn = sqrt(v.rr), bn = FIRST ? sqrt(v.bb) : bnorm, rel = bn > 0.0 ? rn / bn : rn;
+        if (FIRST) c->bnorm = bn;
         c->rnorm = rn;
-        c->rmax = v[2];
+        c->rmax = v.rmax();
         c->rel = rel;
         c->checks = c->checks + 1;
         if (tol >= 0.0 && rel <= tol) {
@@ -246,8 +287,7 @@ __global__ void __launch_bounds__(kStartThreads)
             int test)
 {
     const int W = a.W, H = a.H, ld = a.ld;
-    double v[3] = {0.0, 0.0, 0.0};
-    unsigned long long mbits = 0ull;
+    Norms v;
     int nans = 0;
     const int KQ = (W + 7) >> 3;
     const int last = in_quads ? 8 * KQ : W;
@@ -284,29 +324,28 @@ __global__ void __launch_bounds__(kStartThreads)
                 nans++;
                 continue;
             }
-            if (!ZERO) v[0] = fma(r, r, v[0]);
-            v[1] = fma(bi, bi, v[1]);
-            mbits = max_abs_bits(mbits, r);
+            if (!ZERO) v.rr = fma(r, r, v.rr);
+            v.bb = fma(bi, bi, v.bb);
+            max_abs_words(v.hi, v.lo, r);
         }
     }
-    if (ZERO) v[0] = v[1];
+    if (ZERO) v.rr = v.bb;
     if (nans) atomicAdd(&ctl->nan_cells, nans);
-    v[2] = __longlong_as_double((long long)mbits);
-    block_reduce<3, 4u>(v);
+    rf_block_norms<true>(v);
     const int blk = blockIdx.y * gridDim.x + blockIdx.x, nblk = gridDim.x * gridDim.y;
     if (threadIdx.x == 0) {
-        partials[3 * blk] = v[0];
-        partials[3 * blk + 1] = v[1];
-        partials[3 * blk + 2] = v[2];
+        partials[3 * blk] = v.rr;
+        partials[3 * blk + 1] = v.bb;
+        partials[3 * blk + 2] = v.rmax();
     }
     if (!rf_last_block(ctl, nblk)) return;
-    rf_sum_partials(partials, nblk, v);
+    v = rf_all_norms<true>(partials, nblk);
     if (threadIdx.x == 0) {
         volatile Ctl *c = ctl;
-        const double rn = sqrt(v[0]), bn = sqrt(v[1]), rel = bn > 0.0 ? rn / bn : rn;
+        const double rn = sqrt(v.rr), bn = sqrt(v.bb), rel = bn > 0.0 ? rn / bn : rn;
         c->rnorm = rn;
         c->bnorm = bn;
-        c->rmax = v[2];
+        c->rmax = v.rmax();
         c->rel = rel;
         c->checks = c->checks + 1;
         if (test && rel <= a.tol) {
