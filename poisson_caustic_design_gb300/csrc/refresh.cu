@@ -360,26 +360,28 @@ __global__ void __launch_bounds__(kStartThreads)
 
 }  // namespace
 
-int refresh_shape(int W, int H, int cap, double share, int *rows)
+int refresh_shape(int W, int H, int ld, int cap, double share, int *rows)
 {
     // An SM's time is that of its warps' FP64 instructions, six a row and five
     // for the rows of overlap, on one pipe; with fewer than twelve warps on it,
     // their latency.  All blocks are resident at once, so the fullest SM counts.
     const int strips = ceil_div(W, kRefreshCols);
     const double sms = std::max(1.0, kRefreshSms * share);
+    // (a piece's places are byte offsets in 32 bits: four rows more than it has)
+    const int most = (int)std::max<long>(1, std::min<long>(H, (1l << 32) / (8l * ld) - 4));
     double best = 0.0;
     int best_rows = 0, best_blocks = 1;
-    for (int r = 4; r <= std::max(4, H); r += r < 32 ? 1 : r / 16) {
-        const int blocks = ceil_div((long)strips * ceil_div(H, r), kRefreshWarps);
+    for (int r = std::min(4, most); r <= most; r += r < 32 ? 1 : r / 16) {
+        const long blocks = ((long)strips * ceil_div(H, r) + kRefreshWarps - 1) / kRefreshWarps;
         if (blocks > kRefreshResident * sms || blocks > cap) continue;
         const double t = std::max(12.0, kRefreshWarps * std::ceil(blocks / sms)) * (6 * r + 5);
         if (best_rows && t >= best) continue;
         best = t;
         best_rows = r;
-        best_blocks = blocks;
+        best_blocks = (int)blocks;
     }
-    if (!best_rows) {  // more strips than warps
-        best_rows = std::max(32, H);
+    if (!best_rows) {  // more pieces than warps
+        best_rows = most;
         best_blocks = std::max(1, std::min<int>(cap, (int)(kRefreshResident * sms)));
     }
     *rows = best_rows;

@@ -677,7 +677,7 @@ RefreshJob refresh_job(const SolverWorkspace &ws, const double *b, double *phi, 
     j.W = a.W;
     j.H = a.H;
     j.ld = a.ld;
-    j.nblk = refresh_shape(a.W, a.H, kResidualBlocksMax, 1.0, &j.rows);
+    j.nblk = refresh_shape(a.W, a.H, a.ld, kResidualBlocksMax, 1.0, &j.rows);
     return j;
 }
 
@@ -1141,7 +1141,7 @@ struct ResidentRule {
 
 // Grids that the tile passes take under any schedule.  Others (AUTO alone) keep
 // the stop tests of the schedules that they had before.
-bool tile_grid(int W, int ld) { return W >= 8 && W % 8 == 0 && ld % 4 == 0; }
+bool tile_grid(int W, int ld) { return W >= 8 && W % 8 == 0 && ld % 4 == 0 && ld < kRefreshLdMax; }
 
 // FP32 sweeps between FP64 refreshes of the chunked mixed schedules.
 int mixed_chunk(const SolveArgs &a, const pcd_solve_opts &o)
@@ -1164,7 +1164,7 @@ int mixed_chunk(const SolveArgs &a, const pcd_solve_opts &o)
 int resident_rule(SolverWorkspace &ws, const SolveArgs &a, const pcd_solve_opts &o, ResidentPlan *plan,
                   ResidentRule *rule)
 {
-    if (o.precision != PCD_PREC_MIXED || o.schedule != PCD_SCHED_AUTO) return PCD_BAD_ARG;
+    if (o.precision != PCD_PREC_MIXED || o.schedule != PCD_SCHED_AUTO || a.ld >= kRefreshLdMax) return PCD_BAD_ARG;
     const int W = a.W, H = a.H;
     int st = cached_plan(ws, {kPlanResident, W, H}, plan, [&](ResidentPlan *p) { return resident_plan(ws.dev, W, H, p); });
     if (st != PCD_OK) return st;
@@ -1538,7 +1538,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
     // its refreshes, the stream passes 22.9; 9.1 and 24.5 to the max-update stop.
     TilePlan tp;
     if (!done_already && !masked && mixed && !prefer_tiles && o.schedule == PCD_SCHED_AUTO && W >= 16 && H >= 16 &&
-        (long)W * H >= kTileMinCells) {
+        ld < kRefreshLdMax && (long)W * H >= kTileMinCells) {
         int G = 0, chunk = mixed_chunk(a, o), nsw = 1, name = PCD_SCHED_STRIPES;
         size_t smem = 0;
         StreamPlan probe;
@@ -1759,7 +1759,8 @@ bool batch_tiles_apply(const pcd_instance *inst, int count)
     if (!inst || count < 1 || count > kTileBatchJobsMax) return false;
     for (int i = 0; i < count; i++) {
         const pcd_instance &q = inst[i];
-        if (!q.b || !q.phi || q.width < 8 || q.height < 1 || q.width % 8 != 0 || q.ld < q.width || q.ld % 4 != 0)
+        if (!q.b || !q.phi || q.width < 8 || q.height < 1 || q.width % 8 != 0 || q.ld < q.width || q.ld % 4 != 0 ||
+            q.ld >= kRefreshLdMax)
             return false;
     }
     return true;
@@ -1827,7 +1828,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         r.H = q.height;
         r.ld = q.ld;
         r.blk0 = blocks;
-        r.nblk = refresh_shape(q.width, q.height, kBatchRefineBlocks,
+        r.nblk = refresh_shape(q.width, q.height, q.ld, kBatchRefineBlocks,
                                (double)q.width * q.height / (double)all_cells, &r.rows);
         blocks += r.nblk;
         off += (size_t)q.height * q.ld;
