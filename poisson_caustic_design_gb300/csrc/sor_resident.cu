@@ -288,6 +288,24 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
             sweeps += kr;
             const bool last = sweeps >= target;
             const bool decide = pending && sweeps >= snap_at;
+            // (the border quads leave before anything is waited for, and the
+            // partials below are polled while they travel: 1.92 ms a 512^2 solve,
+            // with the poll first and one warp's sum behind a barrier 1.96)
+            Words *xb = nullptr;
+            if (!last && G > 1) {
+                ++ep;
+                xb = reinterpret_cast<Words *>(a.xb) + (size_t)(ep & 1) * 2 * xplane;
+                // ---- own border quads out
+                if (pub) {
+                    Words *p = xb + ((long)st.y0 * a.KQ + q);
+#pragma unroll
+                    for (int j = 0; j < L; j++, p += a.KQ)
+                        if (pub >> j & 1u) {
+                            st4(p, rs_words(st.e[0][j], ep));
+                            st4(p + xplane, rs_words(st.e[1][j], ep));
+                        }
+                }
+            }
             if (decide && G > 1) {
                 // the partials of every CTA, posted at least half a sweep ago
                 for (int t = threadIdx.x; t < G; t += NT) {
@@ -302,18 +320,6 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
                 }
             }
             if (!last && G > 1) {
-                ++ep;
-                Words *xb = reinterpret_cast<Words *>(a.xb) + (size_t)(ep & 1) * 2 * xplane;
-                // ---- own border quads out
-                if (pub) {
-                    Words *p = xb + ((long)st.y0 * a.KQ + q);
-#pragma unroll
-                    for (int j = 0; j < L; j++, p += a.KQ)
-                        if (pub >> j & 1u) {
-                            st4(p, rs_words(st.e[0][j], ep));
-                            st4(p + xplane, rs_words(st.e[1][j], ep));
-                        }
-                }
                 // ---- halo quads in
                 constexpr int U = L <= 4 ? 4 : 2;
                 for (int id0 = threadIdx.x; id0 < halo_quads; id0 += U * NT) {
@@ -358,24 +364,23 @@ __global__ void __launch_bounds__(32 * rs_warps(L), 1) k_sor_resident(ResidentAr
             }
             if (G > 1 ? __syncthreads_or(failed) : 0) { failed = true; break; }
             if (decide) {
+                float tot;
                 if (G > 1) {
-                    // every CTA sums the same partials in the same order
-                    if (w == 0) {
-                        float x = 0.f;
-                        for (int t = lane; t < G; t += 32) x += s_vals[t];
-                        x = warp_sum_f(x);
-                        if (lane == 0) s_tot = x;
-                    }
-                    __syncthreads();
+                    // every warp of every CTA sums the same partials in the same order
+                    float x = 0.f;
+                    for (int t = lane; t < G; t += 32) x += s_vals[t];
+                    tot = warp_sum_f(x);
+                } else {
+                    __syncthreads();  // (posted behind the last sweep's barrier)
+                    tot = s_tot;
                 }
                 pending = false;
-                const double est2 = (double)s_tot;
+                const double est2 = (double)tot;
                 if (est2 <= s_lim) {
                     if (sweeps > snap_at) saved = true;  // e of sweep snap_at was written then
                     sweeps = snap_at;
                     break;
                 }
-                __syncthreads();
             }
             if (last) break;
             if (sweeps >= next_check) {
