@@ -95,6 +95,15 @@ __device__ __forceinline__ void block_reduce(double (&v)[N])
     __syncthreads();
 }
 
+// Zeroes device memory before work on any stream can use it: the contexts' streams
+// do not wait for the default stream, on which cudaMemset runs, nor does the
+// host wait for it.
+inline cudaError_t zero_now(void *p, size_t bytes)
+{
+    const cudaError_t e = cudaMemset(p, 0, bytes);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace pcd

@@ -130,7 +130,7 @@ int GridScratch::reserve()
     if (!buf) {
         PCD_CUDA(cudaMalloc(&buf, sizeof(double) * (2 + 2 * kBlocks)));
         PCD_CUDA(cudaMalloc(&counter, sizeof(unsigned int)));
-        PCD_CUDA(cudaMemset(counter, 0, sizeof(unsigned int)));
+        PCD_CUDA(zero_now(counter, sizeof(unsigned int)));
     }
     return PCD_OK;
 }

@@ -576,7 +576,7 @@ int *err_word()
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
     std::lock_guard<std::mutex> lk(mu);
-    if (!w[dev] && cudaMalloc(&w[dev], sizeof(int)) == cudaSuccess) cudaMemset(w[dev], 0, sizeof(int));
+    if (!w[dev] && cudaMalloc(&w[dev], sizeof(int)) == cudaSuccess) zero_now(w[dev], sizeof(int));
     return w[dev];
 }
 
@@ -730,7 +730,7 @@ int gemm_tc_error(int *out, bool reset)
     if (!w) return PCD_DEVICE_ERROR;
     PCD_CUDA(cudaDeviceSynchronize());
     PCD_CUDA(cudaMemcpy(out, w, sizeof(int), cudaMemcpyDeviceToHost));
-    if (reset) PCD_CUDA(cudaMemset(w, 0, sizeof(int)));
+    if (reset) PCD_CUDA(zero_now(w, sizeof(int)));
     return PCD_OK;
 }
 

@@ -795,7 +795,7 @@ int Design::alloc()
     PCD_CUDA(cudaMalloc(&qc, sizeof(double) * ((size_t)p.res_x + p.res_y + p.mesh_res_x + p.mesh_res_y)));
     PCD_CUDA(cudaMalloc(&scratch, sizeof(double) * (4 + 2 * 4096)));
     PCD_CUDA(cudaMalloc(&counter, 4 * sizeof(unsigned int)));
-    PCD_CUDA(cudaMemset(counter, 0, 4 * sizeof(unsigned int)));
+    PCD_CUDA(zero_now(counter, 4 * sizeof(unsigned int)));
     PCD_CUDA(cudaMalloc(&small, 8 * sizeof(unsigned long long)));
     PCD_CUDA(cudaMallocHost(&small_host, 8 * sizeof(unsigned long long)));
     return PCD_OK;

@@ -181,7 +181,7 @@ int UNet::build(int S_, int maxB_)
     nparams = np;
     // FP32 master, grad, adam m, v: 4 * np floats
     PCD_CUDA(cudaMalloc(&params_f, 4 * np * sizeof(float)));
-    PCD_CUDA(cudaMemset(params_f, 0, 4 * np * sizeof(float)));
+    PCD_CUDA(zero_now(params_f, 4 * np * sizeof(float)));
 
     // arena layout (bytes), sized for maxB
     const long P0 = (long)maxB * S * S, P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64;
@@ -242,7 +242,7 @@ int UNet::build(int S_, int maxB_)
     size_t total = 0;
     for (auto &pe : plan) total += pe.second;
     PCD_CUDA(cudaMalloc(&arena, total));
-    PCD_CUDA(cudaMemset(arena, 0, total));
+    PCD_CUDA(zero_now(arena, total));
     size_t o = 0;
     for (auto &pe : plan) {
         *pe.first = (unsigned char *)arena + o;
@@ -285,7 +285,7 @@ int UNet::init_random(unsigned long long seed)
 int UNet::set_params(const float *host)
 {
     PCD_CUDA(cudaMemcpy(params_f, host, nparams * sizeof(float), cudaMemcpyHostToDevice));
-    PCD_CUDA(cudaMemset(params_f + 2 * nparams, 0, 2 * nparams * sizeof(float)));
+    PCD_CUDA(zero_now(params_f + 2 * nparams, 2 * nparams * sizeof(float)));
     step = 0;
     PCD_TRY(sync_bf16(nullptr));
     PCD_CUDA(cudaDeviceSynchronize());
