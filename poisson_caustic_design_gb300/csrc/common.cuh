@@ -3,7 +3,10 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <map>
+#include <mutex>
 #include <string>
+#include <utility>
 
 #include "../../include/pcd.h"
 
@@ -102,6 +105,33 @@ inline cudaError_t zero_now(void *p, size_t bytes)
 {
     const cudaError_t e = cudaMemset(p, 0, bytes);
     return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
+// Lets fn be launched with all of an SM's shared memory that its static part
+// leaves.  The limit belongs to the function, not to a context: set to what one
+// plan needs, a smaller plan of another thread's context could lower it between the
+// set and the launch, which then failed with an invalid value.
+inline cudaError_t allow_shared(const void *fn)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, int> most;  // of the functions met so far
+    int dev = 0, bytes = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        const auto key = std::make_pair(dev, fn);
+        auto it = most.find(key);
+        if (it == most.end()) {
+            cudaFuncAttributes at;
+            if ((e = cudaFuncGetAttributes(&at, fn)) != cudaSuccess) return e;
+            if ((e = cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
+                return e;
+            it = most.emplace(key, bytes - (int)at.sharedSizeBytes).first;
+        }
+        bytes = it->second;
+    }
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }

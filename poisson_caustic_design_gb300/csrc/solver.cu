@@ -458,7 +458,7 @@ int stream_plan(int dev, int W, int H, int ld, bool allow_tma, StreamPlan *p)
     if (tma) {
         const void *fns[2] = {G == 1 ? (const void *)k_sweep_tma<1, false> : (const void *)k_sweep_tma<2, false>,
                               G == 1 ? (const void *)k_sweep_tma<1, true> : (const void *)k_sweep_tma<2, true>};
-        for (const void *fn : fns) PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        for (const void *fn : fns) PCD_CUDA(allow_shared(fn));
         int bps_t = 0;
         PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fns[0], T, smem));
         PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps_t, fns[1], T, smem));
@@ -492,7 +492,7 @@ int stream_plan(int dev, int W, int H, int ld, bool allow_tma, StreamPlan *p)
                                G == 1 ? (const void *)k_sweep2_tma<1, true> : (const void *)k_sweep2_tma<2, true>};
         int ok2 = 1;
         for (const void *fn : fns2) {
-            PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+            PCD_CUDA(allow_shared(fn));
             int b2 = 0;
             PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, fn, T, smem2));
             if (b2 < 1) ok2 = 0;

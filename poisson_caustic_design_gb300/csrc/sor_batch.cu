@@ -290,8 +290,7 @@ int batch_solve_device(BatchWorkspace &ws, int dev, const pcd_instance *inst, in
         else gper = std::max(gper, (size_t)C * planes_floats(nmax, plane_stride(q.width)));
     }
     PCD_CUDA(cudaFuncSetAttribute((const void *)k_sor_batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    PCD_CUDA(cudaFuncSetAttribute((const void *)k_sor_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::max<size_t>(smem, 16)));
+    PCD_CUDA(allow_shared((const void *)k_sor_batch));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -505,7 +505,7 @@ int blocks_plan(int dev, int W, int H, int K, bool mixed, BlocksPlan *plan)
 
 int launch_blocks(BlocksArgs &a, size_t smem, cudaStream_t s)
 {
-    PCD_CUDA(cudaFuncSetAttribute(k_sor_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PCD_CUDA(allow_shared((const void *)k_sor_blocks));
     void *params[] = {&a};
     PCD_CUDA(cudaLaunchCooperativeKernel((const void *)k_sor_blocks, dim3(a.G), dim3(kBlocksThreads), params, smem, s));
     count_launches(1);

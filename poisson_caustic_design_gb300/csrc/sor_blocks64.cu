@@ -385,7 +385,7 @@ int launch_blocks64(Blocks64Args &a, const Blocks64Plan &p, cudaStream_t s)
     a.G = p.TY * p.TX;
     a.K = p.K;
     a.RTmax = p.RTmax;
-    PCD_CUDA(cudaFuncSetAttribute(k_sor_blocks64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    PCD_CUDA(allow_shared((const void *)k_sor_blocks64));
     void *params[] = {&a};
     PCD_CUDA(cudaLaunchCooperativeKernel((const void *)k_sor_blocks64, dim3(a.G), dim3(kB64Threads), params, p.smem, s));
     count_launches(1);

@@ -464,7 +464,7 @@ namespace {
 bool cluster_fits(const void *fn, int C, int threads, size_t smem)
 {
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        allow_shared(fn) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -392,7 +392,7 @@ int persist_grid(int dev, int W, int H, bool mixed, int *G_out, size_t *smem_out
 int launch_persist(PersistArgs &a, bool mixed, size_t smem, cudaStream_t s)
 {
     void *fn = mixed ? (void *)k_sor_persist<true> : (void *)k_sor_persist<false>;
-    PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PCD_CUDA(allow_shared(fn));
     void *params[] = {&a};
     PCD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(a.G), dim3(kPersistThreads), params, smem, s));
     count_launches(1);

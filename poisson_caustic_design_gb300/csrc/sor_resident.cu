@@ -556,7 +556,7 @@ int launch_resident(ResidentArgs &a, const ResidentPlan &p, cudaStream_t s)
     a.TY = p.TY;
     a.NG = p.NG;
     a.R = p.R;
-    PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    PCD_CUDA(allow_shared(fn));
     void *params[] = {&a};
     if (p.TX * p.TY == 1) PCD_CUDA(cudaLaunchKernel(fn, dim3(1), dim3(32 * p.NW), params, p.smem, s));
     else PCD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.TX * p.TY), dim3(32 * p.NW), params, p.smem, s));

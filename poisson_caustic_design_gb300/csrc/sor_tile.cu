@@ -637,7 +637,7 @@ int tile_plan(int dev, int W, int H, int depth, TilePlan *plan)
     PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     for (bool track : {false, true}) {
         const void *fn = tile_kernel(track, ragged(W));
-        PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+        PCD_CUDA(allow_shared(fn));
         PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kTBlock, p.smem));
         if (bps < 1) return PCD_BAD_ARG;
     }
@@ -720,10 +720,10 @@ int tile_batch_config(int dev, int njobs, bool narrow, size_t *smem, int *grid)
     }
     const void *fn = batch_kernel(narrow);
     const size_t per_job = 2 * sizeof(int);
-    const size_t most = tile_smem() + kTileBatchJobsMax * per_job, bytes = tile_smem() + (size_t)njobs * per_job;
+    const size_t bytes = tile_smem() + (size_t)njobs * per_job;
     int sms = 0, bps = 0;
     PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PCD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    PCD_CUDA(allow_shared(fn));
     PCD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kTBlock, bytes));
     if (bps < 1) {
         set_error("batched tile pass: the kernel does not fit on an SM");
