@@ -230,9 +230,13 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
                 const unsigned k = (unsigned)(y - yb);
                 if (!FIRST || zero) *reinterpret_cast<double *>(p_out + (k * row + at * 8u)) = xc;
                 *reinterpret_cast<float *>(p_r + (k * row32 + col)) = -(float)r;
-                v.rr = fma(r, r, v.rr);
-                if (FIRST) v.bb = fma(bc, bc, v.bb);
-                max_abs_words(v.hi, v.lo, r);
+                // (a start's norms leave out cells whose b is NaN; after a sweep their
+                // correction is NaN, too, and no norm is a number any more)
+                if (!FIRST || !is_nan_bits(bc)) {
+                    v.rr = fma(r, r, v.rr);
+                    if (FIRST) v.bb = fma(bc, bc, v.bb);
+                    max_abs_words(v.hi, v.lo, r);
+                }
             }
             dp = d;
             xc = xn;
