@@ -1,0 +1,63 @@
+"""Fields beyond 32-bit byte offsets: rows further apart than the FP64 refresh
+takes, and more than 4 GB in a field."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def ctx():
+    import poisson_caustic_design_gb300 as pcd
+
+    c = pcd.Context(0)
+    yield c
+    c.close()
+
+
+def _grid(m, n, ld):
+    import torch
+
+    return torch.empty((m - 1) * ld + n, dtype=torch.float64, device="cuda").as_strided((m, n), (ld, 1))
+
+
+@pytest.mark.parametrize("stop", [0, 1])
+def test_rows_too_far_apart_for_the_refresh(ctx, stop):
+    """ld of 2^26 and more: AUTO falls back, and its solution is the compact grid's."""
+    import torch
+
+    import poisson_caustic_design_gb300 as pcd
+
+    m, n = 20, 40
+    o = pcd.SolveOptions(stop=stop, tol=1e-10, precision=pcd.PREC_MIXED, omega=-1.0, warm_start=0,
+                         max_iterations=20000)
+    rhs = torch.from_numpy(pcd.inputs.poisson_rhs(n, 4, "gaussian", m=m)).cuda()
+    ref = torch.zeros_like(rhs)
+    assert ctx.solve_device(rhs, ref, o)["converged"]
+    b, phi = _grid(m, n, (1 << 26) + 4), _grid(m, n, (1 << 26) + 4)
+    b.copy_(rhs)
+    st = ctx.solve_device(b, phi, o)
+    assert st["converged"] and st["schedule_used"] != pcd.SCHED_TILES
+    a, c = phi - phi.mean(), ref - ref.mean()
+    assert (a - c).abs().max() < 1e-7 * c.abs().max()
+
+
+def test_field_beyond_4_gb(ctx):
+    """131072 x 4100 cells: a strip of the refresh is cut where its byte offsets would
+    leave 32 bits (4092 rows).  The launch schedule's iterate after two sweeps, each with its refresh."""
+    import torch
+
+    import poisson_caustic_design_gb300 as pcd
+
+    m, n = 4100, 131072
+    x = torch.arange(n, dtype=torch.float64, device="cuda")
+    y = torch.arange(m, dtype=torch.float64, device="cuda")
+    b, start, phi = _grid(m, n, n), _grid(m, n, n), _grid(m, n, n)
+    torch.outer(torch.cos(y / 11.0), torch.sin(x / 13.0), out=b)
+    torch.outer(torch.sin(y / 5.0), torch.cos(x / 7.0), out=start)
+    o = dict(stop=pcd.STOP_REL_RESIDUAL, tol=0.0, max_iterations=2, refine_every=1, precision=pcd.PREC_MIXED,
+             omega=1.8, warm_start=1)
+    phi.copy_(start)
+    assert ctx.solve_device(b, phi, pcd.SolveOptions(schedule=pcd.SCHED_AUTO, **o))["schedule_used"] == pcd.SCHED_TILES
+    ctx.solve_device(b, start, pcd.SolveOptions(schedule=pcd.SCHED_LAUNCHES, **o))
+    start_max = start.abs().max()
+    assert (phi - start).abs_().max() < 1e-5 * start_max
