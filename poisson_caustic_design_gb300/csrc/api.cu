@@ -369,6 +369,8 @@ int pcd_ctx_set_wait_limit(pcd_ctx *ctx, long long polls, int withhold_first_fla
     std::lock_guard<std::mutex> lk(ctx->mu);
     ctx->solver.wait_limit = polls;
     ctx->solver.withhold_flag = withhold_first_flag ? 1 : 0;
+    ctx->batch.tiles.wait_limit = polls;
+    ctx->batch.tiles.withhold_flag = withhold_first_flag ? 1 : 0;
     return PCD_OK;
 }
 

@@ -1850,7 +1850,8 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     PCD_TRY(launch_first_refresh(d_rjobs, count, blocks, o.tol, !o.warm_start, s));
 
     // one CUDA graph per batch signature: the chunk's sweeps and the refresh
-    std::vector<long long> key = {count, tiles, blocks, chunk, narrow, grid, (long long)smem,
+    const long long limit = ws.wait_limit > 0 ? ws.wait_limit : kWordPolls;
+    std::vector<long long> key = {count, tiles, blocks, chunk, narrow, grid, (long long)smem, limit, ws.withhold_flag,
                                   (long long)(uintptr_t)ws.jobs, (long long)(uintptr_t)ws.rjobs,
                                   (long long)(uintptr_t)ws.sync};
     {
@@ -1865,7 +1866,8 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     } else {
         cudaGraph_t g;
         PCD_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        int st = launch_tile_batch(d_jobs, count, tiles, chunk, narrow, grid, smem, ws.sync, ws.sync + 2, kWordPolls, s);
+        int st = launch_tile_batch(d_jobs, count, tiles, chunk, narrow, grid, smem, ws.sync, ws.sync + 2, limit,
+                                   ws.withhold_flag, s);
         if (st == PCD_OK) st = launch_refresh(d_rjobs, RefreshJob{}, count, blocks, o.tol, s);
         cudaError_t ce = cudaStreamEndCapture(s, &g);
         if (st != PCD_OK) {

@@ -141,6 +141,9 @@ struct TileBatchWorkspace {
     unsigned *sync = nullptr;
     int sync_tiles = 0;
     int cap = 0;
+    // as the single solves' (pcd_ctx_set_wait_limit)
+    long long wait_limit = 0;
+    int withhold_flag = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     std::map<std::vector<long long>, cudaGraphExec_t> graphs;

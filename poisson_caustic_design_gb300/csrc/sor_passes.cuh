@@ -52,9 +52,10 @@ int tile_batch_config(int dev, int njobs, bool narrow, size_t *smem, int *grid);
 // `sweeps` sweeps (fewer at a grid's sweep cap) in passes of four over ntiles
 // tiles of njobs grids (d_jobs on the device, tile0 ascending), the corrections
 // starting from 0 in ea.  Cooperative.  sync (two words), done (one a tile):
-// zero before a solve's first launch; limit: polls before a wait gives up.
+// zero before a solve's first launch; limit: polls before a wait gives up;
+// withhold: tile 0 is never reported done.
 int launch_tile_batch(const TileJob *d_jobs, int njobs, int ntiles, int sweeps, bool narrow, int grid, size_t smem,
-                      unsigned *sync, unsigned *done, long long limit, cudaStream_t s);
+                      unsigned *sync, unsigned *done, long long limit, int withhold, cudaStream_t s);
 
 // The plan for a W x H grid (W >= 8); depth = sweeps per pass (2 or 4; 0: 4).
 // PCD_BAD_ARG when no form applies.

@@ -516,7 +516,7 @@ __host__ __device__ inline int batch_rows(int H)
 template <bool RAGGED>
 __global__ void __launch_bounds__(kTBlock, 1)
     k_tile_batch(const TileJob *__restrict__ jobs, int njobs, int ntiles, int sweeps, unsigned *sync, unsigned *done,
-                 long long limit)
+                 long long limit, int withhold)
 {
     constexpr int hk = 2 * kTilePassSweeps;
     extern __shared__ __align__(128) float smem_f[];  // (TMA boxes start at 128-byte addresses)
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
                 tile_fetch(smem_f, it.g, it.first ? nullptr : &J.maps.in[it.side], &J.maps.r32,
                            batch_rows(J.H) + 2 * hk, n & 1, shared_at(&sh.full));
             });
-        else if (role == 1) tile_drain(smem_f, &sh, hk, done, &jobs[0].ctl->error, 0,
+        else if (role == 1) tile_drain(smem_f, &sh, hk, done, &jobs[0].ctl->error, withhold,
                                        [&](const TileItem &it) { return &jobs[it.job].maps.out[it.side ? 0 : 1][it.wide]; });
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTRegsSweep));
@@ -735,13 +735,13 @@ int tile_batch_config(int dev, int njobs, bool narrow, size_t *smem, int *grid)
 }
 
 int launch_tile_batch(const TileJob *d_jobs, int njobs, int ntiles, int sweeps, bool narrow, int grid, size_t smem,
-                      unsigned *sync, unsigned *done, long long limit, cudaStream_t s)
+                      unsigned *sync, unsigned *done, long long limit, int withhold, cudaStream_t s)
 {
     if (njobs < 1 || njobs > kTileBatchJobsMax || ntiles < 1 || sweeps < 1) {
         set_error("batched tile pass: bad arguments");
         return PCD_BAD_ARG;
     }
-    void *params[] = {&d_jobs, &njobs, &ntiles, &sweeps, &sync, &done, &limit};
+    void *params[] = {&d_jobs, &njobs, &ntiles, &sweeps, &sync, &done, &limit, &withhold};
     PCD_CUDA(cudaLaunchCooperativeKernel(batch_kernel(narrow), dim3(std::min(grid, ntiles)), dim3(kTBlock), params, smem,
                                          s));
     return PCD_OK;
