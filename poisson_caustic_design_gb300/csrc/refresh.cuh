@@ -13,6 +13,7 @@ struct RefreshJob {
     const float *e0, *e1;    // the correction: e1 when ctl->stream_out is set
     float *r32;              // minus the right-hand side (both in the layout of sor_quads.cuh)
     Ctl *ctl;
+    const int *error;        // of the solve: the control block's, or the one that a batch shares
     double *partials;        // 3 per block
     int W, H, ld;
     int blk0, nblk;
@@ -26,10 +27,10 @@ struct RefreshJob {
 // rows of a piece.  ld < kRefreshLdMax.
 constexpr int kRefreshLdMax = 1 << 26;
 int refresh_shape(int W, int H, int ld, int cap, double share, int *rows);
-// For every job whose solve is not done: phi += e in FP64, r = b - L phi, -r in
-// FP32 to r32, the norms, and (tol >= 0) the relative-residual stop test; a solve
-// that has halted is then done.  jobs: on the device, or nullptr for the single
-// job `one`.
+// For every job whose solve is not done and has no error: phi += e in FP64, r = b -
+// L phi, -r in FP32 to r32, the norms, and (tol >= 0) the relative-residual stop
+// test; a solve that has halted is then done.  jobs: on the device, or nullptr for
+// the single job `one`.
 int launch_refresh(const RefreshJob *jobs, const RefreshJob &one, int njobs, int blocks, double tol, cudaStream_t s);
 // The same for the starts of a batch: e is 0 (zero: so is phi), the norms
 // include ||b||, and phi stays where it is.

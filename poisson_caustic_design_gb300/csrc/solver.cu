@@ -673,6 +673,7 @@ RefreshJob refresh_job(const SolverWorkspace &ws, const double *b, double *phi, 
     j.e1 = ws.e32b;
     j.r32 = ws.r32;
     j.ctl = ws.ctl;
+    j.error = &ws.ctl->error;
     j.partials = ws.partials;
     j.W = a.W;
     j.H = a.H;
@@ -1823,6 +1824,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         r.e1 = t.eb;
         r.r32 = ws.arena + 2 * per + off;
         r.ctl = t.ctl;
+        r.error = &ws.ctl->error;
         r.partials = ws.partials + (size_t)3 * kBatchRefineBlocks * k;
         r.W = q.width;
         r.H = q.height;
@@ -1896,8 +1898,9 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     long launched = 0;
     bool finished = false;
     auto all_done = [&](const Ctl *c) {
+        if (c[0].error) return true;  // (the batch's)
         for (int i = 0; i < count; i++)
-            if (!c[i].done && !c[i].error) return false;
+            if (!c[i].done) return false;
         return true;
     };
     while (!finished) {
@@ -1922,11 +1925,10 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     PCD_CUDA(cudaEventRecord(ws.t1, s));
     PCD_CUDA(cudaMemcpyAsync(ws.ctl_host, ws.ctl, sizeof(Ctl) * count, cudaMemcpyDeviceToHost, s));
     PCD_CUDA(cudaStreamSynchronize(s));
-    for (int k = 0; k < count; k++)
-        if (ws.ctl_host[k].error) {
-            set_error("batched tile solve: a bounded device wait gave up");
-            return ws.ctl_host[k].error;
-        }
+    if (ws.ctl_host[0].error) {
+        set_error("batched tile solve: a bounded device wait gave up");
+        return ws.ctl_host[0].error;
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ws.t0, ws.t1);
     int all = 1;

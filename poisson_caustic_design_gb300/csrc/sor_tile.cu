@@ -524,11 +524,14 @@ __global__ void __launch_bounds__(kTBlock, 1)
     __shared__ bool s_last;
     int *s_tile0 = reinterpret_cast<int *>(reinterpret_cast<Quad *>(smem_f) + kTQuads + kTOutQuads),
         *s_total = s_tile0 + njobs;
+    // the batch's error word is the first grid's
+    int *error = &jobs[0].ctl->error;
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile const int *)error)) return;
     for (int j = threadIdx.x; j < njobs; j += kTBlock) {
         const TileJob &J = jobs[j];
         const volatile Ctl *c = J.ctl;
         s_tile0[j] = J.tile0;
-        s_total[j] = c->halt || c->error ? 0 : max(0, min(sweeps, J.max_iter - c->sweeps));
+        s_total[j] = c->halt ? 0 : max(0, min(sweeps, J.max_iter - c->sweeps));
     }
     tile_begin(smem_f, &sh);
     // (the host wrote the jobs' maps to global memory: a thread for each tile of
@@ -546,7 +549,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
         const int role = ((int)threadIdx.x - kTThreads) >> 5;
         int t = (int)blockIdx.x - (int)gridDim.x, p = 0;
         if (role == 0) tile_produce(
-            &sh, done, base, &jobs[0].ctl->error, limit,
+            &sh, done, base, error, limit,
             [&](TileItem &it, int &nb) {
                 for (;;) {
                     t += gridDim.x;
@@ -575,11 +578,11 @@ __global__ void __launch_bounds__(kTBlock, 1)
                 tile_fetch(smem_f, it.g, it.first ? nullptr : &J.maps.in[it.side], &J.maps.r32,
                            batch_rows(J.H) + 2 * hk, n & 1, shared_at(&sh.full));
             });
-        else if (role == 1) tile_drain(smem_f, &sh, hk, done, &jobs[0].ctl->error, withhold,
+        else if (role == 1) tile_drain(smem_f, &sh, hk, done, error, withhold,
                                        [&](const TileItem &it) { return &jobs[it.job].maps.out[it.side ? 0 : 1][it.wide]; });
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTRegsSweep));
-        tile_consume<false, RAGGED>(smem_f, &sh, hk, &jobs[0].ctl->error, nullptr,
+        tile_consume<false, RAGGED>(smem_f, &sh, hk, error, nullptr,
                                     [&](const TileItem &it, int &W, int &H, const float *&w32) {
                                         const TileJob &J = jobs[it.job];
                                         W = J.W;
@@ -595,6 +598,9 @@ __global__ void __launch_bounds__(kTBlock, 1)
     __syncthreads();
     if (s_last) {
         __threadfence();
+        // (tiles were left out where a wait gave up: no grid's corrections are
+        // whole, and the refresh, which sees the word too, folds none of them in)
+        if (*(volatile const int *)error) return;
         for (int j = threadIdx.x; j < njobs; j += kTBlock) {
             if (s_total[j] < 1) continue;
             volatile Ctl *c = jobs[j].ctl;

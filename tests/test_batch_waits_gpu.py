@@ -55,3 +55,25 @@ def test_batch_wait_runs_out(ctx):
     pcd.batch_solve(other, bs, ref, _options())
     other.close()
     assert all(torch.equal(a, b) for a, b in zip(got, ref))
+
+
+def test_batch_stops_at_the_wait_that_ran_out(ctx):
+    """The chunk that failed is the last one, and no grid's potential takes up what its
+    tiles had left undone: with the failure in the first chunk each is its start."""
+    import torch
+
+    import poisson_caustic_design_gb300 as pcd
+
+    bs, starts = _grids()
+    phis = [s.clone() for s in starts]
+    L = pcd._lib.load()
+    assert L.pcd_ctx_set_wait_limit(ctx.handle, 2000, 1) == 0
+    before = L.pcd_kernel_launches()
+    with pytest.raises(pcd.PCDError) as err:
+        pcd.batch_solve(ctx, bs, phis, _options(max_iterations=20000))
+    # the start, three chunks of a pass and a refresh at most, the return of phi
+    launches = L.pcd_kernel_launches() - before
+    assert err.value.status == pcd._lib.PCD_TIMEOUT
+    assert L.pcd_ctx_set_wait_limit(ctx.handle, 0, 0) == 0
+    assert all(torch.equal(a, b) for a, b in zip(phis, starts))
+    assert launches <= 8, launches
