@@ -1283,7 +1283,8 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     ra.max_iter = a.max_iter;
     ra.cycle = rule.cycle;
     ra.nsw = rule.cycle ? (o.refine_every > 0 ? o.refine_every : 2048) : rule.chunk;
-    ra.check_every = o.check_every > 0 ? o.check_every : 16;
+    // (the kernel adds it to a sweep count: up to 2^30, beyond any launch's sweeps)
+    ra.check_every = o.check_every > 0 ? std::min(o.check_every, 1 << 30) : 16;
     ra.dep = rule.dep;
     ra.lag = rule.lag;
     ra.gran = rule.gran;
@@ -1304,9 +1305,9 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
 int solve_tiles(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const TilePlan &plan, int nsw,
                 int chunk, bool each, int sched, pcd_solve_stats *stats, cudaStream_t s)
 {
-    // a word a tile, and one a pass
-    const size_t tiles = (size_t)plan.ncol * plan.nrow;
-    PCD_TRY(reserve_words(ws, sizeof(unsigned) * (tiles + chunk), s));
+    // a word a tile, and for the max-update stop one a pass
+    const size_t tiles = (size_t)plan.ncol * plan.nrow, passes = (size_t)(chunk - 1) / nsw + 1;
+    PCD_TRY(reserve_words(ws, sizeof(unsigned) * (tiles + (a.stop == PCD_STOP_MAX_UPDATE ? passes : 0)), s));
     unsigned *done = static_cast<unsigned *>(ws.rx);
     TileMaps maps;
     PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, plan.ncol, plan.rows, 2 * plan.K, &maps));
@@ -1553,6 +1554,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
             if (probe.two) nsw = 2;
         }
         if (bands || a.stop != PCD_STOP_MAX_UPDATE) nsw = 4;
+        chunk = std::min(chunk, a.max_iter);
         if (tile_plan(ws.dev, W, H, nsw <= 2 ? 2 : 4, &tp) == PCD_OK) {
             if (!r32_quads) PCD_TRY(start(true));
             return solve_tiles(ws, b, phi, a, tp, nsw, chunk, !bands, name, stats, s);
@@ -1841,7 +1843,8 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     // sweeps between FP64 refreshes (passes of 4, the last one shorter):
     // refine_every, else 128 when the largest side is 1024 or more, down to
     // 32 when it is 256 or less
-    const int chunk = o.refine_every > 0 ? o.refine_every : 4 * std::max(8, std::min(32, maxdim / 32));
+    const int spacing = o.refine_every > 0 ? o.refine_every : 4 * std::max(8, std::min(32, maxdim / 32));
+    const int chunk = std::min(spacing, o.max_iterations);
 
     PCD_CUDA(cudaEventRecord(ws.t0, s));
     PCD_CUDA(cudaMemcpyAsync(ws.jobs, tj.data(), sizeof(TileJob) * count, cudaMemcpyHostToDevice, s));
@@ -1951,7 +1954,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         bstats->cluster_size = 0;
         bstats->smem_bytes = (long long)smem;
         bstats->cell_sweeps = cell_sweeps;
-        bstats->check_every = chunk;
+        bstats->check_every = spacing;
         bstats->refine_drop = 0.0;
         bstats->tuned = 0;
     }
