@@ -576,7 +576,11 @@ int *err_word()
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
     std::lock_guard<std::mutex> lk(mu);
-    if (!w[dev] && cudaMalloc(&w[dev], sizeof(int)) == cudaSuccess) zero_now(w[dev], sizeof(int));
+    int *p = nullptr;
+    if (!w[dev] && cudaMalloc(&p, sizeof(int)) == cudaSuccess) {
+        if (zero_now(p, sizeof(int)) == cudaSuccess) w[dev] = p;
+        else cudaFree(p);
+    }
     return w[dev];
 }
 
