@@ -44,6 +44,8 @@ SEEDS = [(s, "gaussian" if s % 2 == 0 else "binary") for s in range(8)]
 # DRAM bytes (read + write) of one k_sor_resident launch of a 512^2 solve, ncu
 # (profiles/solver_kernels.md)
 RESIDENT_DRAM_BYTES_PER_LAUNCH = 3.237e6
+# what a solve's sweeps ran on (pcd_solve_stats.sweep_form)
+SWEEP_FORMS = {0: "the schedule's kernels", 1: "k_sor_resident", 2: "k_tile_pass"}
 # FP64 operations per cell-sweep of the block schedule's update and the
 # measured FP64 FMA rate of this part (dependent-free FMA loop, all SMs)
 FP64_OPS_PER_CELL = 4
@@ -675,7 +677,7 @@ def run_ours(args, rank, world, local, pg):
         results[name] = {"ms": max_over_ranks(pg, float(np.sum(ms))) / args.steps, "sweeps": float(np.mean(sweeps)),
                          "sweep_ms": float(np.mean(sweep_ms)), "max_rel_residual": float(np.max(rels)),
                          "residual_checks": float(np.mean(checks)),
-                         "schedule": int(st["schedule_used"]),
+                         "schedule": int(st["schedule_used"]), "sweep_form": int(st["sweep_form"]),
                          "tuned": {"check_every": st["check_every_used"], "refine_every": st["refine_every_used"],
                                    "refine_drop": st["refine_drop_used"]}}
         if name == "learned_mixed":
@@ -719,8 +721,8 @@ def run_ours(args, rank, world, local, pg):
     if e2e_ms:
         print("e2e samples (ms): " + " ".join(f"{t:.2f}" for t in e2e_ms), file=sys.stderr, flush=True)
 
-    # roofline of the dominant kernel of the headline step: the resident FP32
-    # sweeps (k_sor_resident, one launch per FP32 cycle).  Algorithmic bytes per
+    # roofline of the dominant kernel of the headline step: the FP32 sweeps, by
+    # default k_sor_resident, one launch per FP32 cycle.  Algorithmic bytes per
     # cell-sweep: 12 (read e, read r32, write e in FP32); a launch runs sweeps /
     # cycles sweeps (cycles = FP64 residual evaluations - 1), over the sweep
     # kernels' device time (CUDA events on the context stream around the cycle
@@ -732,14 +734,18 @@ def run_ours(args, rank, world, local, pg):
     peak, peak_src = measured_hbm_peak()
     cycles = max(1.0, hm["residual_checks"] - 1.0)
     # DRAM bytes per k_sor_resident launch, from one ncu capture: the load of
-    # r32 and the store of e only -- the grid stays on chip for the whole launch
+    # r32 and the store of e only -- the grid stays on chip for the whole launch.
+    # (Where the autotuner took another kernel there is no such figure.)
+    on_chip = hm["sweep_form"] == 1
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": RESIDENT_DRAM_BYTES_PER_LAUNCH, "traffic_unit": "bytes per launch (ncu)",
+            "traffic": RESIDENT_DRAM_BYTES_PER_LAUNCH if on_chip else None, "traffic_unit": "bytes per launch (ncu)",
             "alg_bytes_per_launch": alg_bytes / cycles, "sweeps_per_launch": hm["sweeps"] / cycles,
-            "peak_source": peak_src, "kernel": "k_sor_resident (FP32 sweeps)", "alg_bytes_per_solve": alg_bytes,
+            "peak_source": peak_src, "kernel": SWEEP_FORMS[hm["sweep_form"]] + " (FP32 sweeps)",
+            "alg_bytes_per_solve": alg_bytes,
             "note": "the 512^2 working set stays on all SMs for a whole FP32 cycle (e in registers, r32 in shared "
                     "memory): the kernel is bound by the latency of block barriers and of halo words through L2, "
-                    "not HBM; DRAM traffic per launch is the load and store (ncu summary under profiles/)"}
+                    "not HBM; DRAM traffic per launch is the load and store (ncu summary under profiles/)"
+                    if on_chip else "FP32 sweeps of " + SWEEP_FORMS[hm["sweep_form"]]}
     # the plain FP64 form's sweep kernel (the block schedule at 512^2) is bound
     # by the FP64 pipe: reported against the measured FP64 FMA rate of this part
     if "plain_fp64" in results:
@@ -836,7 +842,8 @@ def run_ours(args, rank, world, local, pg):
                    "l2": "flushed before every solve (512 MiB write)", "instances": len(SEEDS),
                    "autotuned": not args.no_autotune,
                    "schedule": {1: "launches", 2: "persistent", 3: "cluster", 4: "stripes",
-                                5: "stream", 6: "resident"}.get(hm["schedule"], "?")},
+                                5: "stream", 6: "tiles", 7: "blocks"}.get(hm["schedule"], "?"),
+                   "sweeps_on": SWEEP_FORMS[hm["sweep_form"]]},
         "forms": {k: {**v, "err_vs_exact_fp64": acc.get(k)} for k, v in results.items()},
         "speedup_plain_over_mixed": (results["plain_fp64"]["ms"] / results["mixed"]["ms"]
                                      if "plain_fp64" in results else None),

@@ -141,13 +141,16 @@ typedef struct {
     double device_ms;        /* device time of the solve (CUDA events) */
     int residual_checks;     /* FP64 residual evaluations */
     double sweep_ms;         /* device time of the sweep kernel(s) alone (CUDA events) */
-    int schedule_used;       /* pcd_schedule that ran */
+    int schedule_used;       /* pcd_schedule whose stop tests were kept; what its sweeps ran on
+                                under AUTO: sweep_form */
     int warm_used;           /* 0 zero, 1 given, 2 learned, 3 learned prediction rejected (zero) */
     double warm_rel_residual;/* warm_start 2: ||b - L phi|| / ||b|| of the learned prediction after
                                 8 Gauss-Seidel sweeps (red-black, omega = 1) */
     int tuned;               /* 1: the context's autotuner chose the knobs below for this shape */
     int check_every_used;    /* check_every the solve ran with (0 = the schedule's default) */
     int refine_every_used;   /* refine_every the solve ran with (0 = default) */
+    int sweep_form;          /* 0: the kernels of schedule_used; 1: FP32 sweeps on tiles that stay on
+                                the chip; 2: FP32 passes over tiles of a grid in HBM */
     double refine_drop_used; /* refine_drop the solve ran with (0 = default) */
     double warm_zero_rel_residual; /* warm_start 2: the same for a zero guess after the same sweeps;
                                       the prediction is kept when warm_rel_residual is smaller */

@@ -80,6 +80,7 @@ class SolveStats(C.Structure):
         ("tuned", C.c_int),
         ("check_every_used", C.c_int),
         ("refine_every_used", C.c_int),
+        ("sweep_form", C.c_int),
         ("refine_drop_used", C.c_double),
         ("warm_zero_rel_residual", C.c_double),
     ]

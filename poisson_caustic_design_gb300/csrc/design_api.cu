@@ -140,6 +140,7 @@ static int run_lockstep(pcd_design *const *ds, int n, bool height, int *statuses
                 s.device_ms = bs.device_ms;
                 s.residual_checks = is[k].cycles;
                 s.schedule_used = bs.clusters == 0 ? PCD_SCHED_TILES : PCD_SCHED_CLUSTER;
+                s.sweep_form = bs.clusters == 0 ? 2 : 0;
                 s.warm_used = o.warm_start ? 1 : 0;
             }
             st[(size_t)i] = post(i);

@@ -1212,7 +1212,7 @@ int resident_rule(SolverWorkspace &ws, const SolveArgs &a, const pcd_solve_opts 
 // done.  The refresh leaves the control block in host memory itself: a copy
 // between it and the next chunk's launch took 9 us.
 template <typename Launch>
-int run_chunks(SolverWorkspace &ws, RefreshJob job, const SolveArgs &a, long max_launches, int sched,
+int run_chunks(SolverWorkspace &ws, RefreshJob job, const SolveArgs &a, long max_launches, int sched, int form,
                const char *what, pcd_solve_stats *stats, int *nans, cudaStream_t s, Launch launch)
 {
     PCD_CUDA(cudaEventRecord(ws.k0, s));
@@ -1254,6 +1254,7 @@ int run_chunks(SolverWorkspace &ws, RefreshJob job, const SolveArgs &a, long max
         cudaEventElapsedTime(&ms, ws.k0, ws.k1);
         stats->sweep_ms = ms;
         stats->schedule_used = sched;
+        stats->sweep_form = form;
     }
     return c.converged ? PCD_OK : PCD_NOT_CONVERGED;
 }
@@ -1295,7 +1296,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
     ra.withhold = ws.withhold_flag;
 
     const long max_launches = rule.cycle ? (long)a.max_iter + 4 : (long)a.max_iter / std::max(1, rule.chunk) + 3;
-    return run_chunks(ws, refresh_job(ws, b, phi, a), a, max_launches, rule.sched, "resident SOR", stats, nans, s,
+    return run_chunks(ws, refresh_job(ws, b, phi, a), a, max_launches, rule.sched, 1, "resident SOR", stats, nans, s,
                       [&] { return launch_resident(ra, plan, s); });
 }
 
@@ -1312,7 +1313,7 @@ int solve_tiles(SolverWorkspace &ws, const double *b, double *phi, const SolveAr
     TileMaps maps;
     PCD_TRY(tile_maps(ws.e32, ws.e32b, ws.r32, a.W, a.H, plan.ncol, plan.rows, 2 * plan.K, &maps));
     int nans = 0;
-    return run_chunks(ws, refresh_job(ws, b, phi, a), a, (long)a.max_iter / chunk + 3, sched, "tile SOR",
+    return run_chunks(ws, refresh_job(ws, b, phi, a), a, (long)a.max_iter / chunk + 3, sched, 2, "tile SOR",
                       stats, &nans, s, [&] {
                           return launch_tile(plan, maps, ws.ctl, done, done + tiles, a, nsw, chunk, each,
                                              ws.wait_limit > 0 ? ws.wait_limit : kWordPolls, ws.withhold_flag, s);
@@ -1452,6 +1453,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         set_error("pcd solve: bad options");
         return PCD_BAD_ARG;
     }
+    if (stats) stats->sweep_form = 0;
     PCD_TRY(ws.reserve((size_t)H * std::max<size_t>(ld, quads::quad_row_floats(W))));
 
     SolveArgs a;

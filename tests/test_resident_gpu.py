@@ -106,3 +106,15 @@ def test_resident_wait_runs_out():
     st, _ = _solve(c, b, stop=1, tol=1e-6, omega=-1.0)
     assert st["converged"] and st["schedule_used"] == 6
     c.close()
+
+
+@pytest.mark.parametrize("n,m,ld,schedule,used,form", [
+    (512, 512, 512, 0, 6, 1), (512, 512, 512, 6, 6, 2), (252, 188, 252, 0, 6, 1), (2048, 1500, 2048, 0, 6, 2),
+    (1801, 1201, 1801, 0, 4, 2), (2044, 1500, 2044, 0, 5, 2), (512, 512, 512, 3, 3, 0), (512, 512, 512, 1, 1, 0)])
+def test_stats_tell_what_the_sweeps_ran_on(ctx, n, m, ld, schedule, used, form):
+    """schedule_used names whose stop tests a solve keeps; sweep_form the kernel."""
+    import poisson_caustic_design_gb300 as pcd
+
+    b = pcd.inputs.poisson_rhs(max(n, m), 5, "gaussian", m=max(n, m))[:m, :n]
+    st, _ = _solve(ctx, b, ld=ld, stop=1, tol=1e-14, max_iterations=8, omega=1.9, schedule=schedule)
+    assert (st["schedule_used"], st["sweep_form"]) == (used, form)
