@@ -561,10 +561,16 @@ def config4_section(pcd, ctx, device, batch=16):
     steps = pcd.transport_iteration_batch(ds)
     torch.cuda.synchronize()
     t2 = time.perf_counter()
-    sweeps = [d.last_solve_stats["sweeps"] for d in ds]
+    solves = [d.last_solve_stats for d in ds]
+    sweeps = [s["sweeps"] for s in solves]
+    # (a solve at its cap would otherwise only be seen in the mean)
+    unfinished = [k for k, s in enumerate(solves) if not s["converged"]]
+    if unfinished:
+        print(f"config 4: solves that did not converge: {unfinished}", file=sys.stderr, flush=True)
     out = {"mesh": R, "grid": N, "targets": batch, "form": "mixed", "init_ms": (t1 - t0) * 1e3,
            "first_transport_ms": (t2 - t1) * 1e3, "ms_per_target_transport": (t2 - t1) * 1e3 / batch,
-           "sweeps_mean": float(np.mean(sweeps)), "steps_finite": bool(np.all(np.isfinite(steps)))}
+           "sweeps_mean": float(np.mean(sweeps)), "sweeps": sweeps, "all_converged": not unfinished,
+           "not_converged": unfinished, "steps_finite": bool(np.all(np.isfinite(steps)))}
     for d in ds:
         d.close()
     for c in ctxs:
