@@ -21,6 +21,7 @@ void count_launches(unsigned long long n);
     do {                                                                                   \
         cudaError_t e_ = (call);                                                           \
         if (e_ != cudaSuccess) {                                                           \
+            cudaGetLastError(); /* reported here, not by the next launch's check */        \
             ::pcd::set_error(std::string(#call) + ": " + cudaGetErrorString(e_) + " (" +    \
                              __FILE__ + ":" + std::to_string(__LINE__) + ")");             \
             return PCD_DEVICE_ERROR;                                                       \

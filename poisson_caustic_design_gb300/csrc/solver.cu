@@ -579,6 +579,7 @@ int SolverWorkspace::reserve(size_t n)
         if (r32) cudaFree(r32);
         if (r64) cudaFree(r64);
         mask = nullptr; e32 = nullptr; e32b = nullptr; r32 = nullptr; r64 = nullptr;
+        cells = 0;  // (until all of them are there again)
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second.exec);
         graphs.clear();
         PCD_CUDA(cudaMalloc(&mask, n));

@@ -61,3 +61,27 @@ def test_field_beyond_4_gb(ctx):
     ctx.solve_device(b, start, pcd.SolveOptions(schedule=pcd.SCHED_LAUNCHES, **o))
     start_max = start.abs().max()
     assert (phi - start).abs_().max() < 1e-5 * start_max
+
+
+def test_grid_beyond_memory_is_refused_and_the_context_goes_on(ctx):
+    """A grid whose workspace cannot be had (429 GB of its smallest buffer alone) is
+    an error, and the next solve works on buffers of its own again."""
+    import ctypes
+
+    import torch
+
+    import poisson_caustic_design_gb300 as pcd
+
+    b = torch.from_numpy(pcd.inputs.poisson_rhs(64, 4, "gaussian")).cuda()
+    o = pcd.SolveOptions(stop=1, tol=1e-6, precision=pcd.PREC_MIXED, omega=-1.0, warm_start=0)
+    out = []
+    for _ in range(2):
+        phi = torch.zeros_like(b)
+        assert ctx.solve_device(b, phi, o)["converged"]
+        out.append(phi)
+        st = pcd._lib.SolveStats()
+        c = o.to_c()
+        rc = pcd._lib.load().pcd_poisson_solve_device(ctx.handle, b.data_ptr(), phi.data_ptr(), 16, 200, 2**31 - 1,
+                                                      ctypes.byref(c), ctypes.byref(st), None)
+        assert rc == pcd._lib.PCD_DEVICE_ERROR
+    assert torch.equal(*out)
