@@ -32,7 +32,6 @@ namespace {
 
 constexpr int kRefreshWarps = 4;      // warps of a block
 constexpr int kRefreshResident = 4;   // blocks of an SM (4096^2: 305 us, with eight 330)
-constexpr int kRefreshSms = 152;
 constexpr int kRefreshCols = 30;      // columns a warp owns
 constexpr int kStartThreads = 256;
 
@@ -364,13 +363,13 @@ __global__ void __launch_bounds__(kStartThreads)
 
 }  // namespace
 
-int refresh_shape(int W, int H, int ld, int cap, double share, int *rows)
+int refresh_shape(int W, int H, int ld, int cap, double chip_sms, int *rows)
 {
     // An SM's time is that of its warps' FP64 instructions, six a row and five
     // for the rows of overlap, on one pipe; with fewer than twelve warps on it,
     // their latency.  All blocks are resident at once, so the fullest SM counts.
     const int strips = ceil_div(W, kRefreshCols);
-    const double sms = std::max(1.0, kRefreshSms * share);
+    const double sms = std::max(1.0, chip_sms);
     // (a piece's places are byte offsets in 32 bits: four rows more than it has)
     const int most = (int)std::max<long>(1, std::min<long>(H, (1l << 32) / (8l * ld) - 4));
     double best = 0.0;

@@ -23,10 +23,10 @@ struct RefreshJob {
     Ctl *report;
 };
 
-// Blocks of a W x H grid's refresh (at most cap) on `share` of the chip, and the
-// rows of a piece.  ld < kRefreshLdMax.
+// Blocks of a W x H grid's refresh (at most cap) on sms SMs, a batch's grid on its
+// share of them, and the rows of a piece.  ld < kRefreshLdMax.
 constexpr int kRefreshLdMax = 1 << 26;
-int refresh_shape(int W, int H, int ld, int cap, double share, int *rows);
+int refresh_shape(int W, int H, int ld, int cap, double sms, int *rows);
 // For every job whose solve is not done and has no error: phi += e in FP64, r = b -
 // L phi, -r in FP32 to r32, the norms, and (tol >= 0) the relative-residual stop
 // test; a solve that has halted is then done.  jobs: on the device, or nullptr for

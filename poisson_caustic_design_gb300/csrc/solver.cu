@@ -562,6 +562,7 @@ double resolve_omega(double omega, int W, int H)
 int SolverWorkspace::reserve(size_t n)
 {
     if (!ctl) {
+        PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         PCD_CUDA(cudaMalloc(&ctl, sizeof(Ctl)));
         PCD_CUDA(cudaMallocHost(&ctl_host, 2 * sizeof(Ctl)));
         PCD_CUDA(cudaMalloc(&partials, 3 * sizeof(double) * kResidualBlocksMax));
@@ -679,7 +680,7 @@ RefreshJob refresh_job(const SolverWorkspace &ws, const double *b, double *phi, 
     j.W = a.W;
     j.H = a.H;
     j.ld = a.ld;
-    j.nblk = refresh_shape(a.W, a.H, a.ld, kResidualBlocksMax, 1.0, &j.rows);
+    j.nblk = refresh_shape(a.W, a.H, a.ld, kResidualBlocksMax, ws.sms, &j.rows);
     return j;
 }
 
@@ -1785,7 +1786,8 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         return PCD_BAD_ARG;
     }
     size_t smem = 0;
-    int grid = 0;
+    int grid = 0, sms = 0;
+    PCD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     bool narrow = false;
     for (int i = 0; i < count; i++) narrow = narrow || inst[i].width == 8;
     PCD_TRY(tile_batch_config(dev, count, narrow, &smem, &grid));
@@ -1836,7 +1838,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
         r.ld = q.ld;
         r.blk0 = blocks;
         r.nblk = refresh_shape(q.width, q.height, q.ld, kBatchRefineBlocks,
-                               (double)q.width * q.height / (double)all_cells, &r.rows);
+                               sms * ((double)q.width * q.height / (double)all_cells), &r.rows);
         blocks += r.nblk;
         off += (size_t)q.height * q.ld;
     }

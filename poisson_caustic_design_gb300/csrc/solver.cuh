@@ -81,6 +81,7 @@ constexpr double kFp32StopFrac = 0.9;
 
 struct SolverWorkspace {
     int dev = 0;
+    int sms = 0;                // of the device
     size_t cells = 0;           // capacity in elements of the per-cell buffers
     uint8_t *mask = nullptr;    // neighbour-validity bits per cell
     float *e32 = nullptr;       // FP32 correction (mixed precision)
