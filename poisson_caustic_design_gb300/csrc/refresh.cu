@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(32 * kRefreshWarps)
     }
     Ctl *ctl = J.ctl;
     const int side = rf_load(&ctl->phi_side);
-    if (rf_load(&ctl->done) || rf_load(J.error) || rf_load(&ctl->nan_cells)) {
+    if (rf_load(&ctl->done) | rf_load(J.error) | rf_load(&ctl->nan_cells)) {  // (loads side by side)
         if (!J.report) return;
         if ((int)blockIdx.x == J.blk0 && threadIdx.x == 0) rf_report(ctl, J.report);
         if (side)

@@ -1146,6 +1146,10 @@ struct ResidentRule {
 // the stop tests of the schedules that they had before.
 bool tile_grid(int W, int ld) { return W >= 8 && W % 8 == 0 && ld % 4 == 0 && ld < kRefreshLdMax; }
 
+// Most sweeps of a launch of tile passes (their counts of passes are rounded up in 32
+// bits); no solve comes near it.
+constexpr int kChunkSweepsMax = 1 << 30;
+
 // FP32 sweeps between FP64 refreshes of the chunked mixed schedules.
 int mixed_chunk(const SolveArgs &a, const pcd_solve_opts &o)
 {
@@ -1308,6 +1312,7 @@ int solve_resident(SolverWorkspace &ws, const double *b, double *phi, const Solv
 int solve_tiles(SolverWorkspace &ws, const double *b, double *phi, const SolveArgs &a, const TilePlan &plan, int nsw,
                 int chunk, bool each, int sched, pcd_solve_stats *stats, cudaStream_t s)
 {
+    chunk = std::min(chunk, kChunkSweepsMax);
     // a word a tile, and for the max-update stop one a pass
     const size_t tiles = (size_t)plan.ncol * plan.nrow, passes = (size_t)(chunk - 1) / nsw + 1;
     PCD_TRY(reserve_words(ws, sizeof(unsigned) * (tiles + (a.stop == PCD_STOP_MAX_UPDATE ? passes : 0)), s));
@@ -1849,7 +1854,7 @@ int batch_tiles_solve(TileBatchWorkspace &ws, int dev, const pcd_instance *inst,
     // refine_every, else 128 when the largest side is 1024 or more, down to
     // 32 when it is 256 or less
     const int spacing = o.refine_every > 0 ? o.refine_every : 4 * std::max(8, std::min(32, maxdim / 32));
-    const int chunk = std::min(spacing, o.max_iterations);
+    const int chunk = std::min({spacing, o.max_iterations, kChunkSweepsMax});
 
     PCD_CUDA(cudaEventRecord(ws.t0, s));
     PCD_CUDA(cudaMemcpyAsync(ws.jobs, tj.data(), sizeof(TileJob) * count, cudaMemcpyHostToDevice, s));

@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
     __shared__ TileShared sh;
     tile_begin(smem_f, &sh);
     const unsigned base = *(volatile const unsigned *)&ctl->res_epoch;
-    const int ntiles = ncol * nrow, KQ = (a.W + 7) >> 3, passes = (total - 1) / nsw + 1;
+    const int ntiles = ncol * nrow, KQ = (a.W + 7) >> 3, passes = (total + nsw - 1) / nsw;
     if (threadIdx.x >= kTThreads) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTRegsProduce));
         const int role = ((int)threadIdx.x - kTThreads) >> 5;
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
     }
     __syncthreads();
     const unsigned base = *(volatile const unsigned *)(sync + 1);
-    const int passes = (sweeps - 1) / kTilePassSweeps + 1;
+    const int passes = (sweeps + kTilePassSweeps - 1) / kTilePassSweeps;
     if (threadIdx.x >= kTThreads) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTRegsProduce));
         const int role = ((int)threadIdx.x - kTThreads) >> 5;
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kTBlock, 1)
         for (int j = threadIdx.x; j < njobs; j += kTBlock) {
             if (s_total[j] < 1) continue;
             volatile Ctl *c = jobs[j].ctl;
-            c->stream_out = ((s_total[j] - 1) / kTilePassSweeps + 1) & 1;
+            c->stream_out = ((s_total[j] + kTilePassSweeps - 1) / kTilePassSweeps) & 1;
             const int sw = c->sweeps + s_total[j];
             c->sweeps = sw;
             if (sw >= jobs[j].max_iter) c->halt = 1;
