@@ -80,7 +80,8 @@ typedef struct {
                                 once its residual estimate fell by this factor (then the FP64
                                 residual is refreshed); 0 = auto (3e-2) */
     int block_sweeps;        /* block schedule: sweeps between halo exchanges, 1..8 (halo of
-                                2 x that many cells); 0 = auto (FP64 4, FP32 8) */
+                                2 x that many cells); 0 = auto (FP64 1, 2 or 4 by the expected
+                                time, FP32 8 or fewer) */
 } pcd_solve_opts;
 
 typedef enum {
@@ -95,14 +96,21 @@ typedef enum {
 
 typedef enum {
     PCD_SCHED_AUTO = 0,        /* FP32 sweeps: tiles that stay on the chip where the grid fits (up
-                                  to about two million cells; reported as PCD_SCHED_TILES, with
-                                  the stop tests of the schedule they stand for: the cluster's
-                                  estimate cycles, the tile passes' or the persistent bands'
-                                  chunks), else tile passes (widths that are not a multiple of 8
-                                  with the stop tests, and under the name, of the persistent,
-                                  stream or stripe schedule); grids below 64 x 64 cells or 16
-                                  on a side: persistent, else stream; FP64: blocks, else
-                                  persistent, else stripes; else launches, as the grid allows */
+                                  to 2.2 to 2.7 million cells for widths that are a multiple of
+                                  8, about 1.2 million for others; reported as PCD_SCHED_TILES,
+                                  with the stop tests of the schedule they stand for: the
+                                  cluster's estimate cycles, the tile passes' or the persistent
+                                  bands' chunks), else tile passes (widths that are not a
+                                  multiple of 8 with the stop tests, and under the name, of the
+                                  persistent, stream or stripe schedule; pcd_solve_stats.
+                                  sweep_form tells the two apart); grids below 64 x 64 cells or
+                                  16 on a side: persistent, else stream; FP64: blocks, else
+                                  persistent, else stripes; else launches, as the grid allows.
+                                  Made for one solve at a time: the resident tiles take every
+                                  SM, so that solves of several contexts follow one another (a
+                                  512 x 512 solve to 1e-6 takes 2.0 ms alone, 1.86 ms each on
+                                  eight threads); PCD_SCHED_CLUSTER takes 16 SMs a solve (5.5
+                                  and 1.13 ms), a batch all grids in one launch (eight: 1.08) */
     PCD_SCHED_LAUNCHES = 1,    /* one kernel per half sweep, CUDA-graph chunks (any grid) */
     PCD_SCHED_PERSISTENT = 2,  /* one cooperative launch per solve, bands in shared memory
                                   (no NaN cells, band fits on chip) */
@@ -127,7 +135,7 @@ typedef enum {
     PCD_SCHED_BLOCKS = 7       /* grids without NaN cells: one cooperative launch per solve on
                                   2-D blocks (one per SM), each kept in shared memory with a
                                   halo of 2K cells, K red-black sweeps between exchanges of
-                                  the halo rings through L2 (K = 2 FP64, 8 FP32); mixed
+                                  the halo through L2 (K up to 4 FP64, 8 FP32); mixed
                                   precision folds the FP32 correction into phi in FP64 inside
                                   the launch.  Grids up to about a million cells */
 } pcd_schedule;
@@ -170,14 +178,20 @@ int pcd_solve_opts_default(pcd_solve_opts *opts);
 /* Number of kernels this library launched in this process (monotonic). */
 unsigned long long pcd_kernel_launches(void);
 /* Bounded device waits (no counterpart in the reference, whose solver has no
- * device waits).  The persistent schedule's CTAs wait for their neighbours'
- * epoch flags and for a grid barrier; each wait gives up after `polls` polls
- * (0 = the default 2^24, about half a second), records PCD_TIMEOUT and every
- * CTA returns, leaving the context usable; the solve returns PCD_TIMEOUT.
- * withhold_first_flag = 1 is the failure test's switch: the first CTA never
- * raises its epoch flag, a flag that nothing else sets, so a neighbour's wait
- * runs out on purpose.  Both stay in force for later solves on the context
- * until changed. */
+ * device waits).  CTAs that solve a grid together wait for one another: for
+ * epoch flags and grid barriers (the persistent schedule, the mixed block
+ * schedule), for halo words that carry their epoch (FP64 blocks, the resident
+ * sweeps of AUTO's mixed solves), for a neighbouring tile's last pass (tile
+ * passes, batched ones too).  Each such wait gives up after `polls` polls (0 =
+ * the default: 2^24 for flags and barriers, about six seconds at 0.35 us a poll;
+ * 2^21 for words and passes, about half a second at 0.21 us), records PCD_TIMEOUT
+ * and every CTA returns, leaving the context usable; the solve returns
+ * PCD_TIMEOUT.  Waits inside a CTA for its own copies have bounds of their own,
+ * about two seconds, and the limit does not reach them.
+ * withhold_first_flag = 1 is the failure test's switch: the first CTA (tile
+ * passes: the first tile) never reports, which nothing else does for it, so a
+ * neighbour's wait runs out on purpose.  Both stay in force for later solves and
+ * batches on the context until changed. */
 int pcd_ctx_set_wait_limit(pcd_ctx *ctx, long long polls, int withhold_first_flag);
 
 /* ---- Poisson solve ------------------------------------------------------ */

@@ -644,8 +644,8 @@ int launch_stripes(T *phi, const T *rhs, Ctl *ctl, const SolveArgs &a, int R, in
     return PCD_OK;
 }
 
-// Polls of a tagged word before a wait gives up: each is an L2 trip, together
-// about two seconds.
+// Polls of a tagged word before a wait gives up: 0.21 us each, together about half a
+// second (a withheld word ends a 256^2 solve after 21.6 ms with a limit of 100000).
 constexpr long long kWordPolls = 1ll << 21;
 
 // The tagged words' buffer, zeroed: tags start at 1 in every solve, and no word

@@ -3,8 +3,8 @@
 //
 // The grid is cut into TX x TY tiles, one CTA each, all co-resident
 // (cooperative launch).  A CTA holds its tile plus a halo of 2K cells on every
-// side that has a neighbour; e lives in registers for the whole launch, so
-// does -r32 where a lane holds at most two rows (in shared memory otherwise).
+// side that has a neighbour; e lives in registers for the whole launch, -r32 in
+// shared memory.
 // K sweeps run between two exchanges: the dependency cone of K red-black
 // sweeps ends inside the halo, whose values are recomputed with the owner's
 // arithmetic and thrown away at the next exchange.

@@ -4,7 +4,8 @@
 //
 // At 4096 x 4096 a sweep takes 10.6 us (25.8 when every pass was a launch whose
 // warps loaded 16-row tiles before they swept them, 12.4 when it was a launch of
-// these tiles), at 2048 x 1500 2.5 us (5.3; 3.9).  A tile takes 3.3 us, of which its
+// these tiles), at 2048 x 1500 2.5 us (5.3; 3.9); with an FP64 refresh every 512
+// sweeps 11.1 and 2.65.  A tile takes 3.3 us, of which its
 // eight half sweeps take 2.5: 38% of issue slots busy, three warps a scheduler
 // that wait for one another's edge rows.  On grids of two or three tiles a CTA
 // the way of a halo through L2 (store, report, poll, load) comes on top.
@@ -648,9 +649,9 @@ int tile_plan(int dev, int W, int H, int depth, TilePlan *plan)
         if (bps < 1) return PCD_BAD_ARG;
     }
     // The tallest tiles recompute the fewest halo rows, and passes that no barrier
-    // parts have no last round of CTAs to fill (2048 x 1500: 361 tiles of 80 rows
-    // 2.65 us a sweep, 456 of 64 rows, three full rounds, 3.66; 2048^2 3.07 and
-    // 3.56).  Grids that leave SMs idle are cut finer.
+    // parts have no last round of CTAs to fill (with a refresh every 512 sweeps,
+    // 2048 x 1500: 361 tiles of 80 rows 2.65 us a sweep, 456 of 64 rows, three full
+    // rounds, 3.66; 2048^2 3.03 and 3.56).  Grids that leave SMs idle are cut finer.
     const long most = (long)sms * bps, tiles = (long)p.ncol * p.nrow, rounds = (tiles + most - 1) / most;
     if (rounds == 1)
         p.nrow = (int)std::max<long>(p.nrow, std::min<long>(rounds * most / p.ncol, ceil_div(H, 16)));
