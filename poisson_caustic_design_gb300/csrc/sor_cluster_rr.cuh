@@ -226,6 +226,9 @@ __global__ void __launch_bounds__(kRRThreads, 1) k_sor_cluster_rr(ClusterArgs a)
 
     const Ctl *ctl = a.ctl;
     if (*(volatile const int *)&ctl->done) return;  // speculative launch after convergence: all CTAs agree
+    // (the first round stores into the neighbours' inboxes before its cluster barrier:
+    // they must have started by then; the wait is behind the loads)
+    cl.barrier_arrive();
 
     S st;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -284,6 +287,7 @@ __global__ void __launch_bounds__(kRRThreads, 1) k_sor_cluster_rr(ClusterArgs a)
     const double drop_abs = a.drop * rstart;
     const double stop2 = stop_abs * stop_abs, drop2 = drop_abs * drop_abs;
     const int P = (st.ybase + w * L) & 1;
+    cl.barrier_wait();
     __syncthreads();
 
     // A residual estimate taken after round m is summed over the cluster at
