@@ -432,7 +432,9 @@ __global__ void __launch_bounds__(kStreamThreadsMax, 1)
     const int ys = y0 - 1;
     const unsigned bytes = (unsigned)wpad * 4u;
     const int col0 = 4 * G * threadIdx.x;
-    const bool lft_ok = col0 > 0, rgt_ok = col0 + 4 * G < W;
+    // (threads past the last column have no row to read from: on narrow grids their
+    // place lies beyond the rings)
+    const bool lft_ok = col0 > 0 && col0 < W, rgt_ok = col0 + 4 * G < W;
     float w[5];
 #pragma unroll
     for (int c = 0; c < 5; c++) w[c] = a.w32[c];

@@ -1,5 +1,6 @@
 """Narrow grids on the schedules made for wide ones: one sweep a launch on the
-register-resident cluster form."""
+register-resident cluster form, and stream passes whose block has more threads than
+the row has cells."""
 import numpy as np
 import pytest
 
@@ -41,3 +42,9 @@ def _same(ctx, n, m, ld, schedule, **kw):
 def test_cluster_launches_of_few_sweeps(ctx, n, m, refine_every, sweeps):
     """A launch's first halo stores come a few microseconds after its start."""
     _same(ctx, n, m, n, 3, stop=1, refine_every=refine_every, max_iterations=sweeps)
+
+
+@pytest.mark.parametrize("n,m,ld", [(1, 40, 4), (5, 40, 8), (17, 3, 20), (24, 33, 24), (130, 20, 132), (2050, 9, 2052)])
+@pytest.mark.parametrize("stop", [0, 1])
+def test_stream_passes_on_narrow_rows(ctx, n, m, ld, stop):
+    _same(ctx, n, m, ld, 5, stop=stop, refine_every=16, max_iterations=37)
