@@ -374,6 +374,7 @@ int blocks64_plan(int dev, int W, int H, int K, Blocks64Plan *plan)
         }
     }
     if (!best.K) return PCD_BAD_ARG;
+    PCD_CUDA(allow_shared((const void *)k_sor_blocks64));
     *plan = best;
     return PCD_OK;
 }
@@ -385,7 +386,6 @@ int launch_blocks64(Blocks64Args &a, const Blocks64Plan &p, cudaStream_t s)
     a.G = p.TY * p.TX;
     a.K = p.K;
     a.RTmax = p.RTmax;
-    PCD_CUDA(allow_shared((const void *)k_sor_blocks64));
     void *params[] = {&a};
     PCD_CUDA(cudaLaunchCooperativeKernel((const void *)k_sor_blocks64, dim3(a.G), dim3(kB64Threads), params, p.smem, s));
     count_launches(1);

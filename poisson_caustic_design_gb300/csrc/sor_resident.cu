@@ -540,6 +540,8 @@ int resident_plan(int dev, int W, int H, ResidentPlan *plan)
                 }
             }
     if (!best.L) return PCD_BAD_ARG;
+    // (here and not in front of every launch, which it would hold up)
+    PCD_CUDA(allow_shared(rs_kernel(best.K, best.L, best.CL, W % 8 != 0)));
     *plan = best;
     return PCD_OK;
 }
@@ -556,7 +558,6 @@ int launch_resident(ResidentArgs &a, const ResidentPlan &p, cudaStream_t s)
     a.TY = p.TY;
     a.NG = p.NG;
     a.R = p.R;
-    PCD_CUDA(allow_shared(fn));
     void *params[] = {&a};
     if (p.TX * p.TY == 1) PCD_CUDA(cudaLaunchKernel(fn, dim3(1), dim3(32 * p.NW), params, p.smem, s));
     else PCD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.TX * p.TY), dim3(32 * p.NW), params, p.smem, s));
