@@ -118,3 +118,20 @@ def test_stats_tell_what_the_sweeps_ran_on(ctx, n, m, ld, schedule, used, form):
     b = pcd.inputs.poisson_rhs(max(n, m), 5, "gaussian", m=max(n, m))[:m, :n]
     st, _ = _solve(ctx, b, ld=ld, stop=1, tol=1e-14, max_iterations=8, omega=1.9, schedule=schedule)
     assert (st["schedule_used"], st["sweep_form"]) == (used, form)
+
+
+# one grid for each instance of the kernel that a plan takes: sweeps per exchange, rows
+# and lane columns of a lane group, whole and partial lane columns
+@pytest.mark.parametrize("n,m", [(72, 16), (72, 17), (776, 2310), (792, 2436), (16, 144), (200, 2436), (456, 2401),
+                                 (584, 2359), (17, 16), (65, 16), (65, 17), (17, 144), (193, 2436)])
+def test_every_instance_matches_launch_schedule(ctx, n, m):
+    import poisson_caustic_design_gb300 as pcd
+
+    b = pcd.inputs.poisson_rhs(max(n, m), 5, "gaussian", m=max(n, m))[:m, :n]
+    b = b - b.mean()
+    out = {}
+    for sched in (1, 0):
+        st, out[sched] = _solve(ctx, b, stop=1, tol=1e-14, max_iterations=37, omega=1.9, schedule=sched)
+        assert st["sweeps"] == 37
+    assert st["sweep_form"] == 1
+    assert np.abs(out[0] - out[1]).max() < 1e-5 * np.abs(out[1]).max()
