@@ -1460,7 +1460,6 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         set_error("pcd solve: bad options");
         return PCD_BAD_ARG;
     }
-    if (stats) stats->sweep_form = 0;
     PCD_TRY(ws.reserve((size_t)H * std::max<size_t>(ld, quads::quad_row_floats(W))));
 
     SolveArgs a;
@@ -1500,6 +1499,7 @@ int solve_device(SolverWorkspace &ws, const double *b, double *phi, int W, int H
         const int st = solve_resident(ws, b, phi, a, o, rp, rule, stats, &nans, s);
         if (!nans) return st;
     }
+    if (stats) stats->sweep_form = 0;  // (tile passes set their own)
     PCD_CUDA(cudaMemcpyAsync(ws.ctl_host, ws.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     PCD_CUDA(cudaStreamSynchronize(s));
     const int masked = ws.ctl_host[0].nan_cells > 0 ? 1 : 0;

@@ -53,7 +53,7 @@ def test_auto_takes_the_masked_launches(ctx, n, m, ld, stop, warm):
         phi.copy_(start)
         st = ctx.solve_device(b, phi, pcd.SolveOptions(stop=stop, tol=0.0, max_iterations=75, omega=1.8, warm_start=warm,
                                                        precision=pcd.PREC_MIXED, schedule=sched))
-        assert st["sweeps"] == 75
+        assert st["sweeps"] == 75 and st["sweep_form"] == 0
         out.append((phi, st["rel_residual"], st["last_max_update"]))
     assert torch.equal(torch.isnan(out[1][0]), torch.isnan(b))
     assert torch.equal(torch.nan_to_num(out[0][0]), torch.nan_to_num(out[1][0]))
